@@ -67,15 +67,22 @@ __shared__ unsigned long long cot_pst[16][16];
 // cell at the last evaluation
 #define COT_NB_HIDDEN 100
 #define COT_RCAP 32  // ring buffer vertices per cell (the split integration)
-// pixel box above which a cell is integrated first, and above which by
-// COT_SPLIT warps (measured at 65,536 sites on a 1024^2 target, M cell-evals/s:
-// 512/4096 144.6, 1024/4096 142.5, 512/2048 142.0, 1024/8192 140.8,
-// 1024/16384 139.6, 2048/8192 139.3)
+// Pixel box above which a cell is integrated first, by a whole warp, and
+// above which by COT_SPLIT warps.  The others share a warp with three more
+// cells (integrate_walk), where a large one would hold up its neighbours, and
+// one warp on 4,096 pixels takes as long as all the small cells together.
+// Measured as two evaluations at 65,536 sites on 1024^2 / 262,144 on 2048^2
+// (us): first-whole at 512, 256, 128, 64: 725 / 2075, 718 / 2072, 712 / 2066,
+// 712 / 2105; split at 4096, 2048, 1024, 512 (with 128): 712 / 2066,
+// 706 / 2066, 698 / 2068, 699 / 2070.
 #ifndef COT_HEAVY_PIX
-#define COT_HEAVY_PIX 512
+#define COT_HEAVY_PIX 128
 #endif
 #ifndef COT_SPLIT_PIX
-#define COT_SPLIT_PIX 4096
+#define COT_SPLIT_PIX 1024
+#endif
+#ifndef COT_SEG_NV
+#define COT_SEG_NV 16       // largest ring that the 8-lane integration takes
 #endif
 #define CST_HEAVY (-2)      // cstate of a cell on the heavy integration list
 
@@ -1149,6 +1156,219 @@ __device__ __forceinline__ CellAcc integrate_fast(SP &P, int nv, const PixGeo g,
     return acc;
 }
 
+// Scratch of one cell's integration by 8 lanes.  The paddings put the four
+// segments of a warp on different banks when each reads one entry.
+struct WalkScratch {
+    double2 V[COT_SEG_NV + 2];   // ring, relative to the site
+    double IDX[COT_SEG_NV + 2];  // per edge: 1/dx (0 for a vertical edge)
+};
+
+// The pixel line at or before p (spacing s, line 0 at z, is = 1/s), settled
+// against the explicitly rounded positions: lpos(r) <= p < lpos(r + 1).
+__device__ __forceinline__ int line_before(double p, double s, double is, double z, bool &on)
+{
+    int r = (int)floor((p - z) * is);
+    double at = lpos(r, s, z);
+    if (at > p) {
+        r--;
+        at = lpos(r, s, z);
+    } else {
+        const double up = lpos(r + 1, s, z);
+        if (up <= p) {
+            r++;
+            at = up;
+        }
+    }
+    on = at == p;
+    return r;
+}
+
+// The sums of integrate_fast for four cells a warp, 8 lanes each (rings of up
+// to COT_SEG_NV vertices and pixel boxes of up to COT_HEAVY_PIX pixels).  A
+// lane walks one edge from crossing to crossing, and then one vertical pixel
+// line from row to row, so a piece costs only its own terms: no scan hands
+// it out and nothing of the edge is looked up again.  The lane-per-piece form
+// of integrate_fast keeps 32 lanes busy on one cell but pays four times the
+// instructions a piece; with 8 lanes a cell the edges (6) and lines (5 to 8)
+// fill the lanes by themselves.  Bound by instruction issue (129 M warp
+// instructions at 262,144 sites on 2048^2 against 450 M, k_integrate 205
+// against 566 us; 65 against 150 us at 65,536 sites on 1024^2, where the
+// largest cells now take longest).
+//
+// The terms of a piece are taken about its middle (am, bm) with half extents
+// (ha, hb): along it the averages of a, a^2, ab and a^3/3 + ab^2 are am,
+// am^2 + ha^2/3, am bm + ha hb/3 and
+// am (am^2/3 + ha^2/3 + bm^2 + hb^2/3) + 2 bm ha hb/3, exactly.
+__device__ __forceinline__ CellAcc integrate_walk(WalkScratch &P, int nv, const PixGeo g, double2 si)
+{
+    const int sl = threadIdx.x & 7;
+    double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
+    for (int k = sl; k < nv; k += 8) {
+        const double2 p = P.V[k];
+        mnx = fmin(mnx, p.x);
+        mxx = fmax(mxx, p.x);
+        mny = fmin(mny, p.y);
+        mxy = fmax(mxy, p.y);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        mnx = fmin(mnx, __shfl_xor_sync(FULLMASK, mnx, o));
+        mxx = fmax(mxx, __shfl_xor_sync(FULLMASK, mxx, o));
+        mny = fmin(mny, __shfl_xor_sync(FULLMASK, mny, o));
+        mxy = fmax(mxy, __shfl_xor_sync(FULLMASK, mxy, o));
+    }
+    const double ox = 0.5 * (mnx + mxx), oy = 0.5 * (mny + mxy);  // local origin
+    const double cx0 = g.pd0 - si.x, cy0 = g.pd2 - si.y;           // pixel line 0, site frame
+    double sA = 0.0, sIa = 0.0, sIb = 0.0, sI2 = 0.0;
+
+    // ---- (a) edge pieces --------------------------------------------------
+    for (int k = sl; k < nv; k += 8) {
+        const double2 p = P.V[k], q = P.V[(k + 1 >= nv) ? 0 : k + 1];
+        const double dx = q.x - p.x, dy = q.y - p.y;
+        const double idx = dx != 0.0 ? 1.0 / dx : 0.0, idy = dy != 0.0 ? 1.0 / dy : 0.0;
+        P.IDX[k] = idx;
+        bool onx, ony;
+        int ix = line_before(p.x, g.xs, g.ixs, cx0, onx);
+        int iy = line_before(p.y, g.ys, g.iys, cy0, ony);
+        // a horizontal edge has no x-dy term; a vertical edge on a pixel line
+        // is counted with the lines in (b)
+        if (dy == 0.0 || (dx == 0.0 && onx)) continue;
+        // both axes turned so that the edge runs upwards: lines at
+        // U = fma(c, xs, zx), c = the next one on the way, mirrored exactly
+        // where the edge runs down.  The pixel is the one before the line.
+        const bool xu = dx > 0.0, yu = dy > 0.0;
+        const double ux = xu ? p.x : -p.x, ex = xu ? q.x : -q.x, zx = xu ? cx0 : -cx0, jx = fabs(idx);
+        const double uy = yu ? p.y : -p.y, ey = yu ? q.y : -q.y, zy = yu ? cy0 : -cy0, jy = fabs(idy);
+        double c = xu ? (double)(ix + 1) : (double)(onx ? 1 - ix : -ix);
+        double r = yu ? (double)(iy + 1) : (double)(ony ? 1 - iy : -iy);
+        ix -= !xu && onx ? 1 : 0;
+        iy -= !yu && ony ? 1 : 0;
+        const int cs = xu ? 1 : -1, rs = yu ? 1 : -1;
+        // t of the next crossing, 1 when the line is not short of the end
+        const auto tx = [&]() -> double {
+            const double U = __fma_rn(c, g.xs, zx);
+            return U < ex ? line_t(U, ux, jx) : 1.0;
+        };
+        const auto ty = [&]() -> double {
+            const double U = __fma_rn(r, g.ys, zy);
+            return U < ey ? line_t(U, uy, jy) : 1.0;
+        };
+        const double ax = p.x - ox, ay = p.y - oy;
+        double t0 = 0.0, tc = tx(), tr = ty();
+        for (int it = 0; it < 2 * COT_HEAVY_PIX + 16; it++) {
+            const double t1 = tc < tr ? tc : tr;
+            // a piece outside the image (a rounding sliver along the domain
+            // sides) carries no density
+            const bool in = (unsigned)ix < (unsigned)g.nx && (unsigned)iy < (unsigned)g.ny;
+            const double rho = in ? g.rho[ix + iy * g.nx] : 0.0;
+            const double th = 0.5 * (t1 - t0), tm = 0.5 * (t0 + t1);
+            const double ha = th * dx, hb = th * dy;
+            const double am = __fma_rn(tm, dx, ax), bm = __fma_rn(tm, dy, ay);
+            const double h3 = ha * (1.0 / 3.0);
+            const double hxx = h3 * ha, hxy = h3 * hb, hyy = hb * hb * (1.0 / 3.0);
+            const double w = rho * hb, a2 = am * am;
+            sA += w * am;
+            sIa += w * (a2 + hxx);
+            sIb += w * (am * bm + hxy);
+            sI2 += w * (am * (a2 * (1.0 / 3.0) + hxx + (bm * bm + hyy)) + 2.0 * bm * hxy);
+            if (!(t1 < 1.0)) break;
+            const bool gx = tc <= t1, gy = tr <= t1;
+            if (gx) {
+                c += 1.0;
+                ix += cs;
+                tc = tx();
+            }
+            if (gy) {
+                r += 1.0;
+                iy += rs;
+                tr = ty();
+            }
+            t0 = t1;
+        }
+    }
+    // db = 2 hb, and Ia carries a factor 1/2
+    sA *= 2.0;
+    sIb *= 2.0;
+    sI2 *= 2.0;
+    __syncwarp();
+
+    // ---- (b) vertical pixel lines inside the cell --------------------------
+    // pixel columns [lx, hx) and rows [ly, hy) of the cell's box, one pixel
+    // wider on each side; lines lx .. hx, one a lane
+    if (nv > 0) {
+        const int lx = max((int)floor((mnx - cx0) * g.ixs) - 1, 0);
+        const int ly = max((int)floor((mny - cy0) * g.iys) - 1, 0);
+        const int hx = min((int)floor((mxx - cx0) * g.ixs) + 2, g.nx);
+        const int hy = min((int)floor((mxy - cy0) * g.iys) + 2, g.ny);
+        for (int l = lx + sl; l <= hx; l += 8) {
+            const double xl = lpos(l, g.xs, cx0);
+            const bool fl = l - 1 >= lx && mnx < xl && xl <= mxx;  // right side of pixel l-1 (a left limit)
+            const bool fr = l < hx && mnx <= xl && xl < mxx;       // left side of pixel l (a right limit)
+            if (!fl && !fr) continue;
+            double lo = INFINITY, hi = -INFINITY;
+            double2 p = P.V[nv - 1];
+            double dp = xl - p.x;
+            for (int k = 0; k < nv; k++) {
+                // the edge from p, number k - 1
+                const double2 q = P.V[k];
+                const double dq = xl - q.x;
+                if (dp * dq <= 0.0) {
+                    // (the far end exactly; a vertical edge gives its own start,
+                    // its end is the next edge's)
+                    const double t = __dmul_rn(dp, P.IDX[k > 0 ? k - 1 : nv - 1]);
+                    const double y = dq == 0.0 && p.x != q.x ? q.y : __fma_rn(t, q.y - p.y, p.y);
+                    lo = y < lo ? y : lo;
+                    hi = y > hi ? y : hi;
+                }
+                p = q;
+                dp = dq;
+            }
+            if (!(hi > lo)) continue;
+            bool on;
+            int r = line_before(lo, g.ys, g.iys, cy0, on);
+            int rl = line_before(hi, g.ys, g.iys, cy0, on);
+            if (on) rl--;  // the last row that reaches below hi
+            r = max(r, ly);
+            rl = min(rl, hy - 1);
+            const double *__restrict__ pl = g.rho + (l - 1) + r * g.nx;
+            double s1 = 0.0, s2 = 0.0, s3 = 0.0;
+            double b0 = fmax(lo, lpos(r, g.ys, cy0)) - oy;
+            double q0 = b0 * b0, c0 = q0 * b0;
+            for (; r <= rl; r++) {
+                const double wl = fl ? pl[0] : 0.0, wr = fr ? pl[1] : 0.0;
+                pl += g.nx;
+                const double b1 = fmin(hi, lpos(r + 1, g.ys, cy0)) - oy;
+                const double q1 = b1 * b1, c1 = q1 * b1;
+                const double wd = wl - wr;
+                s1 += wd * (b1 - b0);
+                s2 += wd * (q1 - q0);
+                s3 += wd * (c1 - c0);
+                b0 = b1;
+                q0 = q1;
+                c0 = c1;
+            }
+            // upwards: the left pixel's right side
+            const double a = xl - ox;
+            sA += a * s1;
+            sIa += 0.5 * a * a * s1;
+            sIb += 0.5 * a * s2;
+            sI2 += a * (1.0 / 3.0) * (a * a * s1 + s3);
+        }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        sA += __shfl_xor_sync(FULLMASK, sA, o);
+        sIa += __shfl_xor_sync(FULLMASK, sIa, o);
+        sIb += __shfl_xor_sync(FULLMASK, sIb, o);
+        sI2 += __shfl_xor_sync(FULLMASK, sI2, o);
+    }
+    CellAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+    acc.mu = sA;
+    // int |x - s_i|^2 = int |(x - o) + o|^2 in the site frame
+    acc.S = sI2 + 2.0 * (ox * sIa + oy * sIb) + (ox * ox + oy * oy) * sA;
+    return acc;
+}
+
 // Plain area centroid of the polygon (relative to the site).
 template <class SP>
 __device__ void poly_centroid(const SP &P, int nv, int lane, double &cx, double &cy)
@@ -2007,7 +2227,7 @@ __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a,
                 const int c1 = __reduce_max_sync(FULLMASK, lane < nv ? cx : INT_MIN);
                 const int r1 = __reduce_max_sync(FULLMASK, lane < nv ? cy : INT_MIN);
                 const double box = (double)(c1 - c0 + 1) * (double)(r1 - r0 + 1);
-                if (box > (double)COT_HEAVY_PIX && lane == 0) {
+                if ((box > (double)COT_HEAVY_PIX || nv > COT_SEG_NV) && lane == 0) {
                     // the largest boxes are shared by COT_SPLIT warps (while
                     // the split list has room), the others start first whole
                     int slot = a.hsplit_cap;
@@ -2576,23 +2796,41 @@ __global__ void __launch_bounds__(32 * HEAVY_WARPS, 2) k_cells_heavy(const __gri
     }
 }
 
+// Scratch of one cell's integration by a whole warp.
+struct RingScratch {
+    double X[32], Y[32], EIX[32], EIY[32], ESL[32];  // ring; per edge 1/dx, 1/dy, dy/dx
+};
+
 // One part of a split cell's integration, out of line so that the rare path
 // leaves the integration kernel's registers to the common one.
-__device__ __noinline__ void integrate_part(FastScratch &S, int nv, const PixGeo pg, double2 si, int lane, int part,
+__device__ __noinline__ void integrate_part(RingScratch &S, int nv, const PixGeo pg, double2 si, int part,
                                             double *raw)
 {
-    integrate_fast<32, FastScratch, true>(S, nv, pg, si, lane, part, COT_SPLIT, raw);
+    integrate_fast<32, RingScratch, true>(S, nv, pg, si, threadIdx.x & 31, part, COT_SPLIT, raw);
 }
 
-// The masses and objective terms of the cells whose rings k_cells_fast left
-// in the ring buffer: one warp per cell, fetched from a counter, the same
-// edge-walk integration as the fused path (so the same sums).  Cells above
-// COT_RCAP vertices are integrated by the large-ring pass instead.
-template <int MINB>
+// A whole cell by one warp inside the 8-lane instance, out of line likewise.
+__device__ __noinline__ CellAcc integrate_whole(RingScratch &S, int nv, const PixGeo pg, double2 si)
+{
+    return integrate_fast<32>(S, nv, pg, si, threadIdx.x & 31);
+}
+
+// shared memory of one warp of k_integrate
+constexpr int INT_WARP_SMEM =
+    (int)(sizeof(RingScratch) > 4 * sizeof(WalkScratch) ? sizeof(RingScratch) : 4 * sizeof(WalkScratch));
+
+// The masses and objective terms of the cells whose rings the ring kernels
+// left in the ring buffer: 32 / L cells a warp, fetched from a counter.
+// Cells above COT_RCAP vertices are integrated by the large-ring pass
+// instead.  L = 8 needs the heavy list: it holds the cells above COT_SEG_NV
+// vertices or COT_HEAVY_PIX pixels of box, which take a whole warp.
+template <int MINB, int L>
 __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
 {
+    constexpr int CPW = 32 / L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    FastScratch &S = reinterpret_cast<FastScratch *>(smem_raw)[threadIdx.x >> 5];
+    unsigned char *mine = smem_raw + (threadIdx.x >> 5) * INT_WARP_SMEM;
+    RingScratch &S = *reinterpret_cast<RingScratch *>(mine);
     const int lane = threadIdx.x & 31;
     int *fetch = a.ovf_count + 6;
     // the parts of the split cells first, then the heavy list, then every
@@ -2603,7 +2841,7 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
         int f = 0;
         if (lane == 0) f = atomicAdd(fetch, 1);
         f = __shfl_sync(FULLMASK, f, 0);
-        if (f >= g.n + nh + np) break;
+        if (f >= (g.n + CPW - 1) / CPW + nh + np) break;
         if (f < np) {
             // one part of a split cell: its raw sums to the slot, and the
             // part that finishes last adds the parts in order
@@ -2617,7 +2855,7 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
             }
             __syncwarp();
             double raw[6];
-            integrate_part(S, nv, pix_geo(g), g.xy[i], lane, part, raw);
+            integrate_part(S, nv, pix_geo(g), g.xy[i], part, raw);
             if (lane == 0) {
                 double *pp = a.hpart + ((size_t)slot * COT_SPLIT + part) * 4;
                 pp[0] = raw[0];
@@ -2646,32 +2884,53 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
             continue;
         }
         f -= np;
-        int i;
-        if (f < nh) {
-            i = a.hlist[f];
-        } else {
-            i = f - nh;
-            if ((nh > 0 || np > 0) && a.cstate[i] == CST_HEAVY) continue;
-        }
-        const int nv = a.nv[i];
-        if (nv > COT_RCAP) continue;
-        double mu = 0.0, fcv = 0.0;
-        if (nv >= 3) {
-            if (lane < nv) {
-                const double2 v = a.rbuf[(size_t)i * COT_RCAP + lane];
-                S.X[lane] = v.x;
-                S.Y[lane] = v.y;
+        if (L == 32 || f < nh) {
+            // a whole warp for the cell
+            const int i = f < nh ? a.hlist[f] : f - nh;
+            if (f >= nh && (nh > 0 || np > 0) && a.cstate[i] == CST_HEAVY) continue;
+            const int nv = a.nv[i];
+            if (nv > COT_RCAP) continue;
+            double mu = 0.0, fcv = 0.0;
+            if (nv >= 3) {
+                if (lane < nv) {
+                    const double2 v = a.rbuf[(size_t)i * COT_RCAP + lane];
+                    S.X[lane] = v.x;
+                    S.Y[lane] = v.y;
+                }
+                __syncwarp();
+                const CellAcc acc = L == 32 ? integrate_fast<32>(S, nv, pix_geo(g), g.xy[i], lane)
+                                            : integrate_whole(S, nv, pix_geo(g), g.xy[i]);
+                mu = acc.mu;
+                fcv = -(acc.S - a.wt[i] * acc.mu);
+            }
+            if (lane == 0) {
+                a.mu[i] = mu;
+                a.fc[i] = fcv;
             }
             __syncwarp();
-            const CellAcc acc = integrate_fast<32>(S, nv, pix_geo(g), g.xy[i], lane);
-            mu = acc.mu;
-            fcv = -(acc.S - a.wt[i] * acc.mu);
+            continue;
         }
-        if (lane == 0) {
-            a.mu[i] = mu;
-            a.fc[i] = fcv;
+        if constexpr (L < 32) {
+            WalkScratch &T = reinterpret_cast<WalkScratch *>(mine)[lane / L];
+            const int sl = lane & (L - 1);
+            const int i = (f - nh) * CPW + lane / L;
+            // the segment's cell: none past the end, for a heavy cell, or a
+            // ring of the large-ring pass
+            int nv = -1;
+            if (i < g.n && !((nh > 0 || np > 0) && a.cstate[i] == CST_HEAVY)) nv = a.nv[i];
+            if (nv > COT_SEG_NV) nv = -1;
+            const int m = nv >= 3 ? nv : 0;
+            double2 si = make_double2(0.0, 0.0);
+            if (m > 0) si = g.xy[i];
+            for (int k = sl; k < m; k += L) T.V[k] = a.rbuf[(size_t)i * COT_RCAP + k];
+            __syncwarp();
+            const CellAcc acc = integrate_walk(T, m, pix_geo(g), si);
+            if (sl == 0 && nv >= 0) {
+                a.mu[i] = m > 0 ? acc.mu : 0.0;
+                a.fc[i] = m > 0 ? -(acc.S - a.wt[i] * acc.mu) : 0.0;
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
 }
 
@@ -3002,6 +3261,16 @@ static size_t cells_smem(int maxv, int warps)
 #ifndef WALK_MINB
 #define WALK_MINB 8   // k_cells_walk (64 registers; 6 blocks measured 2 % slower)
 #endif
+#ifndef INT_MINB
+#define INT_MINB 6  // k_integrate: 80 registers (8 blocks: 2043 us at 262,144 sites against 2072, but 724 against 718 at 65,536)
+#endif
+// sites above which four cells share a warp of the integration: at 4,096 a
+// warp a cell still fits the GPU at once (148 x 32 warps) and each cell is
+// done sooner (two evaluations at 1,024 sites 325 against 334 us, 25
+// iterations at 4,096 sites 6.47 against 6.58 ms)
+#ifndef COT_SEG_MIN_N
+#define COT_SEG_MIN_N 4096
+#endif
 static int g_blocks_per_sm32 = 0, g_blocks_per_sm16 = 0, g_blocks_per_sm8 = 0, g_blocks_per_smi = 0;
 static int g_blocks_per_smf = 0, g_blocks_per_smw = 0, g_blocks_per_smb = 0;
 
@@ -3098,7 +3367,10 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     if (!exact) {
         const int per_smi = g_blocks_per_smi > 0 ? g_blocks_per_smi : 8;
         const int bi = std::min((g.n + CELLS_WPB - 1) / CELLS_WPB, sms * per_smi);
-        k_integrate<8><<<bi, 32 * CELLS_WPB, sizeof(FastScratch) * CELLS_WPB, s>>>(g, a);
+        if (a.hlist != nullptr && g.n > COT_SEG_MIN_N)
+            k_integrate<INT_MINB, 8><<<bi, 32 * CELLS_WPB, INT_WARP_SMEM * CELLS_WPB, s>>>(g, a);
+        else
+            k_integrate<INT_MINB, 32><<<bi, 32 * CELLS_WPB, INT_WARP_SMEM * CELLS_WPB, s>>>(g, a);
         c.launches++;
     }
     if (timed) {
@@ -3145,7 +3417,9 @@ void configure_cells_kernels()
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, false, 8>, 32 * CELLS_WPB,
                                                       sm8) == cudaSuccess && nb > 0)
         g_blocks_per_sm8 = nb;
-    cudaFuncSetAttribute(k_integrate<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
+    const int smi = INT_WARP_SMEM * CELLS_WPB;
+    cudaFuncSetAttribute(k_integrate<INT_MINB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi);
+    cudaFuncSetAttribute(k_integrate<INT_MINB, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi);
     cudaFuncSetAttribute(k_cells_first<FIRST_MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
     cudaFuncSetAttribute(k_cells_walk<WALK_MINB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
     cudaFuncSetAttribute(k_cells_walk<WALK_MINB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
@@ -3166,7 +3440,7 @@ void configure_cells_kernels()
         nb > 0)
         g_blocks_per_smb = nb;
     nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_integrate<8>, 32 * CELLS_WPB, sm32) == cudaSuccess &&
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_integrate<INT_MINB, 8>, 32 * CELLS_WPB, smi) == cudaSuccess &&
         nb > 0)
         g_blocks_per_smi = nb;
 }

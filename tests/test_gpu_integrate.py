@@ -1,0 +1,54 @@
+"""The 8-lane integration (four cells a warp, problems above 4,096 sites)
+against the oracle: pixel grids that cut the cells every way, cells aligned
+with the pixels, rings around its capacity, boxes around its limits."""
+import numpy as np
+import pytest
+
+from caustic_b200 import problems
+from test_gpu_parity import check_eval, solver_for
+
+pytestmark = pytest.mark.gpu
+
+GX, GY = 73, 59  # 4,307 sites: not a multiple of four cells
+
+
+def lattice(nx, ny, pd, jitter, seed):
+    rng = np.random.default_rng(seed)
+    u = (np.arange(GX) + 0.5 + rng.uniform(-jitter, jitter, (GY, GX))) / GX
+    v = ((np.arange(GY) + 0.5)[:, None] + rng.uniform(-jitter, jitter, (GY, GX))) / GY
+    xy = np.column_stack([pd[0] + (pd[1] - pd[0]) * u.ravel(), pd[2] + (pd[3] - pd[2]) * v.ravel()])
+    nu = rng.uniform(0.5, 1.5, len(xy))
+    pic = rng.uniform(0.0, 1.0, nx * ny) ** 2
+    pic[rng.uniform(size=nx * ny) < 0.1] = 0.0
+    p = problems.SDOTProblem("lattice", xy, nu / nu.sum(), pic / pic.sum(), (nx, ny), np.array(pd, float))
+    return p, (pd[1] - pd[0]) * (pd[3] - pd[2]) / len(xy), rng
+
+
+@pytest.mark.parametrize("nx,ny,pd,jitter", [
+    (292, 236, [0.0, 1.0, 0.0, 1.0], 0.0),      # cell sides on pixel lines, four cells at a vertex
+    (219, 118, [-3.3, 7.1, 0.7, 2.9], 0.0),     # sides half a pixel off the lines
+    (301, 173, [0.0, 160.0, -60.0, 100.0], 0.3),
+    (900, 41, [0.0, 1.0, 0.0, 1.0], 0.3),       # many lines one way, fewer than a row a cell the other
+    (1, 1, [-1.0, 1.0, -1.0, 1.0], 0.3),
+])
+def test_small_cells_match_oracle(gpu, nx, ny, pd, jitter):
+    p, cell, rng = lattice(nx, ny, pd, jitter, nx + ny)
+    s = solver_for(p)
+    for w in (np.zeros(p.n), rng.normal(0.0, 0.4 * cell, p.n)):
+        check_eval(p, w, s)
+
+
+def test_rings_and_boxes_around_the_limits(gpu):
+    """A few strongly weighted sites among small ones: rings of more than 8
+    and more than 16 edges, boxes below and above the limits of both paths."""
+    p, cell, rng = lattice(584, 472, [0.0, 1.0, 0.0, 1.0], 0.3, 3)
+    w = rng.normal(0.0, 0.1 * cell, p.n)
+    big = rng.choice(p.n, 40, replace=False)
+    w[big] += np.linspace(0.5, 40.0, 40) * cell
+    s = solver_for(p)
+    check_eval(p, w, s)
+    off, _, _ = s.cells(w)
+    sizes = np.diff(off)
+    c = s.eval_counters()
+    assert (sizes > 16).any() and ((sizes > 8) & (sizes <= 16)).any(), np.bincount(sizes)
+    assert c["integrated_first"] > 0 and c["integrations_split"] > 0, c
