@@ -49,6 +49,7 @@ struct CotProblemDev {
     int *blist = nullptr, *bcnt = nullptr;  // the bucket walk's leaf lists (solves only)
     double2 *rbuf = nullptr;  // ring vertices between the cell and integration kernels
     int *lbuf = nullptr;      // ring generators between the two ring-building kernels
+    int *flist = nullptr;     // the cells that the thread-per-cell ring kernels leave
     int *cstate = nullptr;    // per-cell state between them
     int *nv = nullptr, *ovf_list = nullptr, *ovf_list2 = nullptr, *ovf_count = nullptr;
     int *wlist = nullptr;  // cells whose certificate walk overflowed (finished a block each)
@@ -175,7 +176,7 @@ using namespace cot;
 // the L-BFGS history, which are sized by the sites too).
 static void free_sized_by_sites(CotProblemDev &P)
 {
-    void *ptrs[] = {P.xy, P.nu, P.sbucket, P.rho, P.perm, P.w, P.wt, P.d, P.mu, P.mut, P.wq, P.fc, P.rbuf, P.lbuf,
+    void *ptrs[] = {P.xy, P.nu, P.sbucket, P.rho, P.perm, P.w, P.wt, P.d, P.mu, P.mut, P.wq, P.fc, P.rbuf, P.lbuf, P.flist,
                     P.cstate, P.nv, P.ovf_list, P.ovf_list2, P.ovf_count, P.wlist, P.hsplit, P.hpart, P.hticket, P.nbc, P.nbn, P.nbc_q, P.nbn_q, P.partials,
                     P.ticket, P.out, P.tmp, P.S, P.Sv, P.Yv, P.hval, P.hdiag, P.hbig_val, P.hcol, P.hcnt,
                     P.hbig_col, P.herr, P.nb_b, P.nb_r, P.nb_z, P.nb_pa, P.nb_pb, P.nb_q, P.nb_part, P.nb_tau, P.pcg,
@@ -184,7 +185,7 @@ static void free_sized_by_sites(CotProblemDev &P)
         if (p) cudaFree(p);
     P.xy = nullptr; P.nu = nullptr; P.sbucket = nullptr; P.rho = nullptr; P.perm = nullptr;
     P.w = P.wt = P.d = P.mu = P.mut = P.wq = P.fc = nullptr;
-    P.rbuf = nullptr; P.lbuf = P.cstate = P.nv = P.ovf_list = P.ovf_list2 = P.ovf_count = P.wlist = nullptr;
+    P.rbuf = nullptr; P.lbuf = P.flist = P.cstate = P.nv = P.ovf_list = P.ovf_list2 = P.ovf_count = P.wlist = nullptr;
     P.hsplit = nullptr; P.hpart = nullptr; P.hticket = nullptr;
     P.nbc = P.nbn = P.nbc_q = P.nbn_q = nullptr;
     P.partials = nullptr; P.ticket = nullptr; P.out = nullptr; P.tmp = nullptr; P.S = nullptr;
@@ -392,8 +393,9 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
         A((void **)&P.w, N * 8);
         A((void **)&P.wt, N * 8);
         A((void **)&P.wq, N * 8);
-        A((void **)&P.rbuf, N * 32 * sizeof(double2));
-        A((void **)&P.lbuf, N * 32 * sizeof(int));
+        A((void **)&P.rbuf, ring_entries(N) * sizeof(double2));
+        A((void **)&P.lbuf, ring_entries(N) * sizeof(int));
+        A((void **)&P.flist, N * sizeof(int));
         A((void **)&P.cstate, N * sizeof(int));
         A((void **)&P.d, N * 8);
         A((void **)&P.mu, N * 8);
@@ -630,6 +632,7 @@ static CellsArgs cells_args(CotProblemDev &P, const double *w, const double *d, 
     a.wbar = P.wbar;
     a.rbuf = P.rbuf;
     a.lbuf = P.lbuf;
+    a.flist = P.flist;
     a.cstate = P.cstate;
     a.mu = P.mut;
     a.fc = P.fc;

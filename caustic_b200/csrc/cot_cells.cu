@@ -2108,8 +2108,8 @@ __device__ __forceinline__ RegPoly cell_walk(const CotGeo &g, const CellsArgs &a
             // with a block and clips the deepest first
             if (!brute && ncur > COT_DEFER_LEAVES && a.wlist != nullptr) {
                 if (lane < P.nv) {
-                    a.rbuf[(size_t)i * COT_RCAP + lane] = make_double2(P.x, P.y);
-                    a.lbuf[(size_t)i * COT_RCAP + lane] = P.l;
+                    a.rbuf[ring_at(i, lane)] = make_double2(P.x, P.y);
+                    a.lbuf[ring_at(i, lane)] = P.l;
                 }
                 if (lane == 0) {
                     a.cstate[i] = P.nv;
@@ -2142,8 +2142,8 @@ __device__ __forceinline__ RegPoly cell_walk(const CotGeo &g, const CellsArgs &a
             // buffer and k_cells_heavy finishes the cell with a block
             if (a.wlist != nullptr) {
                 if (lane < P.nv) {
-                    a.rbuf[(size_t)i * COT_RCAP + lane] = make_double2(P.x, P.y);
-                    a.lbuf[(size_t)i * COT_RCAP + lane] = P.l;
+                    a.rbuf[ring_at(i, lane)] = make_double2(P.x, P.y);
+                    a.lbuf[ring_at(i, lane)] = P.l;
                 }
                 if (lane == 0) {
                     a.cstate[i] = P.nv;
@@ -2214,7 +2214,7 @@ __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a,
         if constexpr (EXACT)
             acc = integrate_cell(S, nv, splat_geo(g, a, S, nv, i, lane), si, lane);
         else if (lane < nv)
-            a.rbuf[(size_t)i * COT_RCAP + lane] = make_double2(P.x, P.y);
+            a.rbuf[ring_at(i, lane)] = make_double2(P.x, P.y);
         if constexpr (!EXACT && LPC == 32) {
             // a cell whose pixel box is large goes on the heavy list: the
             // integration kernel starts those cells first, so that they run
@@ -2240,7 +2240,7 @@ __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a,
         }
         // the Newton solve's Jacobian reads the final ring's generators
         if constexpr (KEEP) {
-            if (lane < nv) a.lbuf[(size_t)i * COT_RCAP + lane] = P.l;
+            if (lane < nv) a.lbuf[ring_at(i, lane)] = P.l;
         }
     }
     PSTAT_CLOCK(t3);
@@ -2359,7 +2359,10 @@ __global__ void __launch_bounds__(128, MINB) k_cells_fast(const __grid_constant_
 // side_line as the clips used, so the same bits) and runs phases 2 and 3.
 // Cells that phase 1 empties or overflows are finished by k_cells_first
 // (cstate < 0); otherwise cstate = nv, plus CST_CACHED for a cached cell.
+// Both work the cells of flist where the kernels below have taken the others,
+// else every cell.
 #define CST_CACHED 0x100
+#define CST_FAST 0x200  // k_rings_cached has the ring, k_certify is to prove it
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) k_cells_first(CotGeo g, CellsArgs a)
 {
@@ -2369,11 +2372,13 @@ __global__ void __launch_bounds__(128, MINB) k_cells_first(CotGeo g, CellsArgs a
     PSTAT_INIT();
     const int lane = threadIdx.x & 31;
     int *fetch = a.ovf_count + 1;
+    const int total = a.flist != nullptr ? a.ovf_count[14] : g.n;
     while (true) {
         int i = 0;
         if (lane == 0) i = atomicAdd(fetch, 1);
         i = __shfl_sync(FULLMASK, i, 0);
-        if (i >= g.n) break;
+        if (i >= total) break;
+        if (a.flist != nullptr) i = a.flist[i];
         const double2 si = g.xy[i];
         const double wi = a.wt[i];
         bool cached = false;
@@ -2384,8 +2389,8 @@ __global__ void __launch_bounds__(128, MINB) k_cells_first(CotGeo g, CellsArgs a
             if (lane == 0) a.cstate[i] = -1;
         } else {
             if (lane < P.nv) {
-                a.rbuf[(size_t)i * COT_RCAP + lane] = make_double2(P.x, P.y);
-                a.lbuf[(size_t)i * COT_RCAP + lane] = P.l;
+                a.rbuf[ring_at(i, lane)] = make_double2(P.x, P.y);
+                a.lbuf[ring_at(i, lane)] = P.l;
             }
             if (lane == 0) a.cstate[i] = P.nv | (cached ? CST_CACHED : 0);
         }
@@ -2433,7 +2438,7 @@ __global__ void __launch_bounds__(128, MINB) k_bucket_walk(CotGeo g, CellsArgs a
             // P_i0 - P_i at s_i + v: (w_i0 - w_i)/2 - |e|^2/2 - v.e, e = s_i - s_i0
             const double k0 = 0.5 * (wo - a.wt[i]) - 0.5 * __fma_rn(ex, ex, ey * ey);
             for (int k = 0; k < nv; k++) {
-                const double2 v = a.rbuf[(size_t)i * COT_RCAP + k];
+                const double2 v = a.rbuf[ring_at(i, k)];
                 const double X = v.x + ex, Y = v.y + ey;
                 lx = fmin(lx, X);
                 hx = fmax(hx, X);
@@ -2506,6 +2511,251 @@ __global__ void __launch_bounds__(128, MINB) k_bucket_walk(CotGeo g, CellsArgs a
     }
 }
 
+// ---------------------------------------------------------------------------
+// a few lanes a cell: the cells whose last ring still stands
+// ---------------------------------------------------------------------------
+// Most cells of a warm evaluation keep the ring of the last one: the same
+// generators in the same order, moved.  Rebuilding such a ring and proving
+// that no other site cuts it takes a warp a cell 1,650 instructions with 6 to
+// 24 lanes busy.  k_rings_cached gives a cell 8 lanes, one an edge, and
+// k_certify 4 or 8 lanes that share its leaves and sites.  Every other cell
+// (no ordered cache, a ring that fails, a site that cuts) is listed for
+// k_cells_first and k_cells_walk.  The lines, vertices and final tests are
+// those of the warp kernels in the same explicitly rounded forms, so a cell
+// has the same bits whichever took it.
+// At 262,144 sites (us): k_cells_first 217 -> 43 + 17 for the cells left to
+// it, k_cells_walk 423 -> 143 + 43, latency of dependent loads and double
+// precision chains the bound (360 warp instructions a cell, 60 % issued).
+#define FAST_THREADS 128
+#define FAST_NV 8      // largest ring of these kernels
+#define FAST_LEFT 12   // leaves whose sites k_certify looks through (3.6 on average)
+#define FAST_CAND 10    // sites near the ring that one lane may have to test in full
+
+// Appends i to list for the threads with `want`, one counter update a warp.
+__device__ __forceinline__ void warp_append(bool want, int i, int *list, int *count)
+{
+    const unsigned m = __ballot_sync(FULLMASK, want);
+    if (m == 0u) return;
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == __ffs(m) - 1) base = atomicAdd(count, __popc(m));
+    base = __shfl_sync(FULLMASK, base, __ffs(m) - 1);
+    if (want) list[base + __popc(m & ((1u << lane) - 1u))] = i;
+}
+
+// ring_try for the cells with an ordered cache of at most FAST_NV generators,
+// a lane an edge: vertex k is where the lines of edges k-1 and k meet;
+// accepted when every vertex lies inside every other line and the domain,
+// every edge runs forward and every corner turns left.  Accepted rings go to
+// the ring buffers with CST_FAST, the other cells to flist.
+__global__ void __launch_bounds__(FAST_THREADS) k_rings_cached(const __grid_constant__ CotGeo g, CellsArgs a)
+{
+    __shared__ double2 LAB[FAST_THREADS];
+    __shared__ double LC[FAST_THREADS];
+    const int sl = threadIdx.x & 7, t0 = threadIdx.x & ~7;
+    const int i = (blockIdx.x * FAST_THREADS + threadIdx.x) >> 3;
+    int m = i < g.n ? a.nbn[i] : 0;
+    if (m < 3 || m > FAST_NV) m = 0;
+    const bool act = sl < m;
+    bool ok = m > 0;
+    double la = 0.0, lb = 0.0, lc = 0.0, vx = 0.0, vy = 0.0;
+    int lab = 0;
+    double4 box = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (act) {
+        lab = a.nbc[(size_t)i * COT_NBC + sl];
+        const double2 si = g.xy[i];
+        box = make_double4(g.pd[0] - si.x, g.pd[1] - si.x, g.pd[2] - si.y, g.pd[3] - si.y);
+        double key;
+        if (lab >= 0) site_line(g.xy[lab], si, a.wt[lab], a.wt[i], la, lb, lc, key);
+        else side_line(-lab - 1, box, la, lb, lc);
+    }
+    LAB[threadIdx.x] = make_double2(la, lb);
+    LC[threadIdx.x] = lc;
+    __syncwarp();
+    if (act) {
+        const int pv = sl == 0 ? m - 1 : sl - 1;
+        const double2 pab = LAB[t0 + pv];
+        ok = line_meet(pab.x, pab.y, LC[t0 + pv], la, lb, lc, vx, vy);
+        for (int j = 0; j < m; j++) {
+            const double2 jab = LAB[t0 + j];
+            if (j != sl && j != pv && side(jab.x, jab.y, LC[t0 + j], vx, vy) > 0.0) ok = false;
+        }
+        // domain sides that the cell now reaches
+        if (vx < box.x || vx > box.y || vy < box.z || vy > box.w) ok = false;
+    }
+    const int nx = act && sl + 1 < m ? sl + 1 : 0;
+    const double nvx = __shfl_sync(FULLMASK, vx, nx, 8), nvy = __shfl_sync(FULLMASK, vy, nx, 8);
+    if (act) {
+        // edge k along (-b, a) from vertex k to the next, and the corner after it
+        const double2 nab = LAB[t0 + nx];
+        if (!(__fma_rn(nvx - vx, -lb, __dmul_rn(nvy - vy, la)) > 0.0)) ok = false;
+        if (!(__fma_rn(-lb, nab.x, __dmul_rn(la, nab.y)) > 0.0)) ok = false;
+    }
+    const bool whole = ((__ballot_sync(FULLMASK, ok) >> (threadIdx.x & 24)) & 0xffu) == 0xffu;
+    if (whole && act) {
+        a.rbuf[ring_at(i, sl)] = make_double2(vx, vy);
+        a.lbuf[ring_at(i, sl)] = lab;
+        if (sl == 0) a.cstate[i] = m | CST_CACHED | CST_FAST;
+    }
+    warp_append(i < g.n && !whole && sl == 0, i, a.flist, a.ovf_count + 14);
+}
+
+// The certificate of the CST_FAST cells against their bucket's leaf list
+// (k_bucket_walk), G lanes a cell: lane s tests every G-th listed leaf against
+// the ring, then every G-th site of the leaves that are left.  A site is
+// dropped when its line stays beyond the ring's circumscribed disk; what is
+// left (the ring's own generators and a few more) is tested against every
+// vertex at the end.  A cell that no site cuts is finished here as
+// cell_finish would (its cache stays as it is); the others with a ring go to
+// flist.
+//
+// The leaf test is node_excluded's in single precision about the disk's
+// centre m, on the safe side: with v = m + u and t = v + a it reads
+// |m + a|^2 + C + 2 (m + a).u + |u|^2 <= dist(m + p + u, box)^2, where the
+// constant is taken in double precision and everything else is of the size of
+// the ring; a margin of 1e-6 of the terms' magnitudes (16 roundings) covers
+// the rest, so a leaf is kept that could be dropped, never the reverse.
+template <int G>
+__global__ void __launch_bounds__(FAST_THREADS) k_certify(const __grid_constant__ CotGeo g, CellsArgs a)
+{
+    constexpr int CELLS = FAST_THREADS / G;
+    __shared__ double2 V[CELLS][FAST_NV];
+    __shared__ float4 U[CELLS][FAST_NV];
+    __shared__ int CAND[FAST_CAND][FAST_THREADS];
+    const int sl = threadIdx.x & (G - 1), tc = threadIdx.x / G;
+    const unsigned gshift = threadIdx.x & 31 & ~(G - 1);
+    const int i = blockIdx.x * CELLS + tc;
+    const int st = i < g.n ? a.cstate[i] : -1;
+    const int bi = st >= 0 ? g.sbucket[i] : 0;
+    int bc = st >= 0 && (st & CST_FAST) != 0 ? a.bcnt[bi] : -1;
+    bool ok = bc >= 0;
+    if (!ok) bc = 0;
+    const int m = ok ? st & 0xff : 0;
+    double2 si = make_double2(0.0, 0.0);
+    double wi = 0.0;
+    double x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
+    if (ok) {
+        si = g.xy[i];
+        wi = a.wt[i];
+        for (int k = sl; k < m; k += G) {
+            const double2 v = a.rbuf[ring_at(i, k)];
+            V[tc][k] = v;
+            x0 = fmin(x0, v.x);
+            x1 = fmax(x1, v.x);
+            y0 = fmin(y0, v.y);
+            y1 = fmax(y1, v.y);
+        }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        x0 = fmin(x0, __shfl_xor_sync(FULLMASK, x0, o));
+        x1 = fmax(x1, __shfl_xor_sync(FULLMASK, x1, o));
+        y0 = fmin(y0, __shfl_xor_sync(FULLMASK, y0, o));
+        y1 = fmax(y1, __shfl_xor_sync(FULLMASK, y1, o));
+    }
+    if (!ok) x0 = x1 = y0 = y1 = 0.0;
+    const double mx = 0.5 * (x0 + x1), my = 0.5 * (y0 + y1);
+    // the disk's radius, widened by far more than the roundings of the tests
+    float ru = 0.0f;
+    for (int k = sl; k < m; k += G) {
+        const float ux = (float)(V[tc][k].x - mx), uy = (float)(V[tc][k].y - my);
+        const float u2 = ux * ux + uy * uy;
+        U[tc][k] = make_float4(ux, uy, u2, __int_as_float(a.lbuf[ring_at(i, k)]));
+        ru = fmaxf(ru, u2);
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) ru = fmaxf(ru, __shfl_xor_sync(FULLMASK, ru, o));
+    ru = sqrtf(ru) * 1.00001f;
+    const double rr = (double)ru + 1e-13 * (fabs(mx) + fabs(my));
+    const double r2 = rr * rr;
+    __syncwarp();
+    // the listed leaves that can hold a cutting site
+    const int *__restrict__ leaves = a.blist + (size_t)bi * COT_BLEAF;
+    unsigned long long left = 0ull;
+    const int rounds = (int)__reduce_max_sync(FULLMASK, (unsigned)(bc + G - 1) / G);
+    for (int q = 0; q < rounds; q++) {
+        const int e = q * G + sl;
+        bool keep = false;
+        if (e < bc) {
+            const int node = leaves[e];
+            const double4 ts = g.tstat[node];
+            const double4 td = g.tdyn[node];
+            const double tx = mx + td.x, ty = my + td.y;
+            const double c0 = __fma_rn(tx, tx, __fma_rn(ty, ty, 2.0 * (si.x * td.x + si.y * td.y + td.z + g.margin) - wi));
+            const float bx = (float)(2.0 * tx), by = (float)(2.0 * ty);
+            const float qx = (float)(mx + si.x - ts.x + td.x), qy = (float)(my + si.y - ts.y + td.y);
+            const float hx = (float)ts.z, hy = (float)ts.w;
+            const float far = fabsf(qx) + fabsf(qy) + hx + hy + ru;
+            const float c = (float)c0;
+            const float cm = c + 1e-6f * (fabsf(c) + (fabsf(bx) + fabsf(by)) * ru + far * far);
+            for (int k = 0; k < m; k++) {
+                const float4 u = U[tc][k];
+                const float ex = fmaxf(fabsf(qx + u.x) - hx, 0.0f), ey = fmaxf(fabsf(qy + u.y) - hy, 0.0f);
+                if (!(fmaf(bx, u.x, fmaf(by, u.y, cm + u.z)) <= fmaf(ex, ex, ey * ey))) {
+                    keep = ts.z >= 0.0;
+                    break;
+                }
+            }
+        }
+        const unsigned long long kb = (__ballot_sync(FULLMASK, keep) >> gshift) & ((1u << G) - 1u);
+        left |= kb << (q * G);
+    }
+    // their sites
+    int nc = 0;
+    if (__popcll(left) > FAST_LEFT) {
+        ok = false;
+        left = 0ull;
+    }
+    while (left != 0ull) {
+        const int b = leaves[__ffsll((long long)left) - 1];
+        left &= left - 1ull;
+        const int end = g.bstart[b + 1];
+        for (int j = g.bstart[b] + sl; j < end; j += G) {
+            double la, lb, lc, key;
+            site_line(g.xy[j], si, a.wt[j], wi, la, lb, lc, key);
+            const double d = lc - (la * mx + lb * my);
+            if (!(d > 0.0 && d * d > key * r2) && j != i) {
+                if (nc < FAST_CAND) CAND[nc][threadIdx.x] = j;
+                nc++;
+            }
+        }
+    }
+    if (nc > FAST_CAND) ok = false;
+    for (int q = 0; q < nc && ok; q++) {
+        const int j = CAND[q][threadIdx.x];
+        bool mine = false;
+        for (int k = 0; k < m; k++) mine = mine || __float_as_int(U[tc][k].w) == j;
+        if (mine) continue;
+        double la, lb, lc, key;
+        site_line(g.xy[j], si, a.wt[j], wi, la, lb, lc, key);
+        for (int k = 0; k < m; k++)
+            if (side(la, lb, lc, V[tc][k].x, V[tc][k].y) > 0.0) ok = false;
+    }
+    ok = ((__ballot_sync(FULLMASK, ok) >> gshift) & ((1u << G) - 1u)) == (1u << G) - 1u;
+    if (ok && sl == 0) {
+        // cell_finish
+        int state = st;
+        if (a.hlist != nullptr) {
+            const double ox = si.x - g.pd[0], oy = si.y - g.pd[2];
+            const double pix = (floor((ox + x1) * g.ixs) - floor((ox + x0) * g.ixs) + 1.0) *
+                               (floor((oy + y1) * g.iys) - floor((oy + y0) * g.iys) + 1.0);
+            if (pix > (double)COT_HEAVY_PIX) {
+                int slot = a.hsplit_cap;
+                if (pix > (double)COT_SPLIT_PIX && a.hsplit != nullptr) slot = atomicAdd(a.ovf_count + 13, 1);
+                if (slot < a.hsplit_cap) a.hsplit[slot] = i;
+                else a.hlist[atomicAdd(a.ovf_count + 10, 1)] = i;
+                state = CST_HEAVY;
+            }
+        }
+        a.cstate[i] = state;
+        a.nv[i] = m;
+    }
+    warp_append(st >= 0 && !ok && sl == 0, i, a.flist, a.ovf_count + 15);
+}
+
+static_assert(FAST_NV <= COT_SEG_NV, "rings of these kernels fit the 8-lane integration");
+static_assert(COT_BLEAF <= 64, "a mask bit a listed leaf");
+
 // KEEP: leave the final ring's generators in lbuf (the Newton solve's
 // Jacobian reads them); a separate instance keeps the solve's path as it is.
 template <int MINB, bool KEEP>
@@ -2517,11 +2767,13 @@ __global__ void __launch_bounds__(128, MINB) k_cells_walk(const __grid_constant_
     PSTAT_INIT();
     const int lane = threadIdx.x & 31;
     int *fetch = a.ovf_count + 8;
+    const int total = a.flist != nullptr ? a.ovf_count[15] : g.n;
     while (true) {
         int i = 0;
         if (lane == 0) i = atomicAdd(fetch, 1);
         i = __shfl_sync(FULLMASK, i, 0);
-        if (i >= g.n) break;
+        if (i >= total) break;
+        if (a.flist != nullptr) i = a.flist[i];
         const int st = a.cstate[i];
         if (st < 0) continue;
         const double2 si = g.xy[i];
@@ -2531,10 +2783,10 @@ __global__ void __launch_bounds__(128, MINB) k_cells_walk(const __grid_constant_
         P.x = P.y = P.a = P.b = P.c = 0.0;
         P.l = 0;
         if (lane < P.nv) {
-            const double2 v = a.rbuf[(size_t)i * COT_RCAP + lane];
+            const double2 v = a.rbuf[ring_at(i, lane)];
             P.x = v.x;
             P.y = v.y;
-            P.l = a.lbuf[(size_t)i * COT_RCAP + lane];
+            P.l = a.lbuf[ring_at(i, lane)];
             if (P.l >= 0) {
                 double key;
                 site_line(g.xy[P.l], si, a.wt[P.l], wi, P.a, P.b, P.c, key);
@@ -2661,10 +2913,10 @@ __global__ void __launch_bounds__(32 * HEAVY_WARPS, 2) k_cells_heavy(const __gri
             P.x = P.y = P.a = P.b = P.c = 0.0;
             P.l = 0;
             if (lane < P.nv) {
-                const double2 v = a.rbuf[(size_t)i * COT_RCAP + lane];
+                const double2 v = a.rbuf[ring_at(i, lane)];
                 P.x = v.x;
                 P.y = v.y;
-                P.l = a.lbuf[(size_t)i * COT_RCAP + lane];
+                P.l = a.lbuf[ring_at(i, lane)];
                 if (P.l >= 0) {
                     double key;
                     site_line(g.xy[P.l], si, a.wt[P.l], wi, P.a, P.b, P.c, key);
@@ -2849,7 +3101,7 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
             const int i = a.hsplit[slot];
             const int nv = a.nv[i];
             if (lane < nv) {
-                const double2 v = a.rbuf[(size_t)i * COT_RCAP + lane];
+                const double2 v = a.rbuf[ring_at(i, lane)];
                 S.X[lane] = v.x;
                 S.Y[lane] = v.y;
             }
@@ -2893,7 +3145,7 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
             double mu = 0.0, fcv = 0.0;
             if (nv >= 3) {
                 if (lane < nv) {
-                    const double2 v = a.rbuf[(size_t)i * COT_RCAP + lane];
+                    const double2 v = a.rbuf[ring_at(i, lane)];
                     S.X[lane] = v.x;
                     S.Y[lane] = v.y;
                 }
@@ -2922,7 +3174,7 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
             const int m = nv >= 3 ? nv : 0;
             double2 si = make_double2(0.0, 0.0);
             if (m > 0) si = g.xy[i];
-            for (int k = sl; k < m; k += L) T.V[k] = a.rbuf[(size_t)i * COT_RCAP + k];
+            for (int k = sl; k < m; k += L) T.V[k] = a.rbuf[ring_at(i, k)];
             __syncwarp();
             const CellAcc acc = integrate_walk(T, m, pix_geo(g), si);
             if (sl == 0 && nv >= 0) {
@@ -3162,8 +3414,8 @@ __global__ void __launch_bounds__(128, MINB) k_cells(CotGeo g, CellsArgs a, int 
             // longer one has its row built here
             if (nv <= COT_RCAP) {
                 if (lane < nv) {
-                    a.rbuf[(size_t)i * COT_RCAP + lane] = make_double2(P.X[lane], P.Y[lane]);
-                    a.lbuf[(size_t)i * COT_RCAP + lane] = P.L[lane];
+                    a.rbuf[ring_at(i, lane)] = make_double2(P.X[lane], P.Y[lane]);
+                    a.lbuf[ring_at(i, lane)] = P.L[lane];
                 }
             } else if (a.hbig_val != nullptr) {
                 int slot = 0;
@@ -3271,6 +3523,19 @@ static size_t cells_smem(int maxv, int warps)
 #ifndef COT_SEG_MIN_N
 #define COT_SEG_MIN_N 4096
 #endif
+// Sites from which the cells whose last ring stands take a few lanes each
+// (k_rings_cached, k_certify), and up to which k_certify takes 8 of them: its
+// two launches cost about what they save at 16,384 sites, and below 8 lanes
+// fill the GPU better.  Two evaluations (us; warp a cell, 8 lanes, 4 lanes):
+// 12,100 sites 348 347 367, 16,384 361 358 369, 20,736 412 386 399,
+// 26,896 447 415 418, 36,100 518 457 455, 65,536 699 555 556,
+// 262,144 2055 1327 1288.
+#ifndef COT_FAST_MIN_N
+#define COT_FAST_MIN_N 16384
+#endif
+#ifndef COT_FAST_G8_N
+#define COT_FAST_G8_N 40000
+#endif
 static int g_blocks_per_sm32 = 0, g_blocks_per_sm16 = 0, g_blocks_per_sm8 = 0, g_blocks_per_smi = 0;
 static int g_blocks_per_smf = 0, g_blocks_per_smw = 0, g_blocks_per_smb = 0;
 
@@ -3298,9 +3563,10 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     // integration kernel's fetch counter, [8]: k_cells_walk's fetch counter,
     // [9]: k_bucket_walk's, [10]: the heavy integration list's size, [11]:
     // the overflowed walks' list size, [12]: k_cells_heavy's fetch counter,
-    // [13]: the split integration list's size
+    // [13]: the split integration list's size, [14], [15]: flist's sizes for
+    // k_cells_first and k_cells_walk
     const int segs = (nb * BSEG + 127) / 128;
-    k_bucket_phi<<<segs, 128, 0, s>>>(g, a.w, a.d, a.tptr, a.wt, a.wbar, a.ovf_count, 14);
+    k_bucket_phi<<<segs, 128, 0, s>>>(g, a.w, a.d, a.tptr, a.wt, a.wbar, a.ovf_count, 16);
     k_tree_build<<<(nb * BSEG + TREE_THREADS - 1) / TREE_THREADS, TREE_THREADS, 0, s>>>(g, a.wt, a.wbar);
     c.launches += 2;
     int upper = 0;  // nodes of levels 1..lmax
@@ -3336,10 +3602,26 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
         const int bw = std::min(g.n, sms * (g_blocks_per_smw > 0 ? g_blocks_per_smw : WALK_MINB) * CELLS_WPB);
         const int bf = std::min(g.n, sms * (g_blocks_per_smf > 0 ? g_blocks_per_smf : FIRST_MINB) * CELLS_WPB);
         const size_t sm = sizeof(FastScratch) * CELLS_WPB;
+        // a thread a cell for the cells whose last ring still stands: not for
+        // a ring dump (written by k_cells_walk)
+        const bool fast = g.n >= COT_FAST_MIN_N && a.flist != nullptr && a.nbn != nullptr && a.bcnt != nullptr &&
+                          a.ring_xy == nullptr;
+        if (!fast) a.flist = nullptr;
+        if (fast) {
+            k_rings_cached<<<(g.n + FAST_THREADS / 8 - 1) / (FAST_THREADS / 8), FAST_THREADS, 0, s>>>(g, a);
+            c.launches++;
+        }
         k_cells_first<FIRST_MINB><<<(bf + CELLS_WPB - 1) / CELLS_WPB, 32 * CELLS_WPB, sm, s>>>(g, a);
         if (a.bcnt != nullptr) {
             const int bb = std::min(nb, sms * (g_blocks_per_smb > 0 ? g_blocks_per_smb : WALK_MINB) * CELLS_WPB);
             k_bucket_walk<WALK_MINB><<<(bb + CELLS_WPB - 1) / CELLS_WPB, 32 * CELLS_WPB, sm, s>>>(g, a);
+            c.launches++;
+        }
+        if (fast) {
+            if (g.n <= COT_FAST_G8_N)
+                k_certify<8><<<(g.n + FAST_THREADS / 8 - 1) / (FAST_THREADS / 8), FAST_THREADS, 0, s>>>(g, a);
+            else
+                k_certify<4><<<(g.n + FAST_THREADS / 4 - 1) / (FAST_THREADS / 4), FAST_THREADS, 0, s>>>(g, a);
             c.launches++;
         }
         if (a.keep_labels)

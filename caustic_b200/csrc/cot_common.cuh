@@ -122,6 +122,15 @@ struct CotCtx {
     int ev_used = 0;
 };
 
+// Vertex k of cell i in the ring buffers: tiles of 32 cells, a row per vertex,
+// so that a thread a cell reads and writes whole rows and a warp of four cells
+// a few sectors a row.
+__host__ __device__ __forceinline__ size_t ring_at(int i, int k)
+{
+    return ((size_t)(i >> 5) << 10) + (size_t)((k << 5) + (i & 31));
+}
+inline size_t ring_entries(size_t n) { return (n + 31) / 32 * 1024; }
+
 // Launchers implemented in cot_cells.cu.
 struct CellsArgs {
     const double *w;       // weights (base point)
@@ -150,8 +159,10 @@ struct CellsArgs {
     double solid_light[3]; // light position
     double *splat;         // render output, nx*ny (nullable)
     double splat_scale;    // gray_multiple of the render
-    double2 *rbuf;         // ring vertices of the solve's path, 32 per cell
-    int *lbuf;             // their edge generators between k_cells_first and k_cells_walk
+    double2 *rbuf;         // ring vertices of the solve's path, at ring_at(cell, vertex)
+    int *lbuf;             // their edge generators between the ring kernels
+    int *flist;            // cells that the thread-per-cell ring kernels leave to the others
+                           // (two-kernel path only; nullable)
     int *cstate;           // per cell: ring size (+ cached flag) after phase 1, -1 = finished
     double *ring_xy;       // optional fixed-stride ring dump (nullable)
     int *ring_lab;

@@ -56,10 +56,10 @@ __global__ void __launch_bounds__(HESS_THREADS) k_hessian(CotGeo g, const double
     double a = 0.0;
     int j = -1;
     if (lane < m) {
-        j = lbuf[(size_t)i * 32 + lane];
+        j = lbuf[ring_at(i, lane)];
         if (j >= 0) {
-            const double2 p = rbuf[(size_t)i * 32 + lane];
-            const double2 q = rbuf[(size_t)i * 32 + (lane + 1 == m ? 0 : lane + 1)];
+            const double2 p = rbuf[ring_at(i, lane)];
+            const double2 q = rbuf[ring_at(i, lane + 1 == m ? 0 : lane + 1)];
             const double2 sj = g.xy[j];
             const double ex = sj.x - si.x, ey = sj.y - si.y;
             a = edge_rho_integral(g, si.x + p.x, si.y + p.y, si.x + q.x, si.y + q.y) / (2.0 * sqrt(ex * ex + ey * ey));

@@ -1,0 +1,48 @@
+"""Cells rebuilt from the last evaluation's ring and certified by a few lanes
+(problems of at least 16,384 sites): the bits of an evaluation without a
+cache, whichever cells the short path takes."""
+import numpy as np
+import pytest
+
+from caustic_b200 import capi, problems
+from test_gpu_parity import check_eval, solver_for
+
+pytestmark = pytest.mark.gpu
+
+
+# 8 lanes a cell and 4; sizes that leave a part of a block and of a tile of
+# cells, and the last one below the short path
+@pytest.mark.parametrize("gx,gy", [(128, 128), (141, 129), (223, 187), (131, 125)])
+def test_cached_evaluation_has_the_bits_of_a_cold_one(gpu, gx, gy):
+    rng = np.random.default_rng(gx)
+    xy = problems.jittered_grid(rng, gx, gy)
+    n = gx * gy
+    nu = rng.uniform(0.5, 1.5, n)
+    pic = problems.gaussian_mixture(rng, 6, 333, 290)
+    p = problems.SDOTProblem("cached", xy, nu / nu.sum(), pic, (333, 290))
+    s = solver_for(p)
+    base = 0.3 / n * np.sin(7 * xy[:, 0]) * np.cos(5 * xy[:, 1]) * np.sqrt(n)
+    w = base + rng.normal(0.0, 0.05 / n, n)
+    # nothing moves, a few rings change, most change, cells hide and return
+    for amp in (0.0, 0.01, 0.3, 3.0, 0.0):
+        w = w + rng.normal(0.0, amp / n, n)
+        f, mu, g, fc = s.eval(w)
+        fresh = solver_for(p)
+        f0, mu0, g0, fc0 = fresh.eval(w)
+        assert np.array_equal(mu, mu0) and np.array_equal(fc, fc0) and f == f0, amp
+        fresh.close()
+    check_eval(p, base, s)
+
+
+def test_jacobian_of_cached_rings(gpu):
+    """The rows of cells finished by the short path: k_hessian reads their
+    generators where k_rings_cached left them."""
+    p = problems.make(4, g=129, res=200)
+    rng = np.random.default_rng(3)
+    w = rng.normal(0.0, 0.05 / p.n, p.n)
+    warm = solver_for(p)
+    warm.eval(w)
+    warm.eval(w + rng.normal(0.0, 0.01 / p.n, p.n))
+    a, b = warm.mass_jacobian(w), solver_for(p).mass_jacobian(w)
+    assert np.array_equal(a.indptr, b.indptr) and np.array_equal(a.indices, b.indices)
+    assert np.array_equal(a.data, b.data)
