@@ -1710,7 +1710,7 @@ static int newton_alloc(cot_handle *h)
     A((void **)&P.nb_pa, N * 8);
     A((void **)&P.nb_pb, N * 8);
     A((void **)&P.nb_q, N * 8);
-    A((void **)&P.nb_part, (size_t)std::max(4 * pcg_blocks, 256 * 5) * 8);
+    A((void **)&P.nb_part, (size_t)std::max(6 * pcg_blocks + 48, 256 * 5) * 8);
     A((void **)&P.nb_tau, 8);
     A((void **)&P.pcg, sizeof(PcgState));
     A((void **)&P.nst, sizeof(NewtonEvalStats));

@@ -244,9 +244,8 @@ struct NewtonEvalStats {
 };
 struct PcgState {
     int iterations;
-    int error;       // a grid barrier gave up waiting
+    int error;       // a block gave up waiting for the others
     double rr0, rr;  // squared residual norms at the start and the end
-    unsigned int bar_count, bar_gen;
 };
 void launch_hessian(const CotGeo &g, const double2 *rbuf, const int *lbuf, const int *nv, double *hval, int *hcol,
                     int *hcnt, double *hdiag, CotCtx &c);
