@@ -407,7 +407,7 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
         A((void **)&P.ovf_count, 16 * sizeof(int));
         A((void **)&P.wlist, N * sizeof(int));
         A((void **)&P.hsplit, COT_HSPLIT_CAP * sizeof(int));
-        A((void **)&P.hpart, (size_t)COT_HSPLIT_CAP * COT_SPLIT * 4 * sizeof(double));
+        A((void **)&P.hpart, (size_t)COT_HSPLIT_CAP * COT_SPLIT * COT_PART * sizeof(double));
         A((void **)&P.hticket, COT_HSPLIT_CAP * sizeof(unsigned int));
         A((void **)&P.nbc, N * COT_NBC * sizeof(int));
         A((void **)&P.nbn, N * sizeof(int));

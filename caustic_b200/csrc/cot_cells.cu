@@ -703,9 +703,80 @@ __device__ PixGeo splat_geo(const CotGeo &g, const CellsArgs &a, const SP &P, in
     return p;
 }
 
-// Integrate the density over the cell (polygon relative to site si).
+// Integrals of one pixel [x0, x1] x [y0, y1] (column c of the scratch's strip
+// tables) and what they add to the cell's sums.  MASKED: only the edges set in
+// `edges` can meet the pixel.
+template <bool MASKED, class SP>
+__device__ __forceinline__ void pixel_sums(const SP &P, int nv, unsigned edges, int c, int ix, int iy, double x0,
+                                           double x1, double y0, double y1, const PixGeo &g, CellAcc &s)
+{
+    double xc = 0.5 * (x0 + x1), yc = 0.5 * (y0 + y1);
+    double hxp = 0.5 * (x1 - x0), hyp = 0.5 * (y1 - y0);
+    Mom m = {0.0, 0.0, 0.0, 0.0};
+    bool full = P.rv[c] && P.lv[c + 1] && P.elo[c] <= y0 && P.ehi[c] >= y1 && P.elo[c + 1] <= y0 &&
+                P.ehi[c + 1] >= y1;
+    if (full) {
+        m.A = 4.0 * hxp * hyp;
+        m.I2 = m.A * (hxp * hxp + hyp * hyp) * (1.0 / 3.0);
+    } else {
+        for (int k = 0; MASKED ? edges != 0u : k < nv; k++) {
+            if constexpr (MASKED) {
+                k = __ffs(edges) - 1;
+                edges &= edges - 1u;
+            }
+            int kn = (k + 1 == nv) ? 0 : k + 1;
+            double px = P.X[k], py = P.Y[k], qx = P.X[kn], qy = P.Y[kn];
+            if (px == qx && (px == x0 || px == x1)) continue;  // counted by the pixel side
+            if (fmax(px, qx) < x0 || fmin(px, qx) > x1 || fmax(py, qy) < y0 || fmin(py, qy) > y1) continue;
+            // Liang-Barsky against the pixel box (reciprocals precomputed)
+            double dx = qx - px, dy = qy - py, t0 = 0.0, t1 = 1.0;
+            if (dx != 0.0) {
+                double ta = (x0 - px) * P.EIX[k], tb = (x1 - px) * P.EIX[k];
+                t0 = fmax(t0, fmin(ta, tb));
+                t1 = fmin(t1, fmax(ta, tb));
+            } else if (px < x0 || px > x1) {
+                continue;
+            }
+            if (dy != 0.0) {
+                double ta = (y0 - py) * P.EIY[k], tb = (y1 - py) * P.EIY[k];
+                t0 = fmax(t0, fmin(ta, tb));
+                t1 = fmin(t1, fmax(ta, tb));
+            } else if (py < y0 || py > y1) {
+                continue;
+            }
+            if (!(t0 < t1)) continue;
+            double ax0 = (t0 == 0.0 ? px : px + t0 * dx) - xc;
+            double by0 = (t0 == 0.0 ? py : py + t0 * dy) - yc;
+            double ax1 = (t1 == 1.0 ? qx : px + t1 * dx) - xc;
+            double by1 = (t1 == 1.0 ? qy : py + t1 * dy) - yc;
+            seg_terms(ax0, by0, ax1, by1, m);
+        }
+        if (P.lv[c + 1]) {  // right side, upwards
+            double b0 = fmax(P.elo[c + 1], y0), b1 = fmin(P.ehi[c + 1], y1);
+            if (b1 > b0) vside_terms(x1 - xc, b0 - yc, b1 - yc, m);
+        }
+        if (P.rv[c]) {      // left side, downwards
+            double b0 = fmax(P.elo[c], y0), b1 = fmin(P.ehi[c], y1);
+            if (b1 > b0) vside_terms(x0 - xc, b1 - yc, b0 - yc, m);
+        }
+    }
+    if (!(m.A > 0.0)) return;
+    if (g.splat != nullptr) atomicAdd(g.splat + ix + iy * g.nx, g.splat_w * m.A);
+    double rho = g.rho[ix + iy * g.nx];
+    s.mu += rho * m.A;
+    s.S += rho * (m.A * (xc * xc + yc * yc) + 2.0 * (xc * m.Ia + yc * m.Ib) + m.I2);
+    if (m.A > 1e-10) {  // compute_center skips tiny pieces (basic_function.cuh:1153)
+        s.Mt += rho * m.A;
+        s.Mx += rho * (m.A * xc + m.Ia);
+        s.My += rho * (m.A * yc + m.Ib);
+    }
+}
+
+// Integrate the density over the cell (polygon relative to site si); with
+// nparts > 1 over every nparts-th row of its pixels, from row `part`.
 template <class SP>
-__device__ __noinline__ CellAcc integrate_cell(SP &P, int nv, const PixGeo g, double2 si, int lane)
+__device__ __noinline__ CellAcc integrate_cell(SP &P, int nv, const PixGeo g, double2 si, int lane, int part = 0,
+                                               int nparts = 1)
 {
     PSTAT_LPC32;
     CellAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -740,7 +811,7 @@ __device__ __noinline__ CellAcc integrate_cell(SP &P, int nv, const PixGeo g, do
     if (hx <= lx || hy <= ly) return acc;
     PSTAT_ADD(6, (hx - lx) * (hy - ly));
     const double pminx = mnx, pmaxx = mxx;
-    double mu = 0.0, S = 0.0, Mt = 0.0, Mx = 0.0, My = 0.0;
+    CellAcc sum = {0.0, 0.0, 0.0, 0.0, 0.0};
     for (int cx0 = lx; cx0 < hx; cx0 += 32) {
         int cw = min(32, hx - cx0);
         // column lines cx0 .. cx0+cw
@@ -769,10 +840,10 @@ __device__ __noinline__ CellAcc integrate_cell(SP &P, int nv, const PixGeo g, do
             P.shi[c] = hi;
         }
         __syncwarp();
-        int rows = hy - ly;
+        int rows = (hy - ly - part + nparts - 1) / nparts;
         int npx = cw * rows;
         for (int p = lane; p < npx; p += 32) {
-            int c = p % cw, r = p / cw;
+            int c = p % cw, r = part + nparts * (p / cw);
             int ix = cx0 + c, iy = ly + r;
             // pixel box exactly as basic_function.cuh:806-809, relative to the site
             double x0 = (double)ix * g.xs + g.pd0 - si.x;
@@ -780,79 +851,24 @@ __device__ __noinline__ CellAcc integrate_cell(SP &P, int nv, const PixGeo g, do
             double y0 = (double)iy * g.ys + g.pd2 - si.y;
             double y1 = (double)(iy + 1) * g.ys + g.pd2 - si.y;
             if (!(P.shi[c] > y0 && P.slo[c] < y1)) continue;
-            double xc = 0.5 * (x0 + x1), yc = 0.5 * (y0 + y1);
-            double hxp = 0.5 * (x1 - x0), hyp = 0.5 * (y1 - y0);
-            Mom m = {0.0, 0.0, 0.0, 0.0};
-            bool full = P.rv[c] && P.lv[c + 1] && P.elo[c] <= y0 && P.ehi[c] >= y1 && P.elo[c + 1] <= y0 &&
-                        P.ehi[c + 1] >= y1;
-            if (full) {
-                m.A = 4.0 * hxp * hyp;
-                m.I2 = m.A * (hxp * hxp + hyp * hyp) * (1.0 / 3.0);
-            } else {
-                for (int k = 0; k < nv; k++) {
-                    int kn = (k + 1 == nv) ? 0 : k + 1;
-                    double px = P.X[k], py = P.Y[k], qx = P.X[kn], qy = P.Y[kn];
-                    if (px == qx && (px == x0 || px == x1)) continue;  // counted by the pixel side
-                    if (fmax(px, qx) < x0 || fmin(px, qx) > x1 || fmax(py, qy) < y0 || fmin(py, qy) > y1) continue;
-                    // Liang-Barsky against the pixel box (reciprocals precomputed)
-                    double dx = qx - px, dy = qy - py, t0 = 0.0, t1 = 1.0;
-                    if (dx != 0.0) {
-                        double ta = (x0 - px) * P.EIX[k], tb = (x1 - px) * P.EIX[k];
-                        t0 = fmax(t0, fmin(ta, tb));
-                        t1 = fmin(t1, fmax(ta, tb));
-                    } else if (px < x0 || px > x1) {
-                        continue;
-                    }
-                    if (dy != 0.0) {
-                        double ta = (y0 - py) * P.EIY[k], tb = (y1 - py) * P.EIY[k];
-                        t0 = fmax(t0, fmin(ta, tb));
-                        t1 = fmin(t1, fmax(ta, tb));
-                    } else if (py < y0 || py > y1) {
-                        continue;
-                    }
-                    if (!(t0 < t1)) continue;
-                    double ax0 = (t0 == 0.0 ? px : px + t0 * dx) - xc;
-                    double by0 = (t0 == 0.0 ? py : py + t0 * dy) - yc;
-                    double ax1 = (t1 == 1.0 ? qx : px + t1 * dx) - xc;
-                    double by1 = (t1 == 1.0 ? qy : py + t1 * dy) - yc;
-                    seg_terms(ax0, by0, ax1, by1, m);
-                }
-                if (P.lv[c + 1]) {  // right side, upwards
-                    double b0 = fmax(P.elo[c + 1], y0), b1 = fmin(P.ehi[c + 1], y1);
-                    if (b1 > b0) vside_terms(x1 - xc, b0 - yc, b1 - yc, m);
-                }
-                if (P.rv[c]) {      // left side, downwards
-                    double b0 = fmax(P.elo[c], y0), b1 = fmin(P.ehi[c], y1);
-                    if (b1 > b0) vside_terms(x0 - xc, b1 - yc, b0 - yc, m);
-                }
-            }
-            if (!(m.A > 0.0)) continue;
-            if (g.splat != nullptr) atomicAdd(g.splat + ix + iy * g.nx, g.splat_w * m.A);
-            double rho = g.rho[ix + iy * g.nx];
-            mu += rho * m.A;
-            S += rho * (m.A * (xc * xc + yc * yc) + 2.0 * (xc * m.Ia + yc * m.Ib) + m.I2);
-            if (m.A > 1e-10) {  // compute_center skips tiny pieces (basic_function.cuh:1153)
-                Mt += rho * m.A;
-                Mx += rho * (m.A * xc + m.Ia);
-                My += rho * (m.A * yc + m.Ib);
-            }
+            pixel_sums<false>(P, nv, 0u, c, ix, iy, x0, x1, y0, y1, g, sum);
         }
         __syncwarp();
     }
-    acc.mu = warp_sum(mu);
-    acc.S = warp_sum(S);
-    acc.Mt = warp_sum(Mt);
-    acc.Mx = warp_sum(Mx);
-    acc.My = warp_sum(My);
+    acc.mu = warp_sum(sum.mu);
+    acc.S = warp_sum(sum.S);
+    acc.Mt = warp_sum(sum.Mt);
+    acc.Mx = warp_sum(sum.Mx);
+    acc.My = warp_sum(sum.My);
     return acc;
 }
 
 // compute_solid_angle (basic_function.cuh:558-588): solid angle of the planar
 // polygon (absolute vertices, plane z) seen from the light, as the sum over
 // the fan from vertex 0 of 2 atan(num / den), triangles with |den| < 1e-6
-// skipped, absolute value at the end.  One lane does the sum in ring order.
-template <class SP>
-__device__ double solid_angle_of(const SP &P, int nv, double2 si, double z, const double *L)
+// skipped, absolute value at the end, summed in ring order: vertex k is ring(k).
+template <class F>
+__device__ double solid_angle_of(F ring, int nv, double2 si, double z, const double *L)
 {
     auto unit = [](double v[3]) {
         double l = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
@@ -862,9 +878,10 @@ __device__ double solid_angle_of(const SP &P, int nv, double2 si, double z, cons
     };
     double ang = 0.0;
     for (int k = 0; k < nv - 2; k++) {
-        double v1[3] = {si.x + P.X[0] - L[0], si.y + P.Y[0] - L[1], z - L[2]};
-        double v2[3] = {si.x + P.X[k + 1] - L[0], si.y + P.Y[k + 1] - L[1], z - L[2]};
-        double v3[3] = {si.x + P.X[k + 2] - L[0], si.y + P.Y[k + 2] - L[1], z - L[2]};
+        const double2 p0 = ring(0), p1 = ring(k + 1), p2 = ring(k + 2);
+        double v1[3] = {si.x + p0.x - L[0], si.y + p0.y - L[1], z - L[2]};
+        double v2[3] = {si.x + p1.x - L[0], si.y + p1.y - L[1], z - L[2]};
+        double v3[3] = {si.x + p2.x - L[0], si.y + p2.y - L[1], z - L[2]};
         unit(v1);
         unit(v2);
         unit(v3);
@@ -1393,14 +1410,10 @@ __device__ void poly_centroid(const SP &P, int nv, int lane, double &cx, double 
 // fast path: the polygon lives in registers, one vertex per lane
 // ---------------------------------------------------------------------------
 struct FastScratch {
-    double X[32], Y[32];              // polygon snapshot (tree tests, integration)
+    double X[32], Y[32];              // polygon snapshot (tree tests)
     double A[32], B[32], C[32];       // compaction scratch of the general clip
     int L[32];
-    double EIX[32], EIY[32], ESL[32]; // per edge: 1/dx, 1/dy, dy/dx
     int fr[2][COT_FRMAX];
-    double elo[33], ehi[33];
-    double slo[32], shi[32];
-    unsigned char lv[33], rv[33];
     int KL[32];                       // ring labels just before the ring emptied
     int kn, kill;                     // their count and the label that emptied it
 };
@@ -2169,7 +2182,7 @@ __device__ __forceinline__ RegPoly cell_walk(const CotGeo &g, const CellsArgs &a
 
 // Phase 3: overflow hand-off, or the ring's integrals (EXACT) / the ring
 // buffer (solve path), the next evaluation's cache and the per-cell outputs.
-template <bool EXACT, int LPC, bool KEEP = false>
+template <int LPC, bool KEEP = false>
 __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a, const int i, const double2 si,
                                             const double wi, RegPoly P, FastScratch &S, int *olist, int *ocount)
 {
@@ -2185,7 +2198,6 @@ __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a,
         SG.sync();
         return;
     }
-    // ---- 3. integrate the density over the cell --------------------------
     PSTAT_CLOCK(t2);
     const int nv = P.nv;
     if (nv >= 3) {
@@ -2205,17 +2217,11 @@ __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a,
     }
     if (lane < nv) { S.X[lane] = P.x; S.Y[lane] = P.y; }
     SG.sync();
-    CellAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
-    // the solve's path only builds the ring here: k_integrate sums over it
-    // from the ring buffer (two kernels with smaller instruction footprints
-    // than one fused kernel)
-    constexpr bool split = !EXACT;
+    // k_integrate sums over the ring from the ring buffer (kernels with smaller
+    // instruction footprints than one fused kernel)
     if (nv >= 3) {
-        if constexpr (EXACT)
-            acc = integrate_cell(S, nv, splat_geo(g, a, S, nv, i, lane), si, lane);
-        else if (lane < nv)
-            a.rbuf[ring_at(i, lane)] = make_double2(P.x, P.y);
-        if constexpr (!EXACT && LPC == 32) {
+        if (lane < nv) a.rbuf[ring_at(i, lane)] = make_double2(P.x, P.y);
+        if constexpr (LPC == 32) {
             // a cell whose pixel box is large goes on the heavy list: the
             // integration kernel starts those cells first, so that they run
             // beside the many small ones instead of after them
@@ -2247,17 +2253,10 @@ __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a,
     PSTAT_ADD(2, t3 - t2);
     PSTAT_ADD(8, 1);
     PSTAT_ADD(11, nv);
-    double pcx = 0.0, pcy = 0.0;
-    if constexpr (EXACT) {
-        if (a.cen != nullptr && nv >= 3 && (!a.weighted || acc.Mt == 0.0)) poly_centroid(S, nv, lane, pcx, pcy);
-    }
     if (a.ring_xy != nullptr && lane < nv && lane < a.ring_cap) {
         a.ring_xy[2 * ((size_t)i * a.ring_cap + lane)] = si.x + P.x;
         a.ring_xy[2 * ((size_t)i * a.ring_cap + lane) + 1] = si.y + P.y;
         a.ring_lab[(size_t)i * a.ring_cap + lane] = P.l;
-    }
-    if constexpr (EXACT) {
-        if (a.solid != nullptr && lane == 0) a.solid[i] = nv >= 3 ? solid_angle_of(S, nv, si, a.solid_z, a.solid_light) : 0.0;
     }
     if (a.nbn != nullptr) {
         // this evaluation seeds the next: a ring of up to COT_NBC edges
@@ -2282,35 +2281,10 @@ __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a,
             if (lane == 0) a.nbn[i] = cnt == 0 ? 0 : (nv == 0 ? -(COT_NB_HIDDEN + cnt) : -cnt);
         }
     }
-    if (lane == 0) {
-        if (!split) {
-            a.mu[i] = acc.mu;
-            // f_i = -w_i nu_i - sum_pix rho (int |x-s_i|^2 - w_i area)   (basic_function.cuh:875-941);
-            // stored without its -w_i nu_i term, which the reduction adds, so
-            // that nu may change after the cells are built
-            a.fc[i] = -(acc.S - wi * acc.mu);
-        }
-        a.nv[i] = nv;
-        if (a.cen != nullptr) {
-            const bool ex = nv >= 3;
-            a.exist[i] = ex ? 1 : 0;
-            double cx = si.x, cy = si.y;
-            if (ex) {
-                if (a.weighted && acc.Mt != 0.0) {
-                    cx = si.x + acc.Mx / acc.Mt;
-                    cy = si.y + acc.My / acc.Mt;
-                } else {
-                    cx = si.x + pcx;
-                    cy = si.y + pcy;
-                }
-            }
-            a.cen[2 * i] = cx;
-            a.cen[2 * i + 1] = cy;
-        }
-    }
+    if (lane == 0) a.nv[i] = nv;
 }
 
-template <bool EXACT, int LPC>
+template <int LPC>
 __device__ __forceinline__ void fast_cell(const CotGeo &g, const CellsArgs &a, const int i, FastScratch &S,
                                           int *olist, int *ocount)
 {
@@ -2319,7 +2293,7 @@ __device__ __forceinline__ void fast_cell(const CotGeo &g, const CellsArgs &a, c
     bool cached = false;
     RegPoly P = cell_first<LPC>(g, a, i, si, wi, S, cached);
     P = cell_walk<LPC>(g, a, i, si, wi, P, cached, S);
-    cell_finish<EXACT, LPC>(g, a, i, si, wi, P, S, olist, ocount);
+    cell_finish<LPC>(g, a, i, si, wi, P, S, olist, ocount);
 }
 
 // The persistent cell kernel: each warp fetches 32 / LPC cells at a time
@@ -2327,10 +2301,9 @@ __device__ __forceinline__ void fast_cell(const CotGeo &g, const CellsArgs &a, c
 // segments of a warp run the same phases together.  pass 0: every cell,
 // rings above LPC vertices into ovf_list; pass 1: the cells of ovf_list,
 // rings above LPC into ovf_list2.
-template <int MINB, bool EXACT, int LPC>
+template <int MINB, int LPC>
 __global__ void __launch_bounds__(128, MINB) k_cells_fast(const __grid_constant__ CotGeo g, CellsArgs a, int pass)
 {
-    static_assert(!EXACT || LPC == 32, "the exact path works a whole warp per cell");
     constexpr int CPW = 32 / LPC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FastScratch &S = reinterpret_cast<FastScratch *>(smem_raw)[threadIdx.x / LPC];
@@ -2345,7 +2318,7 @@ __global__ void __launch_bounds__(128, MINB) k_cells_fast(const __grid_constant_
         base = __shfl_sync(FULLMASK, base, 0);
         if (base >= total) break;
         const int slot = base + (int)(threadIdx.x & 31) / LPC;
-        if (slot < total) fast_cell<EXACT, LPC>(g, a, pass == 0 ? slot : a.ovf_list[slot], S, olist, ocount);
+        if (slot < total) fast_cell<LPC>(g, a, pass == 0 ? slot : a.ovf_list[slot], S, olist, ocount);
         __syncwarp();
     }
     PSTAT_FLUSH();
@@ -2385,7 +2358,7 @@ __global__ void __launch_bounds__(128, MINB) k_cells_first(CotGeo g, CellsArgs a
         const RegPoly P = cell_first<LPC>(g, a, i, si, wi, S, cached);
         if (P.nv <= 0) {
             // emptied (hidden cell) or outgrew 32 vertices: finished here
-            cell_finish<false, LPC>(g, a, i, si, wi, P, S, a.ovf_list, a.ovf_count);
+            cell_finish<LPC>(g, a, i, si, wi, P, S, a.ovf_list, a.ovf_count);
             if (lane == 0) a.cstate[i] = -1;
         } else {
             if (lane < P.nv) {
@@ -2798,7 +2771,7 @@ __global__ void __launch_bounds__(128, MINB) k_cells_walk(const __grid_constant_
         if (lane == 0) S.kn = -1;
         __syncwarp();
         P = cell_walk<LPC>(g, a, i, si, wi, P, (st & CST_CACHED) != 0, S);
-        if (P.nv != COT_DEFERRED) cell_finish<false, LPC, KEEP>(g, a, i, si, wi, P, S, a.ovf_list, a.ovf_count);
+        if (P.nv != COT_DEFERRED) cell_finish<LPC, KEEP>(g, a, i, si, wi, P, S, a.ovf_list, a.ovf_count);
         __syncwarp();
     }
     PSTAT_FLUSH();
@@ -3043,7 +3016,7 @@ __global__ void __launch_bounds__(32 * HEAVY_WARPS, 2) k_cells_heavy(const __gri
             if (nv <= 0 || !over || attempt == HEAVY_RETRY) break;
         }
         if (H.nv > 0 && over && wp == 0) P = scan_all_buckets<32>(g, a.wt, i, si, wi, P, S, 0, 0, -1);
-        if (wp == 0) cell_finish<false, 32, KEEP>(g, a, i, si, wi, P, S, a.ovf_list, a.ovf_count);
+        if (wp == 0) cell_finish<32, KEEP>(g, a, i, si, wi, P, S, a.ovf_list, a.ovf_count);
         __syncthreads();
     }
 }
@@ -3109,7 +3082,7 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
             double raw[6];
             integrate_part(S, nv, pix_geo(g), g.xy[i], part, raw);
             if (lane == 0) {
-                double *pp = a.hpart + ((size_t)slot * COT_SPLIT + part) * 4;
+                double *pp = a.hpart + ((size_t)slot * COT_SPLIT + part) * COT_PART;
                 pp[0] = raw[0];
                 pp[1] = raw[1];
                 pp[2] = raw[2];
@@ -3117,13 +3090,13 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
                 __threadfence();
                 if (atomicAdd(a.hticket + slot, 1u) == COT_SPLIT - 1) {
                     __threadfence();
-                    const volatile double *q = a.hpart + (size_t)slot * COT_SPLIT * 4;
+                    const volatile double *q = a.hpart + (size_t)slot * COT_SPLIT * COT_PART;
                     double sA = q[0], sIa = q[1], sIb = q[2], sI2 = q[3];
                     for (int k = 1; k < COT_SPLIT; k++) {
-                        sA += q[4 * k];
-                        sIa += q[4 * k + 1];
-                        sIb += q[4 * k + 2];
-                        sI2 += q[4 * k + 3];
+                        sA += q[COT_PART * k];
+                        sIa += q[COT_PART * k + 1];
+                        sIb += q[COT_PART * k + 2];
+                        sI2 += q[COT_PART * k + 3];
                     }
                     const double ox = raw[4], oy = raw[5];
                     const double Sv = sI2 + 2.0 * (ox * sIa + oy * sIb) + (ox * ox + oy * oy) * sA;
@@ -3184,6 +3157,328 @@ __global__ void __launch_bounds__(128, MINB) k_integrate(CotGeo g, CellsArgs a)
             __syncwarp();
         }
     }
+}
+
+// Scratch of the per-pixel integration: a whole warp's cell, or one of four.
+template <int L>
+struct PixScratch {
+    static constexpr int NV = L == 32 ? 32 : COT_SEG_NV + 2;
+    double X[NV], Y[NV], EIX[NV], EIY[NV], ESL[NV];  // ring; per edge 1/dx, 1/dy, dy/dx
+    double elo[L + 1], ehi[L + 1];                   // section of the cell at column lines
+    double slo[L], shi[L];                           // y-range of the cell in each column strip
+    unsigned EB[NV];                                 // per edge: its box in the cell's pixels (8 lanes)
+    unsigned char lv[L + 1], rv[L + 1];              // left / right limit of the section valid
+    double pad[2];                                   // the four of a warp on different banks
+};
+
+// The sums of integrate_cell for four cells a warp, 8 lanes each: 8 columns at
+// a time, a lane per column line and strip, then the pixels that the strips
+// hold (and no others) handed out one a lane by a scan.  A warp a cell leaves
+// most lanes idle through the column tables and tests the box's empty pixels
+// too.  Every loop runs as often as the longest of the warp's cells needs.
+// With the rings built by the solve's kernels instead of in the same kernel,
+// weighted centroids at 65,536 sites on 1024^2 take 330 us of kernels against
+// 830 (this one 196: instruction fetch and issue bound), an evaluation with
+// plain centroids at 16,384 sites 105 against 230.
+__device__ __forceinline__ CellAcc integrate_pixels(PixScratch<8> &P, int nv, const PixGeo g, double2 si)
+{
+    const int sl = threadIdx.x & 7;
+    double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
+    for (int k = sl; k < nv; k += 8) {
+        const int kn = (k + 1 == nv) ? 0 : k + 1;
+        const double px = P.X[k], py = P.Y[k], dx = P.X[kn] - px, dy = P.Y[kn] - py;
+        P.EIX[k] = dx != 0.0 ? 1.0 / dx : 0.0;
+        P.EIY[k] = dy != 0.0 ? 1.0 / dy : 0.0;
+        P.ESL[k] = dx != 0.0 ? dy / dx : 0.0;
+        mnx = fmin(mnx, px);
+        mxx = fmax(mxx, px);
+        mny = fmin(mny, py);
+        mxy = fmax(mxy, py);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        mnx = fmin(mnx, __shfl_xor_sync(FULLMASK, mnx, o));
+        mxx = fmax(mxx, __shfl_xor_sync(FULLMASK, mxx, o));
+        mny = fmin(mny, __shfl_xor_sync(FULLMASK, mny, o));
+        mxy = fmax(mxy, __shfl_xor_sync(FULLMASK, mxy, o));
+    }
+    __syncwarp();
+    // pixel range of the bounding box, as integrate_cell
+    int lx = 0, ly = 0, hx = 0, hy = 0;
+    if (nv > 0) {
+        lx = max((int)floor((si.x + mnx - g.pd0) * g.ixs) - 1, 0);
+        ly = max((int)floor((si.y + mny - g.pd2) * g.iys) - 1, 0);
+        hx = min((int)floor((si.x + mxx - g.pd0) * g.ixs) + 2, g.nx);
+        hy = min((int)floor((si.y + mxy - g.pd2) * g.iys) + 2, g.ny);
+    }
+    // the pixel columns and rows that each edge spans, from the cell's first
+    // ones, 7 bits each (a larger one counts as 127); lower bounds as they are,
+    // upper ones from 127 down.  Widened by far more than their rounding: an
+    // edge a rounding short of a pixel line is the side of its pixel.
+    for (int k = sl; k < nv; k += 8) {
+        const int kn = (k + 1 == nv) ? 0 : k + 1;
+        const auto at = [](double v, int o) { return (unsigned)min(max((int)floor(v) - o, 0), 127); };
+        const unsigned c0 = at((si.x + fmin(P.X[k], P.X[kn]) - g.pd0) * g.ixs - 1e-9, lx);
+        const unsigned c1 = at((si.x + fmax(P.X[k], P.X[kn]) - g.pd0) * g.ixs + 1e-9, lx);
+        const unsigned w0 = at((si.y + fmin(P.Y[k], P.Y[kn]) - g.pd2) * g.iys - 1e-9, ly);
+        const unsigned w1 = at((si.y + fmax(P.Y[k], P.Y[kn]) - g.pd2) * g.iys + 1e-9, ly);
+        P.EB[k] = c0 | (127u - c1) << 8 | w0 << 16 | (127u - w1) << 24;
+    }
+    __syncwarp();
+    CellAcc sum = {0.0, 0.0, 0.0, 0.0, 0.0};
+    const int cols = (int)__reduce_max_sync(FULLMASK, (unsigned)max(hx - lx, 0));
+    for (int cx = 0; cx < cols; cx += 8) {
+        const int cx0 = lx + cx, cw = min(8, hx - cx0);
+        for (int c = sl; c <= cw && cw > 0; c += 8) {
+            const double xl = (double)(cx0 + c) * g.xs + g.pd0 - si.x;
+            double lo, hi;
+            section_at(P, nv, xl, lo, hi);
+            P.elo[c] = lo;
+            P.ehi[c] = hi;
+            P.rv[c] = (mnx <= xl && xl < mxx) ? 1 : 0;  // right limit (left side of a pixel)
+            P.lv[c] = (mnx < xl && xl <= mxx) ? 1 : 0;  // left limit (right side of a pixel)
+        }
+        __syncwarp();
+        int r0 = 0, cnt = 0;
+        if (sl < cw) {
+            const int c = sl;
+            const double xl = (double)(cx0 + c) * g.xs + g.pd0 - si.x;
+            const double xr = (double)(cx0 + c + 1) * g.xs + g.pd0 - si.x;
+            double lo = INFINITY, hi = -INFINITY;
+            if (P.rv[c]) { lo = fmin(lo, P.elo[c]); hi = fmax(hi, P.ehi[c]); }
+            if (P.lv[c + 1]) { lo = fmin(lo, P.elo[c + 1]); hi = fmax(hi, P.ehi[c + 1]); }
+            for (int k = 0; k < nv; k++) {
+                const double vx = P.X[k];
+                if (vx > xl && vx < xr) { lo = fmin(lo, P.Y[k]); hi = fmax(hi, P.Y[k]); }
+            }
+            P.slo[c] = lo;
+            P.shi[c] = hi;
+            if (hi > lo) {
+                // rows whose pixel reaches above lo and starts below hi
+                const auto row = [&](int r) { return (double)r * g.ys + g.pd2 - si.y; };
+                int ra = (int)floor((si.y + lo - g.pd2) * g.iys), rb = (int)floor((si.y + hi - g.pd2) * g.iys);
+                if (row(ra) > lo) ra--;
+                else if (row(ra + 1) <= lo) ra++;
+                if (row(rb) >= hi) rb--;
+                else if (row(rb + 1) < hi) rb++;
+                r0 = max(ra, ly);
+                cnt = max(0, min(rb, hy - 1) - r0 + 1);
+            }
+        }
+        __syncwarp();
+        int inc = cnt;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const int v = __shfl_up_sync(FULLMASK, inc, o, 8);
+            if (sl >= o) inc += v;
+        }
+        const int tot = __shfl_sync(FULLMASK, inc, 7, 8);
+        const int top = (int)__reduce_max_sync(FULLMASK, (unsigned)tot);
+        const int first = r0 - (inc - cnt);
+        for (int base = 0; base < top; base += 8) {
+            const int t = base + sl;
+            int k = 0;
+#pragma unroll
+            for (int sft = 4; sft >= 1; sft >>= 1) {
+                const int v = __shfl_sync(FULLMASK, inc, k + sft - 1, 8);
+                if (v <= t) k += sft;
+            }
+            k &= 7;
+            const int iy = __shfl_sync(FULLMASK, first, k, 8) + t, ix = cx0 + k;
+            if (t >= tot) continue;
+            // pixel box exactly as basic_function.cuh:806-809, relative to the site
+            const double x0 = (double)ix * g.xs + g.pd0 - si.x;
+            const double x1 = (double)(ix + 1) * g.xs + g.pd0 - si.x;
+            const double y0 = (double)iy * g.ys + g.pd2 - si.y;
+            const double y1 = (double)(iy + 1) * g.ys + g.pd2 - si.y;
+            if (!(P.shi[k] > y0 && P.slo[k] < y1)) continue;
+            // the edges whose box holds the pixel, one subtraction an edge: each
+            // field's guard bit stays when the pixel is not below the edge's bound
+            const unsigned dc = min(ix - lx, 127), dr = min(iy - ly, 127);
+            const unsigned at = 0x80808080u | dc | (127u - dc) << 8 | dr << 16 | (127u - dr) << 24;
+            unsigned edges = 0u;
+            for (int e = 0; e < nv; e++) edges |= (((at - P.EB[e]) & 0x80808080u) == 0x80808080u ? 1u : 0u) << e;
+            pixel_sums<true>(P, nv, edges, k, ix, iy, x0, x1, y0, y1, g, sum);
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        sum.mu += __shfl_xor_sync(FULLMASK, sum.mu, o);
+        sum.S += __shfl_xor_sync(FULLMASK, sum.S, o);
+        sum.Mt += __shfl_xor_sync(FULLMASK, sum.Mt, o);
+        sum.Mx += __shfl_xor_sync(FULLMASK, sum.Mx, o);
+        sum.My += __shfl_xor_sync(FULLMASK, sum.My, o);
+    }
+    return sum;
+}
+
+// Area and plain area centroid (relative to the site) of a ring, by one
+// thread: vertex k is v(k).
+template <class F>
+__device__ __forceinline__ double ring_centroid(int nv, F v, double &cx, double &cy)
+{
+    double a = 0.0, mx = 0.0, my = 0.0;
+    double2 p = v(nv - 1);
+    for (int k = 0; k < nv; k++) {
+        const double2 q = v(k);
+        const double cr = p.x * q.y - q.x * p.y;
+        a += cr;
+        mx += (p.x + q.x) * cr;
+        my += (p.y + q.y) * cr;
+        p = q;
+    }
+    cx = a != 0.0 ? mx / (3.0 * a) : 0.0;
+    cy = a != 0.0 ? my / (3.0 * a) : 0.0;
+    return 0.5 * a;
+}
+
+// A whole cell by one warp, out of line (the large ones).
+__device__ __noinline__ CellAcc pixels_whole(PixScratch<32> &S, int nv, const PixGeo pg, double2 si, int part,
+                                             int nparts)
+{
+    return integrate_cell(S, nv, pg, si, threadIdx.x & 31, part, nparts);
+}
+
+constexpr int PIX_WARP_SMEM =
+    (int)(sizeof(PixScratch<32>) > 4 * sizeof(PixScratch<8>) ? sizeof(PixScratch<32>) : 4 * sizeof(PixScratch<8>));
+
+// k_integrate's counterpart for what needs each pixel's part of a cell: the
+// weighted centroids and the render.  The cells of the split list take
+// COT_SPLIT warps (each every eighth row of pixels), those of the heavy list
+// one, first; the others share one with three more.
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) k_integrate_pixels(const __grid_constant__ CotGeo g, CellsArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned char *mine = smem_raw + (threadIdx.x >> 5) * PIX_WARP_SMEM;
+    PixScratch<32> &S = *reinterpret_cast<PixScratch<32> *>(mine);
+    const int lane = threadIdx.x & 31, sl = lane & 7;
+    PixScratch<8> &T = reinterpret_cast<PixScratch<8> *>(mine)[lane >> 3];
+    int *fetch = a.ovf_count + 6;
+    // the parts of the split cells first, then the heavy list, then the others
+    const int nh = a.ovf_count[10], np = min(a.ovf_count[13], a.hsplit_cap) * COT_SPLIT;
+    // the results of cell i, by one lane
+    const auto finish = [&](int i, int nv, const CellAcc &acc, double2 si, auto ring) {
+        a.mu[i] = acc.mu;
+        a.fc[i] = -(acc.S - a.wt[i] * acc.mu);
+        if (a.cen == nullptr) return;
+        a.exist[i] = nv >= 3 ? 1 : 0;
+        double cx = 0.0, cy = 0.0;
+        if (nv >= 3 && acc.Mt != 0.0) {
+            cx = acc.Mx / acc.Mt;
+            cy = acc.My / acc.Mt;
+        } else if (nv >= 3) {
+            ring_centroid(nv, ring, cx, cy);
+        }
+        a.cen[2 * (size_t)i] = si.x + cx;
+        a.cen[2 * (size_t)i + 1] = si.y + cy;
+    };
+    // render (basic_function.cuh:660-741): the cell's carried mass spread over
+    // the pixels in proportion to area; the weight is nu_i * gray / area(cell)
+    const auto geo = [&](int i, int nv, auto ring) {
+        PixGeo p = pix_geo(g);
+        if (a.splat != nullptr && nv >= 3) {
+            double cx, cy;
+            const double ar = fabs(ring_centroid(nv, ring, cx, cy));
+            if (ar != 0.0) {
+                p.splat = a.splat;
+                p.splat_w = g.nu[i] * a.splat_scale / ar;
+            }
+        }
+        return p;
+    };
+    while (true) {
+        int f = 0;
+        if (lane == 0) f = atomicAdd(fetch, 1);
+        f = __shfl_sync(FULLMASK, f, 0);
+        if (f >= (g.n + 3) / 4 + nh + np) break;
+        if (f < nh + np) {
+            const int slot = f / COT_SPLIT, part = f < np ? f % COT_SPLIT : 0;
+            const int i = f < np ? a.hsplit[slot] : a.hlist[f - np];
+            const int nv = a.nv[i];
+            if (lane < nv) {
+                const double2 v = a.rbuf[ring_at(i, lane)];
+                S.X[lane] = v.x;
+                S.Y[lane] = v.y;
+            }
+            __syncwarp();
+            const auto ring = [&](int k) { return make_double2(S.X[k], S.Y[k]); };
+            const double2 si = g.xy[i];
+            CellAcc acc = pixels_whole(S, nv, geo(i, nv, ring), si, part, f < np ? COT_SPLIT : 1);
+            if (lane == 0) {
+                bool last = true;
+                if (f < np) {
+                    // the part that finishes last adds the parts in order
+                    double *pp = a.hpart + (size_t)slot * COT_SPLIT * COT_PART;
+                    double *mp = pp + part * COT_PART;
+                    mp[0] = acc.mu;
+                    mp[1] = acc.S;
+                    mp[2] = acc.Mt;
+                    mp[3] = acc.Mx;
+                    mp[4] = acc.My;
+                    __threadfence();
+                    last = atomicAdd(a.hticket + slot, 1u) == COT_SPLIT - 1;
+                    if (last) {
+                        __threadfence();
+                        const volatile double *q = pp;
+                        acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+                        for (int k = 0; k < COT_SPLIT; k++, q += COT_PART) {
+                            acc.mu += q[0];
+                            acc.S += q[1];
+                            acc.Mt += q[2];
+                            acc.Mx += q[3];
+                            acc.My += q[4];
+                        }
+                        a.hticket[slot] = 0u;
+                    }
+                }
+                if (last) finish(i, nv, acc, si, ring);
+            }
+            __syncwarp();
+            continue;
+        }
+        f -= np;
+        const int i = (f - nh) * 4 + (lane >> 3);
+        // the segment's cell: none past the end, for a heavy cell, or a ring
+        // of the large-ring pass
+        int nv = -1;
+        if (i < g.n && !((nh > 0 || np > 0) && a.cstate[i] == CST_HEAVY)) nv = a.nv[i];
+        if (nv > COT_SEG_NV) nv = -1;
+        const int m = nv >= 3 ? nv : 0;
+        double2 si = make_double2(0.0, 0.0);
+        if (nv >= 0) si = g.xy[i];
+        for (int k = sl; k < m; k += 8) {
+            const double2 v = a.rbuf[ring_at(i, k)];
+            T.X[k] = v.x;
+            T.Y[k] = v.y;
+        }
+        __syncwarp();
+        const auto ring = [&](int k) { return make_double2(T.X[k], T.Y[k]); };
+        const CellAcc acc = integrate_pixels(T, m, geo(i, m, ring), si);
+        if (sl == 0 && nv >= 0) finish(i, m, acc, si, ring);
+        __syncwarp();
+    }
+}
+
+// Plain centroids and solid angles of the rings in the ring buffer, a thread
+// a cell (the rows of a tile are read whole).
+__global__ void __launch_bounds__(128) k_cell_points(const __grid_constant__ CotGeo g, CellsArgs a)
+{
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i >= g.n) return;
+    const int nv = a.nv[i];
+    if (nv > COT_RCAP) return;  // the large-ring pass
+    const double2 si = g.xy[i];
+    const auto ring = [&](int k) { return a.rbuf[ring_at(i, k)]; };
+    if (a.cen != nullptr) {
+        double cx = 0.0, cy = 0.0;
+        if (nv >= 3) ring_centroid(nv, ring, cx, cy);
+        a.exist[i] = nv >= 3 ? 1 : 0;
+        a.cen[2 * (size_t)i] = si.x + cx;
+        a.cen[2 * (size_t)i + 1] = si.y + cy;
+    }
+    if (a.solid != nullptr) a.solid[i] = nv >= 3 ? solid_angle_of(ring, nv, si, a.solid_z, a.solid_light) : 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -3407,7 +3702,10 @@ __global__ void __launch_bounds__(128, MINB) k_cells(CotGeo g, CellsArgs a, int 
                 a.ring_lab[(size_t)i * a.ring_cap + k] = P.L[k];
             }
         }
-        if (a.solid != nullptr && lane == 0) a.solid[i] = nv >= 3 ? solid_angle_of(P, nv, si, a.solid_z, a.solid_light) : 0.0;
+        if (a.solid != nullptr && lane == 0) 
+            a.solid[i] = nv >= 3 ? solid_angle_of([&](int k) { return make_double2(P.X[k], P.Y[k]); }, nv, si, a.solid_z,
+                                                  a.solid_light)
+                                 : 0.0;
         if (a.keep_labels && nv >= 3) {
             // the Newton solve's Jacobian: a ring that ended at most COT_RCAP
             // vertices goes to the ring buffer like the fast path's rings, a
@@ -3513,6 +3811,9 @@ static size_t cells_smem(int maxv, int warps)
 #ifndef WALK_MINB
 #define WALK_MINB 8   // k_cells_walk (64 registers; 6 blocks measured 2 % slower)
 #endif
+#ifndef PIX_MINB
+#define PIX_MINB 5    // k_integrate_pixels
+#endif
 #ifndef INT_MINB
 #define INT_MINB 6  // k_integrate: 80 registers (8 blocks: 2043 us at 262,144 sites against 2072, but 724 against 718 at 65,536)
 #endif
@@ -3537,13 +3838,13 @@ static size_t cells_smem(int maxv, int warps)
 #define COT_FAST_G8_N 40000
 #endif
 static int g_blocks_per_sm32 = 0, g_blocks_per_sm16 = 0, g_blocks_per_sm8 = 0, g_blocks_per_smi = 0;
-static int g_blocks_per_smf = 0, g_blocks_per_smw = 0, g_blocks_per_smb = 0;
+static int g_blocks_per_smf = 0, g_blocks_per_smw = 0, g_blocks_per_smb = 0, g_blocks_per_smp = 0;
 
-template <bool EXACT, int LPC>
+template <int LPC>
 static void launch_fast(const CotGeo &g, const CellsArgs &a, int pass, int blocks, cudaStream_t s)
 {
     const size_t sm = sizeof(FastScratch) * CELLS_WPB * (32 / LPC);
-    k_cells_fast<CELLS_MINB, EXACT, LPC><<<blocks, 32 * CELLS_WPB, sm, s>>>(g, a, pass);
+    k_cells_fast<CELLS_MINB, LPC><<<blocks, 32 * CELLS_WPB, sm, s>>>(g, a, pass);
 }
 
 // One evaluation: bucket and tree bounds, then the cells.  cells_per_warp 2
@@ -3576,18 +3877,20 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
         c.launches++;
     }
     const int sms = num_sms > 0 ? num_sms : 148;
-    const bool exact = a.cen != nullptr || a.splat != nullptr || a.solid != nullptr;
-    const int lpc = (exact || cells_per_warp < 2) ? 32 : (cells_per_warp == 2 ? 16 : 8);
+    // what needs each pixel's part of a cell: weighted centroids (the
+    // reference leaves tiny parts out) and the render; plain centroids and
+    // solid angles need the rings alone
+    const bool pixels = a.splat != nullptr || (a.cen != nullptr && a.weighted);
+    const bool points = (a.cen != nullptr && !a.weighted) || a.solid != nullptr;
+    const int lpc = (pixels || points || cells_per_warp < 2) ? 32 : (cells_per_warp == 2 ? 16 : 8);
     // the bucket walk's lists exist only on the path that runs it: every
     // other path walks in full
-    if (exact || lpc != 32) a.blist = a.bcnt = nullptr;
+    if (lpc != 32) a.blist = a.bcnt = nullptr;
     // the heavy integration list (ovf_list2, which only the 16- and 8-lane
     // paths use otherwise) on the two-kernel path
-    a.hlist = (exact || lpc != 32) ? nullptr : a.ovf_list2;
-    if (exact || lpc != 32) {
-        a.wlist = nullptr;
-        a.hsplit = nullptr;
-    }
+    a.hlist = lpc != 32 ? nullptr : a.ovf_list2;
+    if (lpc != 32) a.wlist = nullptr;
+    if (lpc != 32) a.hsplit = nullptr;
     const int per_sm32 = g_blocks_per_sm32 > 0 ? g_blocks_per_sm32 : CELLS_MINB;
     const int per_sm16 = g_blocks_per_sm16 > 0 ? g_blocks_per_sm16 : CELLS_MINB;
     const int per_sm8 = g_blocks_per_sm8 > 0 ? g_blocks_per_sm8 : 1;
@@ -3596,9 +3899,7 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     const int blocks = std::min(want, sms * (lpc == 32 ? per_sm32 : (lpc == 16 ? per_sm16 : per_sm8)));
     bool timed = c.profile && c.ev != nullptr && c.ev_used + 2 <= c.ev_cap;
     if (timed) cudaEventRecord(c.ev[c.ev_used], s);
-    if (exact) {
-        launch_fast<true, 32>(g, a, 0, blocks, s);
-    } else if (lpc == 32) {
+    if (lpc == 32) {
         const int bw = std::min(g.n, sms * (g_blocks_per_smw > 0 ? g_blocks_per_smw : WALK_MINB) * CELLS_WPB);
         const int bf = std::min(g.n, sms * (g_blocks_per_smf > 0 ? g_blocks_per_smf : FIRST_MINB) * CELLS_WPB);
         const size_t sm = sizeof(FastScratch) * CELLS_WPB;
@@ -3638,21 +3939,30 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
             k_cells_heavy<false><<<2 * sms, 32 * HEAVY_WARPS, hsm, s>>>(g, a);
         c.launches++;
     } else if (lpc == 16) {
-        launch_fast<false, 16>(g, a, 0, blocks, s);
-        launch_fast<false, 32>(g, a, 1, sms, s);
+        launch_fast<16>(g, a, 0, blocks, s);
+        launch_fast<32>(g, a, 1, sms, s);
         c.launches++;
     } else {
-        launch_fast<false, 8>(g, a, 0, blocks, s);
-        launch_fast<false, 32>(g, a, 1, sms, s);
+        launch_fast<8>(g, a, 0, blocks, s);
+        launch_fast<32>(g, a, 1, sms, s);
         c.launches++;
     }
-    if (!exact) {
+    if (pixels) {
+        const int per = g_blocks_per_smp > 0 ? g_blocks_per_smp : PIX_MINB;
+        const int bp = std::min((g.n + CELLS_WPB - 1) / CELLS_WPB, sms * per);
+        k_integrate_pixels<PIX_MINB><<<bp, 32 * CELLS_WPB, PIX_WARP_SMEM * CELLS_WPB, s>>>(g, a);
+        c.launches++;
+    } else {
         const int per_smi = g_blocks_per_smi > 0 ? g_blocks_per_smi : 8;
         const int bi = std::min((g.n + CELLS_WPB - 1) / CELLS_WPB, sms * per_smi);
         if (a.hlist != nullptr && g.n > COT_SEG_MIN_N)
             k_integrate<INT_MINB, 8><<<bi, 32 * CELLS_WPB, INT_WARP_SMEM * CELLS_WPB, s>>>(g, a);
         else
             k_integrate<INT_MINB, 32><<<bi, 32 * CELLS_WPB, INT_WARP_SMEM * CELLS_WPB, s>>>(g, a);
+        c.launches++;
+    }
+    if (points) {
+        k_cell_points<<<(g.n + 127) / 128, 128, 0, s>>>(g, a);
         c.launches++;
     }
     if (timed) {
@@ -3682,24 +3992,24 @@ extern "C" __attribute__((visibility("default"))) int cot_debug_phase_stats(unsi
 void configure_cells_kernels()
 {
     const int sm32 = (int)(sizeof(FastScratch) * CELLS_WPB), sm16 = 2 * sm32, sm8 = 4 * sm32;
-    cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
-    cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
-    cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, false, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm16);
-    cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm8);
+    cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
+    cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm16);
+    cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm8);
     cudaFuncSetAttribute(k_cells<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cells_smem(256, 1));
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, false, 32>, 32 * CELLS_WPB,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, 32>, 32 * CELLS_WPB,
                                                       sm32) == cudaSuccess && nb > 0)
         g_blocks_per_sm32 = nb;
     nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, false, 16>, 32 * CELLS_WPB,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, 16>, 32 * CELLS_WPB,
                                                       sm16) == cudaSuccess && nb > 0)
         g_blocks_per_sm16 = nb;
     nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, false, 8>, 32 * CELLS_WPB,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, 8>, 32 * CELLS_WPB,
                                                       sm8) == cudaSuccess && nb > 0)
         g_blocks_per_sm8 = nb;
-    const int smi = INT_WARP_SMEM * CELLS_WPB;
+    const int smi = INT_WARP_SMEM * CELLS_WPB, smp = PIX_WARP_SMEM * CELLS_WPB;
+    cudaFuncSetAttribute(k_integrate_pixels<PIX_MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp);
     cudaFuncSetAttribute(k_integrate<INT_MINB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi);
     cudaFuncSetAttribute(k_integrate<INT_MINB, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi);
     cudaFuncSetAttribute(k_cells_first<FIRST_MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
@@ -3725,6 +4035,11 @@ void configure_cells_kernels()
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_integrate<INT_MINB, 8>, 32 * CELLS_WPB, smi) == cudaSuccess &&
         nb > 0)
         g_blocks_per_smi = nb;
+    nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_integrate_pixels<PIX_MINB>, 32 * CELLS_WPB, smp) ==
+            cudaSuccess &&
+        nb > 0)
+        g_blocks_per_smp = nb;
 }
 
 }  // namespace cot

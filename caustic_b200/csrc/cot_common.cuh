@@ -198,6 +198,7 @@ struct CellsArgs {
 
 #define COT_HBIG_W 256  // entries of a big Jacobian row (the large-ring pass's capacity)
 #define COT_SPLIT 8          // warps that share the integration of a cell with a very large pixel box
+#define COT_PART 5           // sums that each of them hands over
 #define COT_HSPLIT_CAP 2048  // such cells per evaluation (the rest are integrated whole, first)
 
 void launch_eval(const CotGeo &g, const CellsArgs &a, int cells_per_warp, int num_sms,

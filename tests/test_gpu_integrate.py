@@ -4,7 +4,8 @@ with the pixels, rings around its capacity, boxes around its limits."""
 import numpy as np
 import pytest
 
-from caustic_b200 import problems
+from caustic_b200 import capi, problems
+from oracle import oracle as O
 from test_gpu_parity import check_eval, solver_for
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +53,31 @@ def test_rings_and_boxes_around_the_limits(gpu):
     c = s.eval_counters()
     assert (sizes > 16).any() and ((sizes > 8) & (sizes <= 16)).any(), np.bincount(sizes)
     assert c["integrated_first"] > 0 and c["integrations_split"] > 0, c
+
+
+@pytest.mark.parametrize("g,res", [(20, 1024), (40, 640), (72, 300)])
+def test_pixel_parts_of_large_and_small_cells(gpu, g, res):
+    """Weighted centroids and the render: cells that eight warps share (2,600
+    pixels), that one warp takes (256) and that four share a warp for (17)."""
+    p = problems.make(1, g=g, res=res)
+    w = np.random.default_rng(g).normal(0.0, 0.1 / p.n, p.n)
+    s = solver_for(p)
+    xy, ex = s.centroids(w, weighted=True)
+    c = O.cells(p.xy, w, O.proj_corner(p.xy, p.proj_domain))
+    oxy, oex = O.centers(c, p.picture, p.size, p.proj_domain, weighting=True)
+    assert np.array_equal(ex, oex)
+    assert np.abs(xy[ex] - oxy[ex]).max() < 1e-10
+    pxy, pex = s.centroids(w, weighted=False)
+    oxy, oex = O.centers(c, p.picture, p.size, p.proj_domain, weighting=False)
+    assert np.array_equal(pex, oex) and np.abs(pxy[pex] - oxy[pex]).max() < 1e-10
+    # each cell's mass is spread over its pixels in proportion to area: the
+    # whole is kept, and an all-equal density gives an even picture
+    img = s.render(w)
+    assert abs(img.sum() - p.nu.sum()) < 1e-10 * p.nu.sum()
+    _, mu, _, _ = s.eval(w)
+    flat = capi.Solver()
+    flat.set_problem(p.xy, np.ones(p.n) / p.n, np.ones(res * res), p.size, p.proj_domain)
+    area = flat.eval(w)[1] * 1.0
+    flat.set_problem(p.xy, area, np.ones(res * res), p.size, p.proj_domain)
+    img = flat.render(w)
+    assert np.abs(img * res * res - 1.0).max() < 1e-9
