@@ -17,9 +17,42 @@
 #include <cstring>
 #include <climits>
 #include <string>
+#include <utility>
 #include <vector>
 
+// Device buffers of one group in one allocation: add() notes a pointer and its
+// bytes, alloc() makes the block and sets the pointers.  A group is freed by
+// its block alone.
+struct Carve {
+    std::vector<std::pair<void **, size_t>> parts;
+    template <class T>
+    void add(T **p, size_t count)
+    {
+        parts.emplace_back(reinterpret_cast<void **>(p), std::max<size_t>(count * sizeof(T), 16));
+    }
+    cudaError_t alloc(void **block)
+    {
+        size_t total = 0;
+        for (auto &q : parts) total += (q.second + 255) & ~(size_t)255;
+        const cudaError_t e = cudaMalloc(block, total);
+        if (e != cudaSuccess) {
+            *block = nullptr;
+            return e;
+        }
+        unsigned char *at = static_cast<unsigned char *>(*block);
+        for (auto &q : parts) {
+            *q.first = at;
+            at += (q.second + 255) & ~(size_t)255;
+        }
+        return cudaSuccess;
+    }
+};
+
 struct CotProblemDev {
+    // the groups' blocks: sites and pixels, bucket grid, and what the first
+    // call that needs it makes (and keeps): a history longer than COT_HIST0,
+    // the Newton solve, the render
+    void *b_sites = nullptr, *b_grid = nullptr, *b_hist = nullptr, *b_newton = nullptr, *b_image = nullptr;
     int n = 0;
     int nb = 0;
     int nodes = 0;
@@ -40,11 +73,11 @@ struct CotProblemDev {
     double4 *tdyn = nullptr;
     double *rho = nullptr;
     int *perm = nullptr;   // sorted -> caller index
-    std::vector<int> hperm;
+    std::vector<int> hperm;  // its host copy, made when a call needs it
+    bool hperm_valid = false;
     CotGeo geo{};
     // per evaluation
     double *w = nullptr, *wt = nullptr, *d = nullptr, *mu = nullptr, *mut = nullptr, *fc = nullptr;
-    double *wq = nullptr;  // weights of the query entry points, apart from a solve's iterate w
     double *wbar = nullptr;
     int *blist = nullptr, *bcnt = nullptr;  // the bucket walk's leaf lists (solves only)
     double2 *rbuf = nullptr;  // ring vertices between the cell and integration kernels
@@ -61,7 +94,13 @@ struct CotProblemDev {
     double *partials = nullptr;
     unsigned int *ticket = nullptr;
     CotEvalOut *out = nullptr;
-    double *tmp = nullptr;  // caller-order staging (2n doubles)
+    double *tmp = nullptr;  // caller-order staging (COT_TMP(n) doubles)
+    // results of the centroids (sorted order, then caller order), the render,
+    // and the vectors of the Anderson solve
+    double *pcen = nullptr, *img = nullptr;
+    unsigned char *pex = nullptr;
+    double *aa_src = nullptr, *aa_inl = nullptr, *aa_insl = nullptr, *aa_hgt = nullptr, *aa_lam = nullptr;
+    double *aa_energy = nullptr, *aa_row = nullptr, *aa_coef = nullptr, *aa_step = nullptr;
     // solver
     CotSolver *S = nullptr;
     double *Sv = nullptr, *Yv = nullptr;
@@ -79,6 +118,10 @@ struct CotProblemDev {
     unsigned int *nticket = nullptr;
 };
 
+#define COT_HIST0 10                      // L-BFGS (or Anderson) memory that every problem has room for
+#define COT_TMP(n) (8 + 3 * (size_t)(n))  // an evaluation's scalars, then three vectors
+#define COT_STAGE_N 4096                  // sites up to which an evaluation's host vectors go through pinned memory
+
 struct cot_handle {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -92,6 +135,8 @@ struct cot_handle {
     cot::NewtonEvalStats *hN = nullptr;  // pinned copies of the Newton solve's trial statistics
     cot::PcgState *hP = nullptr;         // and of its inner solve's state
     unsigned char *hB = nullptr;         // pinned copy of the set-up's input statistics
+    double *hQ = nullptr;                // pinned vectors of small evaluations
+    unsigned char *pinned = nullptr;     // the block that holds these five
     // the device-driven trial loop's graph, kept while the problem, its
     // buffers and the stream stay the same (instantiating it costs more than
     // a short solve of a small problem)
@@ -146,24 +191,34 @@ __global__ void k_scatter(int n, const int *__restrict__ perm, const double *__r
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[perm[i]] = src[i];
 }
-__global__ void k_scatter2(int n, const int *__restrict__ perm, const double *__restrict__ src, double *__restrict__ dst)
+// Centroids and exist flags to caller order.
+__global__ void k_scatter_points(int n, const int *__restrict__ perm, const double *__restrict__ cen,
+                                 const unsigned char *__restrict__ ex, double *__restrict__ cen_out,
+                                 unsigned char *__restrict__ ex_out)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        dst[2 * perm[i]] = src[2 * i];
-        dst[2 * perm[i] + 1] = src[2 * i + 1];
-    }
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const size_t i = perm[p];
+    cen_out[2 * i] = cen[2 * (size_t)p];
+    cen_out[2 * i + 1] = cen[2 * (size_t)p + 1];
+    ex_out[i] = ex[p];
 }
-__global__ void k_scatter_u8(int n, const int *__restrict__ perm, const unsigned char *__restrict__ src,
-                             unsigned char *__restrict__ dst)
+
+// An evaluation's vectors in caller order (each nullable), and its scalars in
+// front of them (out, nullable).
+__global__ void k_eval_out(int n, const int *__restrict__ perm, const double *__restrict__ mut,
+                           const double *__restrict__ fc, const double *__restrict__ wt, const double *__restrict__ nu,
+                           const CotEvalOut *__restrict__ res, CotEvalOut *out, double *__restrict__ mu,
+                           double *__restrict__ g, double *__restrict__ fcell)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[perm[i]] = src[i];
-}
-__global__ void k_grad(int n, const double *__restrict__ mu, const double *__restrict__ nu, double *__restrict__ g)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) g[i] = mu[i] - nu[i];
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0 && out != nullptr) *out = *res;
+    if (p >= n) return;
+    const int i = perm[p];
+    const double m = mut[p];
+    if (mu) mu[i] = m;
+    if (g) g[i] = m - nu[p];
+    if (fcell) fcell[i] = fc[p] - wt[p] * nu[p];  // with its -w_i nu_i term (the cell kernels store it without)
 }
 
 static inline int nblk(int n) { return (n + 255) / 256; }
@@ -172,37 +227,33 @@ static inline int nblk(int n) { return (n + 255) / 256; }
 
 using namespace cot;
 
-// The buffers sized by the sites and pixels (with the Newton buffers and
-// the L-BFGS history, which are sized by the sites too).
+// The buffers sized by the sites and pixels (with those of the L-BFGS history,
+// the Newton and Anderson solves and the queries, which are sized by them too).
 static void free_sized_by_sites(CotProblemDev &P)
 {
-    void *ptrs[] = {P.xy, P.nu, P.sbucket, P.rho, P.perm, P.w, P.wt, P.d, P.mu, P.mut, P.wq, P.fc, P.rbuf, P.lbuf, P.flist,
-                    P.cstate, P.nv, P.ovf_list, P.ovf_list2, P.ovf_count, P.wlist, P.hsplit, P.hpart, P.hticket, P.nbc, P.nbn, P.nbc_q, P.nbn_q, P.partials,
-                    P.ticket, P.out, P.tmp, P.S, P.Sv, P.Yv, P.hval, P.hdiag, P.hbig_val, P.hcol, P.hcnt,
-                    P.hbig_col, P.herr, P.nb_b, P.nb_r, P.nb_z, P.nb_pa, P.nb_pb, P.nb_q, P.nb_part, P.nb_tau, P.pcg,
-                    P.nst, P.nticket, P.bpart, P.bticket, P.bstat, P.cubtmp};
-    for (void *p : ptrs)
+    void *blocks[] = {P.b_sites, P.b_hist, P.b_newton, P.b_image, P.cubtmp};
+    for (void *p : blocks)
         if (p) cudaFree(p);
-    P.xy = nullptr; P.nu = nullptr; P.sbucket = nullptr; P.rho = nullptr; P.perm = nullptr;
-    P.w = P.wt = P.d = P.mu = P.mut = P.wq = P.fc = nullptr;
-    P.rbuf = nullptr; P.lbuf = P.flist = P.cstate = P.nv = P.ovf_list = P.ovf_list2 = P.ovf_count = P.wlist = nullptr;
-    P.hsplit = nullptr; P.hpart = nullptr; P.hticket = nullptr;
-    P.nbc = P.nbn = P.nbc_q = P.nbn_q = nullptr;
-    P.partials = nullptr; P.ticket = nullptr; P.out = nullptr; P.tmp = nullptr; P.S = nullptr;
-    P.Sv = P.Yv = nullptr; P.hist_alloc = 0;
-    P.hval = P.hdiag = P.hbig_val = nullptr; P.hcol = P.hcnt = P.hbig_col = P.herr = nullptr; P.hbig_cap = 0;
-    P.nb_b = P.nb_r = P.nb_z = P.nb_pa = P.nb_pb = P.nb_q = P.nb_part = P.nb_tau = nullptr;
-    P.pcg = nullptr; P.nst = nullptr; P.nticket = nullptr;
-    P.bpart = nullptr; P.bticket = nullptr; P.bstat = nullptr; P.cubtmp = nullptr; P.cubtmp_bytes = 0;
-    P.cap_n = P.cap_pix = 0;
+    // the grid's group is the other function's
+    CotProblemDev keep;
+    keep.b_grid = P.b_grid;
+    keep.cap_nb = P.cap_nb;
+    keep.cap_nodes = P.cap_nodes;
+    keep.bstart = P.bstart;
+    keep.tstat = P.tstat;
+    keep.tdyn = P.tdyn;
+    keep.wbar = P.wbar;
+    keep.blist = P.blist;
+    keep.bcnt = P.bcnt;
+    keep.gen = P.gen;
+    P = std::move(keep);
 }
 
 // The buffers sized by the bucket grid and the tree.
 static void free_sized_by_grid(CotProblemDev &P)
 {
-    void *ptrs[] = {P.bstart, P.tstat, P.tdyn, P.wbar, P.blist, P.bcnt};
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
+    if (P.b_grid) cudaFree(P.b_grid);
+    P.b_grid = nullptr;
     P.bstart = nullptr; P.tstat = P.tdyn = nullptr; P.wbar = nullptr; P.blist = P.bcnt = nullptr;
     P.cap_nb = P.cap_nodes = 0;
 }
@@ -250,13 +301,18 @@ extern "C" int cot_create(const cot_config *cfg, cot_handle **out)
     e = cudaSetDevice(h->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->hS, sizeof(CotSolver));
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->hN, sizeof(NewtonEvalStats));
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->hP, sizeof(PcgState));
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->hB, 256);
+    const size_t at_n = (sizeof(CotSolver) + 255) & ~(size_t)255, at_p = at_n + 256, at_b = at_p + 256, at_q = at_b + 256;
+    static_assert(sizeof(NewtonEvalStats) <= 256 && sizeof(PcgState) <= 256, "one slot each");
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->pinned, at_q + COT_TMP(COT_STAGE_N) * sizeof(double));
+    if (e == cudaSuccess) {
+        h->hS = reinterpret_cast<CotSolver *>(h->pinned);
+        h->hN = reinterpret_cast<NewtonEvalStats *>(h->pinned + at_n);
+        h->hP = reinterpret_cast<PcgState *>(h->pinned + at_p);
+        h->hB = h->pinned + at_b;
+        h->hQ = reinterpret_cast<double *>(h->pinned + at_q);
+    }
     if (e != cudaSuccess) {
-        if (h->hS) cudaFreeHost(h->hS);
-        if (h->hN) cudaFreeHost(h->hN);
+        if (h->pinned) cudaFreeHost(h->pinned);
         if (h->own_stream) cudaStreamDestroy(h->own_stream);
         delete h;
         return fail(nullptr, COT_ECUDA, "cot_create", cudaGetErrorString(e));
@@ -290,10 +346,7 @@ extern "C" int cot_destroy(cot_handle *h)
         delete[] h->ctx.ev;
     }
     if (h->trial_exec) cudaGraphExecDestroy(h->trial_exec);
-    if (h->hS) cudaFreeHost(h->hS);
-    if (h->hN) cudaFreeHost(h->hN);
-    if (h->hP) cudaFreeHost(h->hP);
-    if (h->hB) cudaFreeHost(h->hB);
+    if (h->pinned) cudaFreeHost(h->pinned);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     delete h;
     return COT_OK;
@@ -381,46 +434,57 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
         P.cap_n = (size_t)n;
         P.cap_pix = npix;
         const size_t N = P.cap_n;
-        cudaError_t e = cudaSuccess;
-        auto A = [&](void **p, size_t bytes) {
-            if (e == cudaSuccess) e = cudaMalloc(p, bytes > 0 ? bytes : 16);
-        };
-        A((void **)&P.xy, N * sizeof(double2));
-        A((void **)&P.nu, N * 8);
-        A((void **)&P.sbucket, N * sizeof(int));
-        A((void **)&P.rho, P.cap_pix * 8);
-        A((void **)&P.perm, N * sizeof(int));
-        A((void **)&P.w, N * 8);
-        A((void **)&P.wt, N * 8);
-        A((void **)&P.wq, N * 8);
-        A((void **)&P.rbuf, ring_entries(N) * sizeof(double2));
-        A((void **)&P.lbuf, ring_entries(N) * sizeof(int));
-        A((void **)&P.flist, N * sizeof(int));
-        A((void **)&P.cstate, N * sizeof(int));
-        A((void **)&P.d, N * 8);
-        A((void **)&P.mu, N * 8);
-        A((void **)&P.mut, N * 8);
-        A((void **)&P.fc, N * 8);
-        A((void **)&P.nv, N * sizeof(int));
-        A((void **)&P.ovf_list, N * sizeof(int));
-        A((void **)&P.ovf_list2, N * sizeof(int));
-        A((void **)&P.ovf_count, 16 * sizeof(int));
-        A((void **)&P.wlist, N * sizeof(int));
-        A((void **)&P.hsplit, COT_HSPLIT_CAP * sizeof(int));
-        A((void **)&P.hpart, (size_t)COT_HSPLIT_CAP * COT_SPLIT * COT_PART * sizeof(double));
-        A((void **)&P.hticket, COT_HSPLIT_CAP * sizeof(unsigned int));
-        A((void **)&P.nbc, N * COT_NBC * sizeof(int));
-        A((void **)&P.nbn, N * sizeof(int));
-        A((void **)&P.nbc_q, N * COT_NBC * sizeof(int));
-        A((void **)&P.nbn_q, N * sizeof(int));
-        A((void **)&P.partials, (size_t)reduce_blocks((int)N) * (5 * COT_MAX_HIST + 8) * 8);
-        A((void **)&P.ticket, sizeof(unsigned int));
-        A((void **)&P.out, sizeof(CotEvalOut));
-        A((void **)&P.tmp, 2 * N * 8);
-        A((void **)&P.S, sizeof(CotSolver));
-        A((void **)&P.bpart, build_partials_doubles() * 8);
-        A((void **)&P.bticket, 2 * sizeof(unsigned int));
-        A((void **)&P.bstat, 256);
+        Carve c;
+        c.add(&P.xy, N);
+        c.add(&P.nu, N);
+        c.add(&P.sbucket, N);
+        c.add(&P.rho, P.cap_pix);
+        c.add(&P.perm, N);
+        c.add(&P.w, N);
+        c.add(&P.wt, N);
+        c.add(&P.rbuf, ring_entries(N));
+        c.add(&P.lbuf, ring_entries(N));
+        c.add(&P.flist, N);
+        c.add(&P.cstate, N);
+        c.add(&P.d, N);
+        c.add(&P.mu, N);
+        c.add(&P.mut, N);
+        c.add(&P.fc, N);
+        c.add(&P.nv, N);
+        c.add(&P.ovf_list, N);
+        c.add(&P.ovf_list2, N);
+        c.add(&P.ovf_count, 16);
+        c.add(&P.wlist, N);
+        c.add(&P.hsplit, COT_HSPLIT_CAP);
+        c.add(&P.hpart, (size_t)COT_HSPLIT_CAP * COT_SPLIT * COT_PART);
+        c.add(&P.hticket, COT_HSPLIT_CAP);
+        c.add(&P.nbc, N * COT_NBC);
+        c.add(&P.nbn, N);
+        c.add(&P.nbc_q, N * COT_NBC);
+        c.add(&P.nbn_q, N);
+        c.add(&P.partials, (size_t)reduce_blocks((int)N) * (5 * COT_MAX_HIST + 8));
+        c.add(&P.ticket, 1);
+        c.add(&P.out, 1);
+        c.add(&P.tmp, COT_TMP(N));
+        c.add(&P.S, 1);
+        c.add(&P.bpart, build_partials_doubles());
+        c.add(&P.bticket, 2);
+        c.add(&P.bstat, 256);
+        c.add(&P.Sv, COT_HIST0 * N);
+        c.add(&P.Yv, COT_HIST0 * N);
+        c.add(&P.pcen, 4 * N);
+        c.add(&P.pex, 2 * N);
+        c.add(&P.aa_src, 2 * N);
+        c.add(&P.aa_inl, 3 * N);
+        c.add(&P.aa_insl, 3 * N);
+        c.add(&P.aa_hgt, N);
+        c.add(&P.aa_lam, N);
+        c.add(&P.aa_energy, N);
+        c.add(&P.aa_row, COT_MAX_HIST);
+        c.add(&P.aa_coef, COT_MAX_HIST);
+        c.add(&P.aa_step, 1);
+        cudaError_t e = c.alloc(&P.b_sites);
+        if (e == cudaSuccess) P.hist_alloc = COT_HIST0;
         if (e == cudaSuccess) e = cudaMemsetAsync(P.bticket, 0, 2 * sizeof(unsigned int), s);
         if (e == cudaSuccess) e = cudaMemsetAsync(P.hticket, 0, COT_HSPLIT_CAP * sizeof(unsigned int), s);
         if (e != cudaSuccess) {
@@ -492,12 +556,14 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
         free_sized_by_grid(P);
         P.cap_nb = (size_t)nb;
         P.cap_nodes = (size_t)total;
-        cudaError_t e = cudaMalloc(&P.bstart, (P.cap_nb + 1) * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&P.tstat, P.cap_nodes * sizeof(double4));
-        if (e == cudaSuccess) e = cudaMalloc(&P.tdyn, P.cap_nodes * sizeof(double4));
-        if (e == cudaSuccess) e = cudaMalloc(&P.wbar, P.cap_nb * 8);
-        if (e == cudaSuccess) e = cudaMalloc(&P.blist, P.cap_nb * COT_BLEAF * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&P.bcnt, P.cap_nb * sizeof(int));
+        Carve c;
+        c.add(&P.bstart, P.cap_nb + 1);
+        c.add(&P.tstat, P.cap_nodes);
+        c.add(&P.tdyn, P.cap_nodes);
+        c.add(&P.wbar, P.cap_nb);
+        c.add(&P.blist, P.cap_nb * COT_BLEAF);
+        c.add(&P.bcnt, P.cap_nb);
+        const cudaError_t e = c.alloc(&P.b_grid);
         if (e != cudaSuccess) {
             free_sized_by_grid(P);
             return fail(h, COT_ENOMEM, "cot_set_problem: device allocation", cudaGetErrorString(e));
@@ -532,8 +598,7 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
     COT_CUDA_TRY(cudaMemsetAsync(P.nbn_q, 0, P.cap_n * sizeof(int), s));
     COT_CUDA_TRY(cudaMemsetAsync(P.bcnt, 0xff, P.cap_nb * sizeof(int), s));     // no bucket list yet
     if (P.hcnt) COT_CUDA_TRY(cudaMemsetAsync(P.hcnt, 0, P.cap_n * sizeof(int), s));
-    P.hperm.resize(n);
-    COT_CUDA_TRY(cudaMemcpyAsync(P.hperm.data(), P.perm, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, s));
+    P.hperm_valid = false;
     COT_CUDA_TRY(cudaStreamSynchronize(s));
 
     CotGeo &g = P.geo;
@@ -588,6 +653,35 @@ extern "C" int cot_set_problem(cot_handle *h, const double *sites_xy, const doub
     return COT_OK;
 }
 
+// The host copy of the sites' order.
+static int need_hperm(cot_handle *h, CotProblemDev &P)
+{
+    if (P.hperm_valid) return COT_OK;
+    P.hperm.resize(P.n);
+    COT_CUDA_TRY(cudaMemcpyAsync(P.hperm.data(), P.perm, (size_t)P.n * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    COT_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    P.hperm_valid = true;
+    return COT_OK;
+}
+
+// The weights of a query as a device vector in caller order: device arrays
+// are read in place, host arrays go to the staging vector (small ones through
+// pinned memory, which the caller's call does not wait for).
+static int query_weights(cot_handle *h, const double *w, int mem, const double **dev)
+{
+    CotProblemDev &P = h->P;
+    *dev = w;
+    if (mem == COT_MEM_DEVICE) return COT_OK;
+    const double *src = w;
+    if (P.n <= COT_STAGE_N) {
+        std::memcpy(h->hQ, w, (size_t)P.n * sizeof(double));
+        src = h->hQ;
+    }
+    COT_CUDA_TRY(cudaMemcpyAsync(P.tmp, src, (size_t)P.n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    *dev = P.tmp;
+    return COT_OK;
+}
+
 // Caller-order vector -> sorted device vector.
 static int upload_sorted(cot_handle *h, const double *src, int mem, double *dst)
 {
@@ -622,10 +716,14 @@ static int download_sorted(cot_handle *h, const double *src, double *dst, int me
     return COT_OK;
 }
 
-static CellsArgs cells_args(CotProblemDev &P, const double *w, const double *d, const double *tptr)
+// query: w is in caller order, and the entry point keeps its own neighbour
+// cache, so that a query made during a solve does not change the solve's clip
+// order.
+static CellsArgs cells_args(CotProblemDev &P, const double *w, const double *d, const double *tptr, bool query = false)
 {
     CellsArgs a{};
     a.w = w;
+    a.perm = query ? P.perm : nullptr;
     a.d = d;
     a.tptr = tptr;
     a.wt = P.wt;
@@ -645,10 +743,6 @@ static CellsArgs cells_args(CotProblemDev &P, const double *w, const double *d, 
     a.hpart = P.hpart;
     a.hticket = P.hticket;
     a.hsplit_cap = COT_HSPLIT_CAP;
-    // the query entry points (weights in P.wq) keep their own neighbour cache
-    // so that a query made during a solve does not change the solve's clip
-    // order
-    const bool query = (w == P.wq);
     a.nbc = query ? P.nbc_q : P.nbc;
     a.nbn = query ? P.nbn_q : P.nbn;
     // scratch of the bucket walk (rebuilt by every evaluation that uses it)
@@ -667,26 +761,46 @@ extern "C" int cot_eval(cot_handle *h, const double *w, double *f_total, double 
     CotProblemDev &P = h->P;
     cudaStream_t s = h->stream;
     int r;
-    if ((r = upload_sorted(h, w, mem, P.wq)) != COT_OK) return r;
-    CellsArgs a = cells_args(P, P.wq, nullptr, nullptr);
+    const double *dw;
+    if ((r = query_weights(h, w, mem, &dw)) != COT_OK) return r;
+    CellsArgs a = cells_args(P, dw, nullptr, nullptr, true);
     launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, h->c());
     launch_reduce(P.geo, P.mut, P.fc, P.nv, P.wt, nullptr, h->cfg.max_ring, P.partials, P.ticket, P.out, nullptr, h->c());
     COT_CUDA_TRY(cudaGetLastError());
     CotEvalOut o;
-    COT_CUDA_TRY(cudaMemcpyAsync(&o, P.out, sizeof o, cudaMemcpyDeviceToHost, s));
-    if (mu && (r = download_sorted(h, P.mut, mu, mem)) != COT_OK) return r;
-    // per-cell results staged in the second half of P.tmp (the first half
-    // is the scatter's staging); the solve's vectors stay untouched
-    double *stage = P.tmp + P.n;
-    if (f_cell) {
-        launch_fcell_full(P.n, P.fc, P.wt, P.nu, stage, h->c());
-        if ((r = download_sorted(h, stage, f_cell, mem)) != COT_OK) return r;
+    const size_t N = (size_t)P.n;
+    static_assert(sizeof(CotEvalOut) <= 8 * sizeof(double), "the scalars in front of the staging vectors");
+    // host results: the scalars and the vectors asked for, one after the
+    // other in the staging vectors; small ones come back in one copy
+    double *stage = P.tmp + 8;
+    double *dmu = mu, *dg = g, *df = f_cell;
+    size_t used = 0;
+    if (mem == COT_MEM_HOST) {
+        const auto place = [&](double *want) { return want ? stage + N * used++ : nullptr; };
+        dmu = place(mu);
+        dg = place(g);
+        df = place(f_cell);
     }
-    if (g) {
-        k_grad<<<nblk(P.n), 256, 0, s>>>(P.n, P.mut, P.nu, stage);
-        if ((r = download_sorted(h, stage, g, mem)) != COT_OK) return r;
+    k_eval_out<<<nblk(P.n), 256, 0, s>>>(P.n, P.perm, P.mut, P.fc, P.wt, P.nu, P.out,
+                                         reinterpret_cast<CotEvalOut *>(P.tmp), dmu, dg, df);
+    h->ctx.launches++;
+    COT_CUDA_TRY(cudaGetLastError());
+    if (mem == COT_MEM_HOST && P.n <= COT_STAGE_N) {
+        COT_CUDA_TRY(cudaMemcpyAsync(h->hQ, P.tmp, (8 + N * used) * sizeof(double), cudaMemcpyDeviceToHost, s));
+        COT_CUDA_TRY(cudaStreamSynchronize(s));
+        if (mu) std::memcpy(mu, h->hQ + (dmu - P.tmp), N * sizeof(double));
+        if (g) std::memcpy(g, h->hQ + (dg - P.tmp), N * sizeof(double));
+        if (f_cell) std::memcpy(f_cell, h->hQ + (df - P.tmp), N * sizeof(double));
+    } else {
+        COT_CUDA_TRY(cudaMemcpyAsync(h->hQ, P.tmp, sizeof o, cudaMemcpyDeviceToHost, s));
+        if (mem == COT_MEM_HOST) {
+            if (mu) COT_CUDA_TRY(cudaMemcpyAsync(mu, dmu, N * sizeof(double), cudaMemcpyDeviceToHost, s));
+            if (g) COT_CUDA_TRY(cudaMemcpyAsync(g, dg, N * sizeof(double), cudaMemcpyDeviceToHost, s));
+            if (f_cell) COT_CUDA_TRY(cudaMemcpyAsync(f_cell, df, N * sizeof(double), cudaMemcpyDeviceToHost, s));
+        }
+        COT_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    COT_CUDA_TRY(cudaStreamSynchronize(s));
+    std::memcpy(&o, h->hQ, sizeof o);
     if (f_total) *f_total = o.f;
     if (o.maxnv > 256) return failf(h, COT_ERING, "cot_eval: a cell has more than 256 vertices");
     return COT_OK;
@@ -711,11 +825,13 @@ extern "C" int cot_cells(cot_handle *h, const double *w, int *ring_offsets, doub
         cudaFree(rxy);
         return fail(h, COT_ENOMEM, "cot_cells: device allocation", cudaGetErrorString(e));
     }
-    int r = upload_sorted(h, w, COT_MEM_HOST, P.wq);
+    const double *dw;
+    int r = query_weights(h, w, COT_MEM_HOST, &dw);
+    if (r == COT_OK) r = need_hperm(h, P);
     std::vector<double> hxy;
     std::vector<int> hlab, hnv(N);
     if (r == COT_OK) {
-        CellsArgs a = cells_args(P, P.wq, nullptr, nullptr);
+        CellsArgs a = cells_args(P, dw, nullptr, nullptr, true);
         a.ring_xy = rxy;
         a.ring_lab = rlab;
         a.ring_cap = cap;
@@ -767,31 +883,24 @@ extern "C" int cot_centroids(cot_handle *h, const double *w, double *xy, unsigne
     cudaStream_t s = h->stream;
     size_t N = (size_t)P.n;
     int r;
-    if ((r = upload_sorted(h, w, mem, P.wq)) != COT_OK) return r;
-    double *cen = nullptr;
-    unsigned char *ex = nullptr, *ex2 = nullptr;
-    COT_CUDA_TRY(cudaMalloc(&cen, N * 2 * 8 * 2));
-    cudaError_t e = cudaMalloc(&ex, N * 2);
-    if (e != cudaSuccess) {
-        cudaFree(cen);
-        return fail(h, COT_ENOMEM, "cot_centroids: device allocation", cudaGetErrorString(e));
-    }
-    ex2 = ex + N;
-    CellsArgs a = cells_args(P, P.wq, nullptr, nullptr);
-    a.cen = cen;
-    a.exist = ex;
+    const double *dw;
+    if ((r = query_weights(h, w, mem, &dw)) != COT_OK) return r;
+    CellsArgs a = cells_args(P, dw, nullptr, nullptr, true);
+    a.cen = P.pcen;
+    a.exist = P.pex;
     a.weighted = weighted ? 1 : 0;
     launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, h->c());
-    double *cen2 = cen + 2 * N;
-    k_scatter2<<<nblk(P.n), 256, 0, s>>>(P.n, P.perm, cen, cen2);
-    k_scatter_u8<<<nblk(P.n), 256, 0, s>>>(P.n, P.perm, ex, ex2);
-    cudaMemcpyKind k = mem == COT_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    e = cudaMemcpyAsync(xy, cen2, N * 2 * 8, k, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(exist, ex2, N, k, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(cen);
-    cudaFree(ex);
-    if (e != cudaSuccess) return fail(h, COT_ECUDA, "cot_centroids", cudaGetErrorString(e));
+    const bool host = mem != COT_MEM_DEVICE;
+    double *xy_out = host ? P.pcen + 2 * N : xy;
+    unsigned char *ex_out = host ? P.pex + N : exist;
+    k_scatter_points<<<nblk(P.n), 256, 0, s>>>(P.n, P.perm, P.pcen, P.pex, xy_out, ex_out);
+    h->ctx.launches++;
+    COT_CUDA_TRY(cudaGetLastError());
+    if (host) {
+        COT_CUDA_TRY(cudaMemcpyAsync(xy, xy_out, N * 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+        COT_CUDA_TRY(cudaMemcpyAsync(exist, ex_out, N, cudaMemcpyDeviceToHost, s));
+    }
+    COT_CUDA_TRY(cudaStreamSynchronize(s));
     return COT_OK;
 }
 
@@ -827,7 +936,8 @@ static int source_masses_impl(cot_handle *h, const double *points_xy, int n, con
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (solid) cudaFree(solid);
-    std::vector<int> perm = Q.hperm;
+    if (e == cudaSuccess && need_hperm(h, Q) != COT_OK) e = cudaErrorUnknown;
+    const std::vector<int> perm = Q.hperm;
     free_problem(Q);
     if (e != cudaSuccess) return fail(h, COT_ECUDA, "cot_source_masses", cudaGetErrorString(e));
     const double dom = (sd[1] - sd[0]) * (sd[3] - sd[2]);
@@ -872,21 +982,22 @@ extern "C" int cot_render(cot_handle *h, const double *w, double gray_multiple, 
     CotProblemDev &P = h->P;
     cudaStream_t s = h->stream;
     const size_t npx = (size_t)P.geo.nx * P.geo.ny;
-    double *img = nullptr;
-    COT_CUDA_TRY(cudaMalloc(&img, npx * 8));
-    int r = upload_sorted(h, w, COT_MEM_HOST, P.wq);
-    cudaError_t e = cudaMemsetAsync(img, 0, npx * 8, s);
-    if (r == COT_OK && e == cudaSuccess) {
-        CellsArgs a = cells_args(P, P.wq, nullptr, nullptr);
-        a.splat = img;
-        a.splat_scale = gray_multiple;
-        launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, h->c());
-        e = cudaMemcpyAsync(out, img, npx * 8, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (!P.b_image) {
+        Carve c;
+        c.add(&P.img, P.cap_pix);
+        const cudaError_t e = c.alloc(&P.b_image);
+        if (e != cudaSuccess) return fail(h, COT_ENOMEM, "cot_render: device allocation", cudaGetErrorString(e));
     }
-    cudaFree(img);
-    if (r != COT_OK) return r;
-    if (e != cudaSuccess) return fail(h, COT_ECUDA, "cot_render", cudaGetErrorString(e));
+    int r;
+    const double *dw;
+    if ((r = query_weights(h, w, COT_MEM_HOST, &dw)) != COT_OK) return r;
+    COT_CUDA_TRY(cudaMemsetAsync(P.img, 0, npx * sizeof(double), s));
+    CellsArgs a = cells_args(P, dw, nullptr, nullptr, true);
+    a.splat = P.img;
+    a.splat_scale = gray_multiple;
+    launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, h->c());
+    COT_CUDA_TRY(cudaMemcpyAsync(out, P.img, npx * sizeof(double), cudaMemcpyDeviceToHost, s));
+    COT_CUDA_TRY(cudaStreamSynchronize(s));
     return COT_OK;
 }
 
@@ -1016,6 +1127,27 @@ static int build_trial_graph(cot_handle *h, double *tptr, cudaGraphExec_t *exec,
     return COT_OK;
 }
 
+// Room for a history of m pairs.
+static int need_history(cot_handle *h, int m)
+{
+    CotProblemDev &P = h->P;
+    if (P.hist_alloc >= m) return COT_OK;
+    void *old = P.b_hist;
+    // sized for the buffers' capacity: a later problem that fits them reuses these
+    Carve hc;
+    hc.add(&P.Sv, (size_t)m * P.cap_n);
+    hc.add(&P.Yv, (size_t)m * P.cap_n);
+    const cudaError_t e = hc.alloc(&P.b_hist);
+    if (e != cudaSuccess) {
+        P.b_hist = old;  // the shorter history stays
+        return fail(h, COT_ENOMEM, "solve: history allocation", cudaGetErrorString(e));
+    }
+    if (old) cudaFree(old);
+    P.hist_alloc = m;
+    P.gen = ++g_problem_gen;  // a graph that captured the old history buffers is stale
+    return COT_OK;
+}
+
 // History buffers and the device control block of a solve from the weights
 // in P.w, on the handle's stream.
 static int solve_prepare(cot_handle *h, const cot_solve_opts &o, int stop_nonempty = 0)
@@ -1024,18 +1156,8 @@ static int solve_prepare(cot_handle *h, const cot_solve_opts &o, int stop_nonemp
     cudaStream_t s = h->stream;
     const int n = P.n;
     const int m = o.history;
-    if (P.hist_alloc < m) {
-        if (P.Sv) cudaFree(P.Sv);
-        if (P.Yv) cudaFree(P.Yv);
-        P.Sv = P.Yv = nullptr;
-        P.hist_alloc = 0;
-        // sized for the buffers' capacity: a later problem that fits them reuses these
-        cudaError_t e = cudaMalloc(&P.Sv, (size_t)m * P.cap_n * 8);
-        if (e == cudaSuccess) e = cudaMalloc(&P.Yv, (size_t)m * P.cap_n * 8);
-        if (e != cudaSuccess) return fail(h, COT_ENOMEM, "solve: history allocation", cudaGetErrorString(e));
-        P.hist_alloc = m;
-        P.gen = ++g_problem_gen;  // a graph that captured the old history buffers is stale
-    }
+    int rh;
+    if ((rh = need_history(h, m)) != COT_OK) return rh;
     COT_CUDA_TRY(cudaMemsetAsync(P.Sv, 0, (size_t)m * n * 8, s));
     COT_CUDA_TRY(cudaMemsetAsync(P.Yv, 0, (size_t)m * n * 8, s));
     CotSolver &hs = *h->hS;
@@ -1422,6 +1544,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
     cudaStream_t s = h->stream;
     const int n = P.n;
     const size_t N = (size_t)n;
+    if ((r = need_hperm(h, P)) != COT_OK) return r;
     // sorted copies of the per-site inputs
     const std::vector<int> &perm = P.hperm;
     std::vector<double> src(2 * N), inl(3 * N), insl(3 * N), hgt(N);
@@ -1436,33 +1559,14 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
         hgt[p] = in->height[i];
     }
     // device workspace of this call
-    double *dsrc = nullptr, *dinl = nullptr, *dinsl = nullptr, *dhgt = nullptr, *lam = nullptr, *energy = nullptr;
-    double *cen = nullptr, *G = nullptr, *F = nullptr, *row = nullptr, *coef = nullptr, *step = nullptr;
-    unsigned char *ex = nullptr;
-    auto release = [&]() {
-        void *ps[] = {dsrc, dinl, dinsl, dhgt, lam, energy, cen, G, F, row, coef, step, ex};
-        for (void *q : ps)
-            if (q) cudaFree(q);
-    };
-    cudaError_t e = cudaMalloc(&dsrc, 2 * N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&dinl, 3 * N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&dinsl, 3 * N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&dhgt, N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&lam, N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&energy, N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&cen, 2 * N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&ex, N);
-    if (e == cudaSuccess) e = cudaMalloc(&G, (size_t)M * N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&F, (size_t)M * N * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&row, COT_MAX_HIST * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&coef, COT_MAX_HIST * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&step, 8);
-    if (e != cudaSuccess) {
-        release();
-        return fail(h, COT_ENOMEM, "cot_solve_aarl: device allocation", cudaGetErrorString(e));
-    }
+    // the Anderson history takes the L-BFGS history's place, which is free
+    // again when its phase begins
+    if ((r = need_history(h, std::max(M, o.history))) != COT_OK) return r;
+    double *dsrc = P.aa_src, *dinl = P.aa_inl, *dinsl = P.aa_insl, *dhgt = P.aa_hgt, *lam = P.aa_lam;
+    double *energy = P.aa_energy, *cen = P.pcen, *G = P.Sv, *F = P.Yv, *row = P.aa_row, *coef = P.aa_coef;
+    double *step = P.aa_step;
+    unsigned char *ex = P.pex;
     auto cuda_fail = [&](const char *what, cudaError_t err) {
-        release();
         return fail(h, COT_ECUDA, what, cudaGetErrorString(err));
     };
 #define AARL_TRY(expr)                                  \
@@ -1482,7 +1586,6 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
     double area_scalar = 0;
     for (double v : hl) area_scalar += v;
     if ((r = upload_sorted(h, w_inout, COT_MEM_HOST, P.w)) != COT_OK) {
-        release();
         return r;
     }
     cudaEvent_t e0, e1;
@@ -1500,20 +1603,19 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
         a.weighted = 0;
         launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, h->c());
         evals++;
-        // ring check first (polygons_in_VD + the max_edge_num/2 test)
+        // ring check first (polygons_in_VD + the max_edge_num/2 test): the
+        // re-weighting leaves nu alone when a ring is too complex
         launch_reduce(P.geo, P.mut, P.fc, P.nv, P.wt, nullptr, h->cfg.max_ring, P.partials, P.ticket, P.out, nullptr, h->c());
-        cudaError_t err = cudaMemcpyAsync(&ho, P.out, sizeof ho, cudaMemcpyDeviceToHost, s);
-        if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-        if (err != cudaSuccess) return -1;
-        if (ho.overflow > 0) return 1;
         if (update_nu) {
             launch_fresnel_nu(n, cen, dsrc, dinl, dinsl, dhgt, lam, in->z_of_len, in->z_of_receiver,
-                              in->refraction_index, area_scalar, energy, P.partials, P.nu, h->c());
+                              in->refraction_index, area_scalar, energy, P.partials, P.out, P.nu, h->c());
             launch_reduce(P.geo, P.mut, P.fc, P.nv, P.wt, nullptr, h->cfg.max_ring, P.partials, P.ticket, P.out, nullptr, h->c());
-            err = cudaMemcpyAsync(&ho, P.out, sizeof ho, cudaMemcpyDeviceToHost, s);
-            if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-            if (err != cudaSuccess) return -1;
         }
+        cudaError_t err = cudaMemcpyAsync(h->hQ, P.out, sizeof ho, cudaMemcpyDeviceToHost, s);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+        if (err != cudaSuccess) return -1;
+        std::memcpy(&ho, h->hQ, sizeof ho);
+        if (ho.overflow > 0) return 1;
         return 0;
     };
     // 1. nu from the centroids at the warm start
@@ -1532,8 +1634,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
             }
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
-            release();
-        }
+            }
         return rr;
     };
     if ((r = report_start(COT_PHASE_PREPASS)) != COT_OK) return r;
@@ -1548,8 +1649,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
             }
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
-            release();
-            return r;
+                return r;
         }
         evals += pre.evals;
         // 3. nu again from the centroids at the pre-pass result
@@ -1577,8 +1677,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
         for (int i = 0; i < cnt; i++)
             for (int j = 0; j < cnt; j++) As[(size_t)i * cnt + j] = A[(size_t)i * M + j] + (i == j ? 1e-10 : 0.0);
         if (!ldlt_solve_ones(As, cnt, a)) {
-            release();
-            return fail(h, COT_ENOTCONV, "cot_solve_aarl: singular Anderson system", nullptr);
+                return fail(h, COT_ENOTCONV, "cot_solve_aarl: singular Anderson system", nullptr);
         }
         double sa = 0;
         for (double v : a) sa += v;
@@ -1636,8 +1735,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
                 }
                 cudaEventDestroy(e0);
                 cudaEventDestroy(e1);
-                release();
-                return r;
+                        return r;
             }
         }
         if (conv_now) {
@@ -1647,7 +1745,6 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
     }
     AARL_TRY(cudaEventRecord(e1, s));
     if ((r = download_sorted(h, P.w, w_inout, COT_MEM_HOST)) != COT_OK) {
-        release();
         return r;
     }
     AARL_TRY(cudaStreamSynchronize(s));
@@ -1655,7 +1752,6 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    release();
 #undef AARL_TRY
     if (stats) {
         stats->iterations = iters;
@@ -1693,38 +1789,28 @@ static int newton_alloc(cot_handle *h)
     const size_t N = P.cap_n;
     const int pcg_blocks = pcg_max_blocks((int)N, h->num_sms);
     P.hbig_cap = std::max(16, std::min((int)N, 4096));
-    cudaError_t e = cudaSuccess;
-    auto A = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, bytes > 0 ? bytes : 16);
-    };
-    A((void **)&P.hval, 32 * N * sizeof(double));
-    A((void **)&P.hcol, 32 * N * sizeof(int));
-    A((void **)&P.hcnt, N * sizeof(int));
-    A((void **)&P.hdiag, N * sizeof(double));
-    A((void **)&P.hbig_val, (size_t)P.hbig_cap * COT_HBIG_W * sizeof(double));
-    A((void **)&P.hbig_col, (size_t)P.hbig_cap * COT_HBIG_W * sizeof(int));
-    A((void **)&P.herr, sizeof(int));
-    A((void **)&P.nb_b, N * 8);
-    A((void **)&P.nb_r, N * 8);
-    A((void **)&P.nb_z, N * 8);
-    A((void **)&P.nb_pa, N * 8);
-    A((void **)&P.nb_pb, N * 8);
-    A((void **)&P.nb_q, N * 8);
-    A((void **)&P.nb_part, (size_t)std::max(6 * pcg_blocks + 48, 256 * 5) * 8);
-    A((void **)&P.nb_tau, 8);
-    A((void **)&P.pcg, sizeof(PcgState));
-    A((void **)&P.nst, sizeof(NewtonEvalStats));
-    A((void **)&P.nticket, sizeof(unsigned int));
+    Carve c;
+    c.add(&P.hval, 32 * N);
+    c.add(&P.hcol, 32 * N);
+    c.add(&P.hcnt, N);
+    c.add(&P.hdiag, N);
+    c.add(&P.hbig_val, (size_t)P.hbig_cap * COT_HBIG_W);
+    c.add(&P.hbig_col, (size_t)P.hbig_cap * COT_HBIG_W);
+    c.add(&P.herr, 1);
+    c.add(&P.nb_b, N);
+    c.add(&P.nb_r, N);
+    c.add(&P.nb_z, N);
+    c.add(&P.nb_pa, N);
+    c.add(&P.nb_pb, N);
+    c.add(&P.nb_q, N);
+    c.add(&P.nb_part, (size_t)std::max(6 * pcg_blocks + 48, 256 * 5));
+    c.add(&P.nb_tau, 1);
+    c.add(&P.pcg, 1);
+    c.add(&P.nst, 1);
+    c.add(&P.nticket, 1);
+    const cudaError_t e = c.alloc(&P.b_newton);
     if (e != cudaSuccess) {
-        void *ptrs[] = {P.hval, P.hcol, P.hcnt, P.hdiag, P.hbig_val, P.hbig_col, P.herr, P.nb_b, P.nb_r, P.nb_z,
-                        P.nb_pa, P.nb_pb, P.nb_q, P.nb_part, P.nb_tau, P.pcg, P.nst, P.nticket};
-        for (void *p : ptrs)
-            if (p) cudaFree(p);
-        P.hval = P.hdiag = P.hbig_val = P.nb_b = P.nb_r = P.nb_z = P.nb_pa = P.nb_pb = P.nb_q = P.nb_part = P.nb_tau = nullptr;
-        P.hcol = P.hcnt = P.hbig_col = P.herr = nullptr;
-        P.pcg = nullptr;
-        P.nst = nullptr;
-        P.nticket = nullptr;
+        // alloc() left the pointers as they were: none set
         return fail(h, COT_ENOMEM, "cot_solve_newton: device allocation", cudaGetErrorString(e));
     }
     COT_CUDA_TRY(cudaMemsetAsync(P.nticket, 0, sizeof(unsigned int), h->stream));
@@ -1734,9 +1820,10 @@ static int newton_alloc(cot_handle *h)
 
 // CellsArgs of an evaluation that keeps what the Jacobian needs: the final
 // rings' generators and the long rings' rows.
-static CellsArgs jacobian_args(CotProblemDev &P, const double *w, const double *d, const double *tptr)
+static CellsArgs jacobian_args(CotProblemDev &P, const double *w, const double *d, const double *tptr,
+                               bool query = false)
 {
-    CellsArgs a = cells_args(P, w, d, tptr);
+    CellsArgs a = cells_args(P, w, d, tptr, query);
     a.keep_labels = 1;
     a.hbig_val = P.hbig_val;
     a.hbig_col = P.hbig_col;
@@ -1774,8 +1861,10 @@ extern "C" int cot_mass_jacobian(cot_handle *h, const double *w, int mem, int *r
     if ((r = newton_alloc(h)) != COT_OK) return r;
     CotProblemDev &P = h->P;
     cudaStream_t s = h->stream;
-    if ((r = upload_sorted(h, w, mem, P.wq)) != COT_OK) return r;
-    CellsArgs a = jacobian_args(P, P.wq, nullptr, nullptr);
+    if ((r = need_hperm(h, P)) != COT_OK) return r;
+    const double *dw;
+    if ((r = query_weights(h, w, mem, &dw)) != COT_OK) return r;
+    CellsArgs a = jacobian_args(P, dw, nullptr, nullptr, true);
     COT_CUDA_TRY(cudaMemsetAsync(P.herr, 0, sizeof(int), s));
     launch_eval(P.geo, a, 1, h->num_sms, h->c());
     launch_hessian(P.geo, P.rbuf, P.lbuf, P.nv, P.hval, P.hcol, P.hcnt, P.hdiag, h->c());

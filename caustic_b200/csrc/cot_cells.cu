@@ -118,7 +118,8 @@ __device__ __forceinline__ double bseg_max(double v, unsigned m)
 
 // Trial weights of bucket b's sites and their mean phi (0 for an empty
 // bucket).  Block 0 also clears the cell kernels' counters.
-__global__ void k_bucket_phi(CotGeo g, const double *__restrict__ w, const double *__restrict__ d,
+__global__ void k_bucket_phi(CotGeo g, const double *__restrict__ w, const int *__restrict__ perm,
+                             const double *__restrict__ d,
                              const double *__restrict__ tptr, double *__restrict__ wt,
                              double *__restrict__ wbar, int *counters, int ncounters)
 {
@@ -131,7 +132,7 @@ __global__ void k_bucket_phi(CotGeo g, const double *__restrict__ w, const doubl
     const int s0 = g.bstart[b], s1 = g.bstart[b + 1];
     double acc = 0.0;
     for (int j = s0 + sl; j < s1; j += BSEG) {
-        const double wj = trial_weight(w, d, t, j);
+        const double wj = perm != nullptr ? w[perm[j]] : trial_weight(w, d, t, j);
         wt[j] = wj;
         acc = __dadd_rn(acc, wj);
     }
@@ -3867,7 +3868,7 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     // [13]: the split integration list's size, [14], [15]: flist's sizes for
     // k_cells_first and k_cells_walk
     const int segs = (nb * BSEG + 127) / 128;
-    k_bucket_phi<<<segs, 128, 0, s>>>(g, a.w, a.d, a.tptr, a.wt, a.wbar, a.ovf_count, 16);
+    k_bucket_phi<<<segs, 128, 0, s>>>(g, a.w, a.perm, a.d, a.tptr, a.wt, a.wbar, a.ovf_count, 16);
     k_tree_build<<<(nb * BSEG + TREE_THREADS - 1) / TREE_THREADS, TREE_THREADS, 0, s>>>(g, a.wt, a.wbar);
     c.launches += 2;
     int upper = 0;  // nodes of levels 1..lmax

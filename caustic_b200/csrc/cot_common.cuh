@@ -134,6 +134,7 @@ inline size_t ring_entries(size_t n) { return (n + 31) / 32 * 1024; }
 // Launchers implemented in cot_cells.cu.
 struct CellsArgs {
     const double *w;       // weights (base point)
+    const int *perm;       // w in caller order: site j's is w[perm[j]] (nullable: sorted)
     const double *d;       // direction (nullable)
     const double *tptr;    // device scalar step (nullable => 0)
     double *wt;            // trial weights out
@@ -257,10 +258,9 @@ cudaError_t launch_pcg(int n, const double *hval, const int *hcol, const int *hc
                        const int *hbig_col, const double *hdiag, const double *b, double *x, double *r, double *z,
                        double *pa, double *pb, double *q, double *partials, PcgState *st, double rtol, int max_it,
                        int blocks, CotCtx &c);
-void launch_fcell_full(int n, const double *fc, const double *wt, const double *nu, double *out, CotCtx &c);
 void launch_fresnel_nu(int n, const double *cen, const double *src, const double *inl, const double *insl,
                        const double *hgt, const double *lam, double zl, double zr, double eta, double total,
-                       double *energy, double *partials, double *nu, CotCtx &c);
+                       double *energy, double *partials, const CotEvalOut *eval, double *nu, CotCtx &c);
 void launch_aa_store_gram(int n, const double *w, const double *mu, const double *nu, double alpha, double *G,
                           double *F, int h, int cnt, double *partials, unsigned int *ticket, double *row, CotCtx &c);
 void launch_aa_combine(int n, const double *F, const double *coef, int cnt, const double *w, double *d, CotCtx &c);

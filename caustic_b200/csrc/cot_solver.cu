@@ -612,20 +612,6 @@ void launch_init_from_eval(CotSolver *S, const CotEvalOut *out, CotCtx &c)
 // helpers of cot_eval and of the Fresnel-reweighted Anderson solve
 // ---------------------------------------------------------------------------
 
-// f_i with its -w_i nu_i term (the cell kernels store it without)
-__global__ void k_fcell_full(int n, const double *__restrict__ fc, const double *__restrict__ wt,
-                             const double *__restrict__ nu, double *__restrict__ out)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = fc[i] - wt[i] * nu[i];
-}
-
-void launch_fcell_full(int n, const double *fc, const double *wt, const double *nu, double *out, CotCtx &c)
-{
-    k_fcell_full<<<(n + 255) / 256, 256, 0, c.s>>>(n, fc, wt, nu, out);
-    c.launches++;
-}
-
 // fresnel_T_unpolarized (basic_function.cuh:407-435)
 __device__ double fresnel_t(const double wi[3], const double wt[3], const double nrm[3], double eta_i, double eta_t)
 {
@@ -693,10 +679,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_sum_partials(int n, const doubl
     if (threadIdx.x == 0) partials[blockIdx.x] = v;
 }
 
-// nu_i = energy_i / sum(energy) * total
+// nu_i = energy_i / sum(energy) * total, unless the evaluation it comes from
+// had rings that are too complex
 __global__ void k_scale_to_total(int n, const double *__restrict__ energy, const double *__restrict__ partials,
-                                 int nparts, double total, double *__restrict__ nu)
+                                 int nparts, double total, const CotEvalOut *__restrict__ eval,
+                                 double *__restrict__ nu)
 {
+    if (eval->overflow > 0) return;
     double s = 0.0;
     for (int k = 0; k < nparts; k++) s += partials[k];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -705,12 +694,12 @@ __global__ void k_scale_to_total(int n, const double *__restrict__ energy, const
 
 void launch_fresnel_nu(int n, const double *cen, const double *src, const double *inl, const double *insl,
                        const double *hgt, const double *lam, double zl, double zr, double eta, double total,
-                       double *energy, double *partials, double *nu, CotCtx &c)
+                       double *energy, double *partials, const CotEvalOut *eval, double *nu, CotCtx &c)
 {
     k_fresnel_energy<<<(n + 255) / 256, 256, 0, c.s>>>(n, cen, src, inl, insl, hgt, lam, zl, zr, eta, energy);
     int nb = reduce_blocks(n);
     k_sum_partials<<<nb, RED_THREADS, 0, c.s>>>(n, energy, partials);
-    k_scale_to_total<<<(n + 255) / 256, 256, 0, c.s>>>(n, energy, partials, nb, total, nu);
+    k_scale_to_total<<<(n + 255) / 256, 256, 0, c.s>>>(n, energy, partials, nb, total, eval, nu);
     c.launches += 3;
 }
 
