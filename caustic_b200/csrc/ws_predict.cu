@@ -4,7 +4,7 @@
 // the BF16 weights and FP32 biases on the device, prepares the inputs of one
 // problem on the host exactly as warmstart.make_input does, and runs the
 // forward pass with the same kernels the Python host layer strings together
-// (ws_im2col, ws_gemm, ws_bias_act, ws_pool2, ws_up2, ws_put_channels).
+// (ws_im2col, ws_im2col_up, ws_layer, ws_pool2, ws_gemm).
 // No counterpart in the reference: its solver starts from the previous
 // outer iteration's weights or from zero (main.cu:193-198).
 #include <cuda_bf16.h>
@@ -254,15 +254,25 @@ extern "C" WS_API int cot_warmstart_predict(ws_net *net, const double *sites_xy,
     size_t ws_bytes = 0;
     void *wsp = nullptr;
     // one convolution: x [H][W][cin] bf16 -> fp32 d [H*W][cout]; with a bias,
-    // y = act(d + b) in bf16
-    auto conv = [&](const Layer &L, const __nv_bfloat16 *in, int H, int W, float **d_out) -> __nv_bfloat16 * {
+    // y = relu(d + b) in bf16.  skip: the input is x, upsampled, and skip's
+    // channels after it.
+    auto conv = [&](const Layer &L, const __nv_bfloat16 *in, int H, int W, float **d_out,
+                    const __nv_bfloat16 *skip = nullptr, int cskip = 0) -> __nv_bfloat16 * {
         const int M = H * W, K = L.k * L.k * L.cin;
         const void *cols = in;
         if (L.k == 3) {
             auto *c = pool.get<__nv_bfloat16>((size_t)M * K, e);
             if (e != cudaSuccess) return nullptr;
-            if ((rc = ws_im2col(1, H, W, L.cin, in, c, s)) != WS_OK) return nullptr;
+            rc = skip ? ws_im2col_up(1, H, W, L.cin - cskip, in, cskip, skip, c, s)
+                      : ws_im2col(1, H, W, L.cin, in, c, s);
+            if (rc != WS_OK) return nullptr;
             cols = c;
+        }
+        if (L.has_bias) {
+            auto *y = pool.get<__nv_bfloat16>((size_t)M * L.cout, e);
+            if (e != cudaSuccess) return nullptr;
+            if ((rc = ws_layer(M, L.cout, K, cols, L.w16, L.b, y, s)) != WS_OK) return nullptr;
+            return y;
         }
         float *d = pool.get<float>((size_t)M * L.cout, e);
         const size_t need = ws_gemm_workspace(WS_GEMM_RC, M, L.cout, K);
@@ -275,11 +285,7 @@ extern "C" WS_API int cot_warmstart_predict(ws_net *net, const double *sites_xy,
             WS_OK)
             return nullptr;
         if (d_out) *d_out = d;
-        if (!L.has_bias) return nullptr;
-        auto *y = pool.get<__nv_bfloat16>((size_t)M * L.cout, e);
-        if (e != cudaSuccess) return nullptr;
-        if ((rc = ws_bias_act(M, L.cout, d, L.b, 1, y, nullptr, s)) != WS_OK) return nullptr;
-        return y;
+        return nullptr;
     };
     const int levels = net->levels;
     std::vector<const __nv_bfloat16 *> skips(levels);
@@ -301,19 +307,12 @@ extern "C" WS_API int cot_warmstart_predict(ws_net *net, const double *sites_xy,
         }
     }
     for (int l = levels - 2; l >= 0; l--) {
-        const int ct = net->ch[l + 1] + net->ch[l];
-        auto *cat = pool.get<__nv_bfloat16>((size_t)(2 * H) * (2 * W) * ct, e);
-        if (e != cudaSuccess) goto fail;
-        if ((rc = ws_up2(1, H, W, net->ch[l + 1], cur, ct, 0, cat, s)) != WS_OK) goto fail;
         H *= 2;
         W *= 2;
-        if ((rc = ws_put_channels((long long)H * W, net->ch[l], skips[l], ct, net->ch[l + 1], cat, s)) != WS_OK)
-            goto fail;
-        cur = cat;
-        for (int t = 0; t < 2; t++) {
-            cur = conv(net->layers[q++], cur, H, W, nullptr);
-            if (!cur) goto fail;
-        }
+        cur = conv(net->layers[q++], cur, H, W, nullptr, skips[l], net->ch[l]);
+        if (!cur) goto fail;
+        cur = conv(net->layers[q++], cur, H, W, nullptr);
+        if (!cur) goto fail;
     }
     {
         float *d = nullptr;

@@ -16,7 +16,12 @@
 #include <cutlass/gemm/kernel/gemm_universal.hpp>
 #include <cutlass/gemm/collective/collective_builder.hpp>
 #include <cutlass/epilogue/collective/collective_builder.hpp>
+#include <cutlass/epilogue/fusion/operations.hpp>
+#include <cutlass/epilogue/thread/activation.h>
 #include <cutlass/util/packed_stride.hpp>
+
+#include <algorithm>
+#include <initializer_list>
 
 #include "../../include/causticws.h"
 
@@ -29,10 +34,10 @@ using bf16 = __nv_bfloat16;
 // ---------------------------------------------------------------------------
 // One GEMM configuration per operand layout: 128x128x64 tiles on one SM,
 // fp32 accumulators in tensor memory, fp32 output.
-#define WS_GEMM_CONFIG(NAME, LA, LB)                                                                                \
+#define WS_GEMM_CONFIG(NAME, LA, LB, MT, NT)                                                                        \
     namespace NAME {                                                                                                \
     using ElemAB = cutlass::bfloat16_t;                                                                            \
-    using Tile = cute::Shape<cute::_128, cute::_128, cute::_64>;                                                   \
+    using Tile = cute::Shape<cute::Int<MT>, cute::Int<NT>, cute::_64>;                                             \
     using Cluster = cute::Shape<cute::_1, cute::_1, cute::_1>;                                                     \
     using Epilogue = cutlass::epilogue::collective::CollectiveBuilder<                                             \
         cutlass::arch::Sm100, cutlass::arch::OpClassTensorOp, Tile, Cluster,                                       \
@@ -72,13 +77,281 @@ using bf16 = __nv_bfloat16;
     }
 
 // A[M,K] K-contiguous, B stored [N][K]  (forward: D = cols W^T)
-WS_GEMM_CONFIG(GemmRC, cutlass::layout::RowMajor, cutlass::layout::ColumnMajor)
+WS_GEMM_CONFIG(GemmRC, cutlass::layout::RowMajor, cutlass::layout::ColumnMajor, 128, 128)
 // A stored [K][M], B[K,N] N-contiguous   (weight gradient: dW = dZ^T cols)
-WS_GEMM_CONFIG(GemmCR, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor)
+WS_GEMM_CONFIG(GemmCR, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor, 128, 128)
+// the same with narrow tiles: a weight gradient has few of them and thousands
+// of rows to add up.  Its rows are one chain of sums in the tensor memory, in
+// order (sharing them out would round elsewhere), so more and lighter tiles
+// are what shortens it.
+WS_GEMM_CONFIG(GemmCR32, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor, 64, 64)
 // A[M,K], B[K,N] both row-major         (input gradient: dcols = dZ W)
-WS_GEMM_CONFIG(GemmRR, cutlass::layout::RowMajor, cutlass::layout::RowMajor)
+WS_GEMM_CONFIG(GemmRR, cutlass::layout::RowMajor, cutlass::layout::RowMajor, 128, 128)
+
+// The forward layer: y[M,N] (bf16) = relu(A[M,K] W[N,K]^T + bias), the sums of
+// GemmRC (same K blocks, same order) with the bias, the ReLU and the rounding
+// in the epilogue, so the fp32 result is never written.  NT columns a tile: as
+// wide as the layer where that still gives every SM a tile, else narrower.
+template <int NT>
+struct GemmAct {
+    using ElemAB = cutlass::bfloat16_t;
+    using Tile = cute::Shape<cute::_128, cute::Int<NT>, cute::_64>;
+    using Cluster = cute::Shape<cute::_1, cute::_1, cute::_1>;
+    using Fusion = cutlass::epilogue::fusion::LinCombPerColBiasEltAct<cutlass::epilogue::thread::ReLu, ElemAB, float,
+                                                                      float, void>;
+    using Epilogue = typename cutlass::epilogue::collective::CollectiveBuilder<
+        cutlass::arch::Sm100, cutlass::arch::OpClassTensorOp, Tile, Cluster,
+        cutlass::epilogue::collective::EpilogueTileAuto, float, float, void, cutlass::layout::RowMajor, 8, ElemAB,
+        cutlass::layout::RowMajor, 8, cutlass::epilogue::collective::EpilogueScheduleAuto, Fusion>::CollectiveOp;
+    using Mainloop = typename cutlass::gemm::collective::CollectiveBuilder<
+        cutlass::arch::Sm100, cutlass::arch::OpClassTensorOp, ElemAB, cutlass::layout::RowMajor, 8, ElemAB,
+        cutlass::layout::ColumnMajor, 8, float, Tile, Cluster,
+        cutlass::gemm::collective::StageCountAutoCarveout<static_cast<int>(sizeof(typename Epilogue::SharedStorage))>,
+        cutlass::gemm::collective::KernelScheduleAuto>::CollectiveOp;
+    using Kernel = cutlass::gemm::kernel::GemmUniversal<cute::Shape<int, int, int, int>, Mainloop, Epilogue, void>;
+    using Gemm = cutlass::gemm::device::GemmUniversalAdapter<Kernel>;
+    static typename Gemm::Arguments args(int M, int N, int K, const void *A, const void *B, const float *bias, void *D)
+    {
+        auto sa = cutlass::make_cute_packed_stride(typename Kernel::StrideA{}, cute::make_shape(M, K, 1));
+        auto sb = cutlass::make_cute_packed_stride(typename Kernel::StrideB{}, cute::make_shape(N, K, 1));
+        auto sd = cutlass::make_cute_packed_stride(typename Kernel::StrideD{}, cute::make_shape(M, N, 1));
+        typename Gemm::Arguments a{cutlass::gemm::GemmUniversalMode::kGemm,
+                                   {M, N, K, 1},
+                                   {static_cast<const ElemAB *>(A), sa, static_cast<const ElemAB *>(B), sb},
+                                   {{}, nullptr, {}, static_cast<ElemAB *>(D), sd}};
+        a.epilogue.thread.alpha = 1.f;
+        a.epilogue.thread.beta = 0.f;
+        a.epilogue.thread.bias_ptr = bias;
+        return a;
+    }
+    static int run(int M, int N, int K, const void *A, const void *B, const float *bias, void *D, cudaStream_t s)
+    {
+        auto a = args(M, N, K, A, B, bias, D);
+        Gemm g;
+        if (g.can_implement(a) != cutlass::Status::kSuccess || Gemm::get_workspace_size(a) > 0) return WS_EINVAL;
+        if (g.initialize(a, nullptr, s) != cutlass::Status::kSuccess) return WS_ECUDA;
+        return g.run(s) == cutlass::Status::kSuccess ? WS_OK : WS_ECUDA;
+    }
+};
 
 constexpr int T = 256;
+constexpr int kSms = 148;
+
+// n / d for n < 2^31 by a multiplication (Granlund and Montgomery 1994).
+struct FastDiv {
+    unsigned d, mul, shift;
+    explicit FastDiv(unsigned div) : d(div)
+    {
+        shift = 0;
+        while ((1ull << shift) < d) shift++;
+        mul = (unsigned)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
+    }
+    __device__ __forceinline__ unsigned div(unsigned n) const { return (__umulhi(n, mul) + n) >> shift; }
+    __device__ __forceinline__ void divmod(unsigned n, unsigned &q, unsigned &r) const
+    {
+        q = div(n);
+        r = n - q * d;
+    }
+};
+
+// The layers around the GEMMs move 16 bytes a thread (8 bf16 or 4 fp32
+// channels, which the GEMMs' 16-byte rows guarantee); what does not fit that
+// (channel counts or addresses that are no multiple, 2^31 pieces) takes the
+// element-wise kernels further down.  One thread an element with 64-bit
+// divisions ran at 1/12 of the memory's rate (im2col of 16 x 128^2 x 96: 1.2
+// ms against 0.1 now).
+inline bool wide(int C, int per, long long pieces, std::initializer_list<const void *> ps)
+{
+    if (C % per || pieces >= (1ll << 31)) return false;
+    for (const void *p : ps)
+        if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+    return true;
+}
+
+// im2col of one or two sources: channels [0, C0) from in0 (half the
+// resolution where UP: a nearest 2x upsampling read in place), the rest from
+// in1 (a skip connection), as the concatenated tensor would give.
+template <bool UP>
+__global__ void __launch_bounds__(T) k_im2col16(unsigned total, int H, int W, int c0, int c1, FastDiv dk, FastDiv dc,
+                                                FastDiv dw, FastDiv dh, const uint4 *__restrict__ in0,
+                                                const uint4 *__restrict__ in1, uint4 *__restrict__ cols)
+{
+    for (unsigned q = blockIdx.x * T + threadIdx.x; q < total; q += gridDim.x * T) {
+        unsigned row, k, tap, c, x, y, b, t;
+        dk.divmod(q, row, k);
+        dc.divmod(k, tap, c);
+        dw.divmod(row, t, x);
+        dh.divmod(t, b, y);
+        const int dy = (int)(tap * 11u >> 5), dx = (int)tap - 3 * dy;  // tap / 3, tap % 3 for tap < 9
+        const int yy = (int)y + dy - 1, xx = (int)x + dx - 1;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (yy >= 0 && yy < H && xx >= 0 && xx < W) {
+            if ((int)c >= c0) v = in1[(((size_t)b * H + yy) * W + xx) * c1 + c - c0];
+            else if (UP) v = in0[(((size_t)b * (H / 2) + yy / 2) * (W / 2) + xx / 2) * c0 + c];
+            else v = in0[(((size_t)b * H + yy) * W + xx) * c0 + c];
+        }
+        cols[q] = v;
+    }
+}
+
+// col2im, 4 channels a thread: the taps in k_col2im's order.
+__global__ void __launch_bounds__(T) k_col2im4(unsigned total, int H, int W, int c4, FastDiv dc, FastDiv dw, FastDiv dh,
+                                               const float4 *__restrict__ dcols, float4 *__restrict__ dx)
+{
+    for (unsigned q = blockIdx.x * T + threadIdx.x; q < total; q += gridDim.x * T) {
+        unsigned pix, c, x, y, b, t;
+        dc.divmod(q, pix, c);
+        dw.divmod(pix, t, x);
+        dh.divmod(t, b, y);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int tap = 0; tap < 9; tap++) {
+            const int oy = (int)y - (tap / 3 - 1), ox = (int)x - (tap % 3 - 1);
+            if (oy < 0 || oy >= H || ox < 0 || ox >= W) continue;
+            const float4 v = __ldcs(dcols + ((((size_t)b * H + oy) * W + ox) * 9 + tap) * c4 + c);
+            acc.x += v.x;
+            acc.y += v.y;
+            acc.z += v.z;
+            acc.w += v.w;
+        }
+        dx[q] = acc;
+    }
+}
+
+__device__ __forceinline__ uint2 pack4(float4 v)
+{
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    return make_uint2(reinterpret_cast<const unsigned &>(a), reinterpret_cast<const unsigned &>(b));
+}
+__device__ __forceinline__ float4 unpack4(uint2 v)
+{
+    const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 &>(v.x));
+    const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 &>(v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// dz = dy where the layer's output y is positive (y null: everywhere; bf16, for the GEMMs), and
+// the column sums of that: a block's rows in a fixed order into part[block][C].
+// A thread takes 4 channels of every T / (C / 4)-th row.
+__global__ void __launch_bounds__(T) k_act_back_sum(long long M, int Cn, int rows_per, const float4 *__restrict__ dy,
+                                                    const uint2 *__restrict__ y, uint2 *__restrict__ dz,
+                                                    float4 *__restrict__ part)
+{
+    extern __shared__ float4 sh[];
+    const int c4 = Cn / 4, lanes = T / c4;
+    const int c = threadIdx.x % c4, lane = threadIdx.x / c4;
+    const long long r0 = (long long)blockIdx.x * rows_per, r1 = min(M, r0 + rows_per);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < lanes) {
+        for (long long r = r0 + lane; r < r1; r += lanes) {
+            float4 g = dy[r * c4 + c];
+            if (y != nullptr) {
+                const float4 v = unpack4(y[r * c4 + c]);
+                g.x = v.x > 0.f ? g.x : 0.f;
+                g.y = v.y > 0.f ? g.y : 0.f;
+                g.z = v.z > 0.f ? g.z : 0.f;
+                g.w = v.w > 0.f ? g.w : 0.f;
+            }
+            dz[r * c4 + c] = pack4(g);
+            acc.x += g.x;
+            acc.y += g.y;
+            acc.z += g.z;
+            acc.w += g.w;
+        }
+        sh[threadIdx.x] = acc;
+    }
+    __syncthreads();
+    if (lane == 0) {
+        for (int l = 1; l < lanes; l++) {
+            const float4 v = sh[l * c4 + c];
+            acc.x += v.x;
+            acc.y += v.y;
+            acc.z += v.z;
+            acc.w += v.w;
+        }
+        part[(size_t)blockIdx.x * c4 + c] = acc;
+    }
+}
+
+// out[i] += the sum of `count` slices part[s][i] in a fixed order: 8 strands
+// of slices, then the strands.
+__global__ void __launch_bounds__(256) k_sum_slices(int n, int count, const float *__restrict__ part,
+                                                    float *__restrict__ out)
+{
+    __shared__ float sh[8][33];
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    float acc = 0.f;
+    if (i < n)
+        for (int s = threadIdx.y; s < count; s += 8) acc += part[(size_t)s * n + i];
+    sh[threadIdx.y][threadIdx.x] = acc;
+    __syncthreads();
+    if (threadIdx.y == 0 && i < n) {
+        for (int k = 1; k < 8; k++) acc += sh[k][threadIdx.x];
+        out[i] += acc;
+    }
+}
+
+// 2x2 average pooling, 8 channels a thread (k_pool2's sums).
+__global__ void __launch_bounds__(T) k_pool16(unsigned total, int W, int c8, FastDiv dc, FastDiv dw, FastDiv dh,
+                                              const uint4 *__restrict__ in, uint4 *__restrict__ out)
+{
+    for (unsigned q = blockIdx.x * T + threadIdx.x; q < total; q += gridDim.x * T) {
+        unsigned p, c, x, y, b, t;
+        dc.divmod(q, p, c);
+        dw.divmod(p, t, x);
+        dh.divmod(t, b, y);
+        const uint4 *src = in + (((size_t)b * 2 * dh.d + 2 * y) * W + 2 * x) * c8 + c;
+        const uint4 v0 = src[0], v1 = src[c8], v2 = src[(size_t)W * c8], v3 = src[(size_t)(W + 1) * c8];
+        uint4 r;
+        const auto avg = [](unsigned a, unsigned b2, unsigned c2, unsigned d) {
+            const float2 fa = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 &>(a));
+            const float2 fb = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 &>(b2));
+            const float2 fc = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 &>(c2));
+            const float2 fd = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 &>(d));
+            const __nv_bfloat162 m = __floats2bfloat162_rn(0.25f * (fa.x + fb.x + fc.x + fd.x),
+                                                           0.25f * (fa.y + fb.y + fc.y + fd.y));
+            return reinterpret_cast<const unsigned &>(m);
+        };
+        r.x = avg(v0.x, v1.x, v2.x, v3.x);
+        r.y = avg(v0.y, v1.y, v2.y, v3.y);
+        r.z = avg(v0.z, v1.z, v2.z, v3.z);
+        r.w = avg(v0.w, v1.w, v2.w, v3.w);
+        out[q] = r;
+    }
+}
+
+// The adjoint of the pooling with the skip connection's gradient added:
+// din = dout / 4 + dskip, dskip being channels c0.. of rows of ct channels.
+__global__ void __launch_bounds__(T) k_pool_back_skip(unsigned total, int W, int c4, int ct4, int c04, FastDiv dc,
+                                                      FastDiv dw, FastDiv dh, const float4 *__restrict__ dout,
+                                                      const float4 *__restrict__ skip, float4 *__restrict__ din)
+{
+    for (unsigned q = blockIdx.x * T + threadIdx.x; q < total; q += gridDim.x * T) {
+        unsigned p, c, x, y, b, t;
+        dc.divmod(q, p, c);
+        dw.divmod(p, t, x);
+        dh.divmod(t, b, y);
+        const float4 d = dout[(((size_t)b * (dh.d / 2) + y / 2) * (W / 2) + x / 2) * c4 + c];
+        const float4 s = skip[(size_t)p * ct4 + c04 + c];
+        din[q] = make_float4(0.25f * d.x + s.x, 0.25f * d.y + s.y, 0.25f * d.z + s.z, 0.25f * d.w + s.w);
+    }
+}
+
+// The adjoint of the upsampling, 4 channels a thread (k_up2_back's sums).
+__global__ void __launch_bounds__(T) k_up_back4(unsigned total, int W, int c4, int ct4, FastDiv dc, FastDiv dw, FastDiv dh,
+                                                const float4 *__restrict__ dout, float4 *__restrict__ din)
+{
+    for (unsigned q = blockIdx.x * T + threadIdx.x; q < total; q += gridDim.x * T) {
+        unsigned p, c, x, y, b, t;
+        dc.divmod(q, p, c);
+        dw.divmod(p, t, x);
+        dh.divmod(t, b, y);
+        const float4 *src = dout + (((size_t)b * 2 * dh.d + 2 * y) * 2 * W + 2 * x) * ct4 + c;
+        const float4 v0 = src[0], v1 = src[ct4], v2 = src[(size_t)2 * W * ct4], v3 = src[(size_t)(2 * W + 1) * ct4];
+        din[q] = make_float4(v0.x + v1.x + v2.x + v3.x, v0.y + v1.y + v2.y + v3.y, v0.z + v1.z + v2.z + v3.z,
+                             v0.w + v1.w + v2.w + v3.w);
+    }
+}
 
 // ---------------------------------------------------------------------------
 // im2col / col2im for 3x3, stride 1, zero padding 1, NHWC
@@ -327,6 +600,13 @@ __global__ void k_to_bf16(long long n, const float *__restrict__ x, bf16 *__rest
         y[q] = __float2bfloat16(x[q]);
 }
 
+inline int grid16(unsigned total)
+{
+    return (int)std::min<unsigned>((total + T - 1) / T, kSms * 16u);
+}
+
+inline bool narrow_cr(int M, int N) { return ((M + 127) / 128) * ((N + 127) / 128) < kSms; }
+
 inline int grid_for(long long n)
 {
     const long long b = (n + T - 1) / T;
@@ -352,6 +632,7 @@ WS_API int ws_gemm(int layout, int M, int N, int K, const void *A, const void *B
     case WS_GEMM_RC: return GemmRC::run(M, N, K, A, B, D, alpha, beta, workspace, workspace_bytes, s);
     case WS_GEMM_CR:
         if (M % 8 != 0 || N % 8 != 0) return WS_EINVAL;
+        if (narrow_cr(M, N)) return GemmCR32::run(M, N, K, A, B, D, alpha, beta, workspace, workspace_bytes, s);
         return GemmCR::run(M, N, K, A, B, D, alpha, beta, workspace, workspace_bytes, s);
     case WS_GEMM_RR:
         if (N % 8 != 0) return WS_EINVAL;
@@ -364,7 +645,7 @@ WS_API size_t ws_gemm_workspace(int layout, int M, int N, int K)
 {
     switch (layout) {
     case WS_GEMM_RC: return GemmRC::workspace(M, N, K);
-    case WS_GEMM_CR: return GemmCR::workspace(M, N, K);
+    case WS_GEMM_CR: return narrow_cr(M, N) ? GemmCR32::workspace(M, N, K) : GemmCR::workspace(M, N, K);
     case WS_GEMM_RR: return GemmRR::workspace(M, N, K);
     default: return 0;
     }
@@ -373,14 +654,80 @@ WS_API size_t ws_gemm_workspace(int layout, int M, int N, int K)
 WS_API int ws_im2col(int B, int H, int W, int C, const void *in, void *cols, void *stream)
 {
     const long long n = (long long)B * H * W * 9 * C;
+    if (n > 0 && wide(C, 8, n / 8, {in, cols})) {
+        const unsigned c8 = C / 8, total = (unsigned)(n / 8);
+        k_im2col16<false><<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
+            total, H, W, (int)c8, 0, FastDiv(9 * c8), FastDiv(c8), FastDiv(W), FastDiv(H),
+            static_cast<const uint4 *>(in), nullptr, static_cast<uint4 *>(cols));
+        return last_error();
+    }
     k_im2col<<<grid_for(n), T, 0, static_cast<cudaStream_t>(stream)>>>(B, H, W, C, static_cast<const bf16 *>(in),
                                                                         static_cast<bf16 *>(cols));
+    return last_error();
+}
+
+WS_API int ws_im2col_up(int B, int H, int W, int C0, const void *up, int C1, const void *skip, void *cols, void *stream)
+{
+    const long long n = (long long)B * H * W * 9 * (C0 + C1);
+    if (n <= 0 || H % 2 || W % 2 || C0 % 8 || !wide(C1, 8, n / 8, {up, skip, cols})) return WS_EINVAL;
+    const unsigned c8 = (C0 + C1) / 8, total = (unsigned)(n / 8);
+    k_im2col16<true><<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
+        total, H, W, C0 / 8, C1 / 8, FastDiv(9 * c8), FastDiv(c8), FastDiv(W), FastDiv(H),
+        static_cast<const uint4 *>(up), static_cast<const uint4 *>(skip), static_cast<uint4 *>(cols));
+    return last_error();
+}
+
+WS_API int ws_layer(int M, int N, int K, const void *A, const void *Wt, const float *bias, void *y, void *stream)
+{
+    if (M <= 0 || N <= 0 || K <= 0 || !A || !Wt || !bias || !y || K % 8 || N % 8) return WS_EINVAL;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int rows = (M + 127) / 128;
+    if (N > 64 && rows * ((N + 127) / 128) >= kSms) return GemmAct<128>::run(M, N, K, A, Wt, bias, y, s);
+    if (N > 32 && rows * ((N + 63) / 64) >= kSms) return GemmAct<64>::run(M, N, K, A, Wt, bias, y, s);
+    return GemmAct<32>::run(M, N, K, A, Wt, bias, y, s);
+}
+
+WS_API size_t ws_act_back_sum_workspace(int C) { return (size_t)kSms * 4 * C * sizeof(float); }
+
+WS_API int ws_act_back_sum(long long M, int C, const float *dy, const void *y, void *dz, float *gb, void *workspace,
+                           size_t workspace_bytes, void *stream)
+{
+    if (M <= 0 || C <= 0 || !dy || !dz || !workspace || C % 8 || C > 1024) return WS_EINVAL;
+    if (!wide(C, 4, M * (C / 4), {dy, y, dz, workspace}) || workspace_bytes < ws_act_back_sum_workspace(C))
+        return WS_EINVAL;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    float *part = static_cast<float *>(workspace);
+    const int rows_per = (int)std::max<long long>((M + 4 * kSms - 1) / (4 * kSms), 32);
+    const int blocks = (int)((M + rows_per - 1) / rows_per);
+    k_act_back_sum<<<blocks, T, T * sizeof(float4), s>>>(M, C, rows_per, reinterpret_cast<const float4 *>(dy),
+                                                         static_cast<const uint2 *>(y), static_cast<uint2 *>(dz),
+                                                         reinterpret_cast<float4 *>(part));
+    if (gb) k_sum_slices<<<(C + 31) / 32, dim3(32, 8), 0, s>>>(C, blocks, part, gb);
+    return last_error();
+}
+
+WS_API int ws_pool2_back_skip(int B, int H, int W, int C, const float *dout, const float *dskip, int Ct, int c0, float *din,
+                              void *stream)
+{
+    const long long n = (long long)B * H * W * C;
+    if (n <= 0 || H % 2 || W % 2 || Ct % 4 || c0 % 4 || !wide(C, 4, n / 4, {dout, dskip, din})) return WS_EINVAL;
+    const unsigned total = (unsigned)(n / 4);
+    k_pool_back_skip<<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
+        total, W, C / 4, Ct / 4, c0 / 4, FastDiv(C / 4), FastDiv(W), FastDiv(H), reinterpret_cast<const float4 *>(dout),
+        reinterpret_cast<const float4 *>(dskip), reinterpret_cast<float4 *>(din));
     return last_error();
 }
 
 WS_API int ws_col2im(int B, int H, int W, int C, const float *dcols, float *dx, void *stream)
 {
     const long long n = (long long)B * H * W * C;
+    if (n > 0 && wide(C, 4, n * 9 / 4, {dcols, dx})) {
+        const unsigned total = (unsigned)(n / 4);
+        k_col2im4<<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
+            total, H, W, C / 4, FastDiv(C / 4), FastDiv(W), FastDiv(H), reinterpret_cast<const float4 *>(dcols),
+            reinterpret_cast<float4 *>(dx));
+        return last_error();
+    }
     k_col2im<<<grid_for(n), T, 0, static_cast<cudaStream_t>(stream)>>>(B, H, W, C, dcols, dx);
     return last_error();
 }
@@ -410,6 +757,13 @@ WS_API int ws_pool2(int B, int H, int W, int C, const void *in, void *out, void 
 {
     if (H % 2 || W % 2) return WS_EINVAL;
     const long long n = (long long)B * (H / 2) * (W / 2) * C;
+    if (n > 0 && wide(C, 8, n / 2, {in, out})) {
+        const unsigned total = (unsigned)(n / 8);
+        k_pool16<<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
+            total, W, C / 8, FastDiv(C / 8), FastDiv(W / 2), FastDiv(H / 2), static_cast<const uint4 *>(in),
+            static_cast<uint4 *>(out));
+        return last_error();
+    }
     k_pool2<<<grid_for(n), T, 0, static_cast<cudaStream_t>(stream)>>>(B, H, W, C, static_cast<const bf16 *>(in),
                                                                         static_cast<bf16 *>(out));
     return last_error();
@@ -434,6 +788,13 @@ WS_API int ws_up2(int B, int H, int W, int C, const void *in, int Ct, int c0, vo
 WS_API int ws_up2_back(int B, int H, int W, int C, const float *dout, int Ct, int c0, float *din, void *stream)
 {
     const long long n = (long long)B * H * W * C;
+    if (n > 0 && Ct % 4 == 0 && c0 % 4 == 0 && wide(C, 4, (long long)B * H * W * Ct, {dout, din})) {
+        const unsigned total = (unsigned)(n / 4);
+        k_up_back4<<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
+            total, W, C / 4, Ct / 4, FastDiv(C / 4), FastDiv(W), FastDiv(H),
+            reinterpret_cast<const float4 *>(dout) + c0 / 4, reinterpret_cast<float4 *>(din));
+        return last_error();
+    }
     k_up2_back<<<grid_for(n), T, 0, static_cast<cudaStream_t>(stream)>>>(B, H, W, C, dout, Ct, c0, din);
     return last_error();
 }

@@ -65,9 +65,16 @@ def load():
         L.ws_mse_centered.argtypes = [i, i, i, f, vp, vp, vp, vp, vp]
         L.ws_adam.argtypes = [ll, vp, vp, vp, vp, vp, f, f, f, f, i, vp]
         L.ws_to_bf16.argtypes = [ll, vp, vp, vp]
+        L.ws_im2col_up.argtypes = [i, i, i, i, vp, i, vp, vp, vp]
+        L.ws_layer.argtypes = [i, i, i, vp, vp, vp, vp, vp]
+        L.ws_act_back_sum.argtypes = [ll, i, vp, vp, vp, vp, vp, ctypes.c_size_t, vp]
+        L.ws_act_back_sum_workspace.argtypes = [i]
+        L.ws_act_back_sum_workspace.restype = ctypes.c_size_t
+        L.ws_pool2_back_skip.argtypes = [i, i, i, i, vp, vp, i, i, vp, vp]
         for name in ("ws_gemm", "ws_im2col", "ws_col2im", "ws_bias_act", "ws_act_back", "ws_colsum", "ws_pool2",
                      "ws_pool2_back", "ws_up2", "ws_up2_back", "ws_put_channels", "ws_take_channels",
-                     "ws_mse_centered", "ws_adam", "ws_to_bf16"):
+                     "ws_mse_centered", "ws_adam", "ws_to_bf16", "ws_im2col_up", "ws_layer", "ws_act_back_sum",
+                     "ws_pool2_back_skip"):
             getattr(L, name).restype = ctypes.c_int
         _lib = L
     return _lib
@@ -138,6 +145,8 @@ class WarmStartNet:
         self.trace = None
         self._ws = None
         self._ws_bytes = 0
+        self._sides = []  # side streams of backward(), and what runs on them
+        self._held = []
 
     def layers(self):
         for pair in self.enc:
@@ -220,6 +229,53 @@ class WarmStartNet:
         _ok(L.ws_bias_act(M, c.cout, _p(d), _p(c.b), 1 if c.relu else 0, _p(y), _p(pre), self._stream), "bias_act")
         return y, cols, pre
 
+    def _layer_fwd(self, c: Conv, x, Bn, H, W, skip=None):
+        """A 3x3 convolution with bias and ReLU in two launches; with skip, its
+        input is the concatenation of x, upsampled, and skip.  Returns
+        (y, cols)."""
+        torch = self.torch
+        L = load()
+        M = Bn * H * W
+        cols = torch.empty(M, 9 * c.cin, dtype=torch.bfloat16, device=self.dev)
+        if skip is None:
+            _ok(L.ws_im2col(Bn, H, W, c.cin, x.data_ptr(), cols.data_ptr(), self._stream), "im2col")
+        else:
+            cs = skip.shape[-1]
+            _ok(L.ws_im2col_up(Bn, H, W, c.cin - cs, x.data_ptr(), cs, skip.data_ptr(), cols.data_ptr(), self._stream),
+                "im2col_up")
+        y = torch.empty(M, c.cout, dtype=torch.bfloat16, device=self.dev)
+        _ok(L.ws_layer(M, c.cout, 9 * c.cin, cols.data_ptr(), c.w16.data_ptr(), c.b.data_ptr(), y.data_ptr(),
+                       self._stream), "layer")
+        return y, cols
+
+    def _layer_bwd(self, c: Conv, dy, cols, y, Bn, H, W):
+        """Backward of _layer_fwd (y its output) or of the head (y None): dy
+        fp32 [M, cout].  Accumulates c.gw, c.gb; returns dx fp32.  The weight
+        gradient, which no layer waits for and which fills few SMs, runs on a
+        side stream; backward() joins it and keeps its operands until then."""
+        torch = self.torch
+        L = load()
+        M, K = Bn * H * W, c.k * c.k * c.cin
+        dz = torch.empty(M, c.cout, dtype=torch.bfloat16, device=self.dev)
+        need = L.ws_act_back_sum_workspace(c.cout)
+        ws = torch.empty(need, dtype=torch.uint8, device=self.dev)
+        _ok(L.ws_act_back_sum(M, c.cout, dy.data_ptr(), 0 if y is None else y.data_ptr(), dz.data_ptr(),
+                              0 if c.b is None else c.gb.data_ptr(), ws.data_ptr(), need, self._stream), "act_back_sum")
+        need = L.ws_gemm_workspace(GEMM_CR, c.cout, K, M)
+        ws = torch.empty(need, dtype=torch.uint8, device=self.dev) if need else None
+        side = self._sides[len(self._held) % len(self._sides)]
+        side.wait_stream(torch.cuda.current_stream(self.dev))
+        self._held.append((dz, cols, ws))
+        _ok(L.ws_gemm(GEMM_CR, c.cout, K, M, dz.data_ptr(), cols.data_ptr(), c.gw.data_ptr(), 1.0, 1.0,
+                      ws.data_ptr() if need else None, need, side.cuda_stream), "weight gradient")
+        dcols = torch.empty(M, K, dtype=torch.float32, device=self.dev)
+        self._gemm(GEMM_RR, M, K, c.cout, dz, c.w16, dcols)
+        if c.k == 1:
+            return dcols
+        dx = torch.empty(M, c.cin, dtype=torch.float32, device=self.dev)
+        _ok(L.ws_col2im(Bn, H, W, c.cin, dcols.data_ptr(), dx.data_ptr(), self._stream), "col2im")
+        return dx
+
     def _conv_bwd(self, c: Conv, dy, cols, pre, Bn, H, W):
         """dy: fp32 [M, cout].  Accumulates c.gw, c.gb; returns dx fp32."""
         torch = self.torch
@@ -260,10 +316,18 @@ class WarmStartNet:
         tape = []
         skips = []
         h, hh, ww = x.contiguous(), H, W
+        # a trace wants every layer's pre-activations and gradients: the layers
+        # run launch by launch then
+        fused = self.trace is None
         for l in range(self.levels):
             for c in self.enc[l]:
-                y, cols, pre = self._conv_fwd(c, h, Bn, hh, ww)
-                tape.append((c, cols, pre, hh, ww))
+                if fused:
+                    y, cols = self._layer_fwd(c, h, Bn, hh, ww)
+                    pre = y
+                else:
+                    y, cols, pre = self._conv_fwd(c, h, Bn, hh, ww)
+                if keep:
+                    tape.append((c, cols, pre, hh, ww))
                 h = y
             skips.append((h, hh, ww))
             if l < self.levels - 1:
@@ -272,6 +336,14 @@ class WarmStartNet:
                 h, hh, ww = p, hh // 2, ww // 2
         for j, l in enumerate(range(self.levels - 2, -1, -1)):
             ct = self.ch[l + 1] + self.ch[l]
+            if fused:
+                sk, hh, ww = skips[l]
+                c0, c1 = self.dec[j]
+                h0, cols0 = self._layer_fwd(c0, h, Bn, hh, ww, skip=sk)
+                h, cols1 = self._layer_fwd(c1, h0, Bn, hh, ww)
+                if keep:
+                    tape += [(c0, cols0, h0, hh, ww), (c1, cols1, h, hh, ww)]
+                continue
             cat = torch.empty(Bn, hh * 2, ww * 2, ct, dtype=torch.bfloat16, device=self.dev)
             _ok(L.ws_up2(Bn, hh, ww, self.ch[l + 1], _p(h), ct, 0, _p(cat), self._stream), "up2")
             sk, sh, sw = skips[l]
@@ -280,10 +352,12 @@ class WarmStartNet:
             h, hh, ww = cat, sh, sw
             for c in self.dec[j]:
                 y, cols, pre = self._conv_fwd(c, h, Bn, hh, ww)
-                tape.append((c, cols, pre, hh, ww))
+                if keep:
+                    tape.append((c, cols, pre, hh, ww))
                 h = y
         d, cols, _ = self._conv_fwd(self.head, h, Bn, hh, ww)
-        tape.append((self.head, cols, None, hh, ww))
+        if keep:
+            tape.append((self.head, cols, None, hh, ww))
         pred = d[:, 0].contiguous().view(Bn, hh * ww)
         if keep:
             self._tape = (tape, Bn, H, W)
@@ -293,13 +367,29 @@ class WarmStartNet:
         """dpred: fp32 [B, H*W], gradient of the loss w.r.t. forward()'s
         output.  Accumulates the parameter gradients."""
         torch = self.torch
+        if not self._sides:
+            self._sides = [torch.cuda.Stream(device=self.dev) for _ in range(4)]
+        self._held = []
+        try:
+            return self._backward(dpred)
+        finally:
+            cur = torch.cuda.current_stream(self.dev)
+            for s in self._sides:
+                cur.wait_stream(s)
+            self._held = []
+
+    def _backward(self, dpred):
+        torch = self.torch
         L = load()
         tape, Bn, H, W = self._tape
         t = len(tape) - 1
         c, cols, pre, hh, ww = tape[t]
         dd = torch.zeros(Bn * hh * ww, 8, dtype=torch.float32, device=self.dev)
         dd[:, 0] = dpred.reshape(-1)
-        dh = self._conv_bwd(c, dd, cols, pre, Bn, hh, ww)
+        # layers that the forward pass ran fused carry their output (bf16)
+        fused = tape[0][2].dtype == torch.bfloat16
+        conv_bwd = self._layer_bwd if fused else self._conv_bwd
+        dh = conv_bwd(c, dd, cols, pre, Bn, hh, ww)
         t -= 1
         dskip = [None] * self.levels
         # decoder, last level first
@@ -308,9 +398,16 @@ class WarmStartNet:
             l = dec_levels[j]
             for _ in range(2):
                 c, cols, pre, hh, ww = tape[t]
-                dh = self._conv_bwd(c, dh, cols, pre, Bn, hh, ww)
+                dh = conv_bwd(c, dh, cols, pre, Bn, hh, ww)
                 t -= 1
             ct = self.ch[l + 1] + self.ch[l]
+            if fused:
+                dskip[l] = dh  # its last channels, read where the encoder needs them
+                du = torch.empty(Bn * (hh // 2) * (ww // 2), self.ch[l + 1], dtype=torch.float32, device=self.dev)
+                _ok(L.ws_up2_back(Bn, hh // 2, ww // 2, self.ch[l + 1], dh.data_ptr(), ct, 0, du.data_ptr(),
+                                  self._stream), "up2_back")
+                dh = du
+                continue
             ds = torch.empty(Bn * hh * ww, self.ch[l], dtype=torch.float32, device=self.dev)
             _ok(L.ws_take_channels(Bn * hh * ww, self.ch[l], _p(dh), ct, self.ch[l + 1], 0, _p(ds), self._stream),
                 "take_channels")
@@ -324,11 +421,18 @@ class WarmStartNet:
             ww = W >> l
             if l < self.levels - 1:
                 dp = torch.empty(Bn * hh * ww, self.ch[l], dtype=torch.float32, device=self.dev)
-                _ok(L.ws_pool2_back(Bn, hh, ww, self.ch[l], _p(dh), _p(dp), self._stream), "pool2_back")
-                dh = dp + dskip[l]
+                if fused:
+                    _ok(L.ws_pool2_back_skip(Bn, hh, ww, self.ch[l], dh.data_ptr(), dskip[l].data_ptr(),
+                                             self.ch[l + 1] + self.ch[l], self.ch[l + 1], dp.data_ptr(), self._stream),
+                        "pool2_back_skip")
+                    dskip[l] = None
+                    dh = dp
+                else:
+                    _ok(L.ws_pool2_back(Bn, hh, ww, self.ch[l], _p(dh), _p(dp), self._stream), "pool2_back")
+                    dh = dp + dskip[l]
             for _ in range(2):
                 c, cols, pre, ch_, cw_ = tape[t]
-                dh = self._conv_bwd(c, dh, cols, pre, Bn, ch_, cw_)
+                dh = conv_bwd(c, dh, cols, pre, Bn, ch_, cw_)
                 t -= 1
         assert t == -1
         self._tape = None

@@ -49,6 +49,31 @@ WS_API int ws_im2col(int B, int H, int W, int C, const void *in, void *cols, voi
  * each pixel (a gather in fixed order, fp32). */
 WS_API int ws_col2im(int B, int H, int W, int C, const float *dcols, float *dx, void *stream);
 
+/* ws_im2col of the concatenation of a nearest 2x upsampling of up[B][H/2][W/2][C0]
+ * and skip[B][H][W][C1] (bf16; C0, C1 multiples of 8, 16-byte aligned), which is
+ * not written out. */
+WS_API int ws_im2col_up(int B, int H, int W, int C0, const void *up, int C1, const void *skip, void *cols,
+                        void *stream);
+
+/* A layer in one launch: y[M][N] = relu(A[M][K] Wt[N][K]^T + bias) in bf16, the
+ * values of ws_gemm (WS_GEMM_RC) followed by ws_bias_act.  K and N multiples
+ * of 8. */
+WS_API int ws_layer(int M, int N, int K, const void *A, const void *Wt, const float *bias, void *y, void *stream);
+
+/* The backward of such a layer's bias and ReLU from dy[M][C] (fp32) and its
+ * output y (NULL: no ReLU): dz = dy where y > 0 (bf16, for the GEMMs), and
+ * gb[C] += the column sums of the masked dy (fp32, in a fixed order; NULL: no
+ * bias).  C a multiple of 8, at most 1024; workspace:
+ * ws_act_back_sum_workspace() bytes of device scratch. */
+WS_API int ws_act_back_sum(long long M, int C, const float *dy, const void *y, void *dz, float *gb, void *workspace,
+                           size_t workspace_bytes, void *stream);
+WS_API size_t ws_act_back_sum_workspace(int C);
+
+/* ws_pool2_back plus the gradient of the skip connection that leaves the same
+ * tensor: channels c0 .. c0 + C of dskip[B*H*W][Ct] (multiples of 4). */
+WS_API int ws_pool2_back_skip(int B, int H, int W, int C, const float *dout, const float *dskip, int Ct, int c0,
+                              float *din, void *stream);
+
 /* y = act(d + bias) (bf16 out; act = ReLU if relu, else identity); pre
  * (nullable) keeps d + bias in fp32.  d, pre: [M][C]. */
 WS_API int ws_bias_act(long long M, int C, const float *d, const float *bias, int relu, void *y, float *pre,
