@@ -26,6 +26,7 @@
 #include "cot_edge.cuh"
 #include <math.h>
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 
 namespace cot {
@@ -36,7 +37,8 @@ namespace cot {
 #define COT_REFINE_ROUNDS 4  // point-location rounds of one refinement
 #define COT_DEFERRED (-3)    // ring size of a cell handed to k_cells_heavy
 #ifndef COT_DEFER_LEAVES
-#define COT_DEFER_LEAVES 24  // surviving leaf buckets above which a walk is handed to k_cells_heavy
+#define COT_DEFER_LEAVES 12  // surviving leaf buckets above which a walk is handed to k_cells_heavy (25 cold iterations at
+                             // 4,096 sites with 24, 16, 12, 8: 5.33, 5.19, 5.01, 5.10 ms; at 65,536 sites 5.65, 5.56, 5.57, 5.55)
 #endif
 #ifndef COT_DEFER_PASS
 #define COT_DEFER_PASS 1  // refinement passes before a walk is handed to k_cells_heavy (1, 2, 3 measured 134.9, 134.8, 134.3 M cell-evals/s: 65,536 sites, 1024² target)
@@ -62,6 +64,9 @@ __shared__ unsigned long long cot_pst[16][16];
 #define PSTAT_LPC32 do { } while (0)
 #endif
 #define COT_WIN 1  // window radius in buckets
+#ifndef COT_DEEP_MIN
+#define COT_DEEP_MIN 8  // cutting candidates from which a chunk is clipped deepest first (4: 65,536 sites 1 % slower)
+#endif
 // neighbour cache count nbn[i]: +m an ordered ring of m generators, -m an
 // unordered list of m sites, -(COT_NB_HIDDEN + m) the m sites that hid the
 // cell at the last evaluation
@@ -1578,6 +1583,44 @@ __device__ __forceinline__ RegPoly apply_chunk(RegPoly P, int jl, const double2 
     PSTAT_ADD(4, ntested);
 #endif
     if (have == 0u) return P;
+    if constexpr (LPC == 32) {
+        // many that cut: the one whose line goes deepest into the ring next,
+        // and the others tested again on what it leaves.  A clip is a chain
+        // of some 500 cycles whether or not it still cuts; the deepest first
+        // leaves little for the rest (a chunk of a far too large ring 8 to 10
+        // us in order of the lanes).
+        if (__popc(have) >= COT_DEEP_MIN) {
+            const float rs = cut ? rsqrtf((float)key) : 0.0f;
+            while (true) {
+                unsigned dep = 0u;
+                if (cut) {
+                    double dm = 0.0;
+                    for (int k = 0; k < P.nv; k++) {
+                        const double d = side(al, bl, cl, S.X[k], S.Y[k]);
+                        dm = d > dm ? d : dm;
+                    }
+                    cut = dm > 0.0;
+                    // (positive floats order as their bits)
+                    if (cut) dep = __float_as_uint(fmaxf((float)dm * rs, FLT_MIN));
+                }
+                const unsigned top = __reduce_max_sync(FULLMASK, dep);
+                if (top == 0u) return P;
+                const int src = __ffs(__ballot_sync(FULLMASK, dep == top)) - 1;
+                const int j = W.shfl(jl, src);
+                const double a = W.shfl(al, src), b = W.shfl(bl, src), c = W.shfl(cl, src);
+                if (lane == src) cut = false;
+                if (!rclip<LPC>(P, a, b, c, j, lane, S)) {
+                    P.nv = -1;
+                    return P;
+                }
+                PSTAT_ADD(3, 1);
+                if (P.nv <= 0) return P;
+                W.sync();
+                if (lane < P.nv) { S.X[lane] = P.x; S.Y[lane] = P.y; }
+                W.sync();
+            }
+        }
+    }
     int ord = lane;
     if (nearest && __popc(have) > 1) {
         double k2 = cut ? key : INFINITY;
@@ -1800,62 +1843,89 @@ __device__ __forceinline__ double node_upper(const CotGeo &g, int node, double x
 }
 
 // Shrinks a ring that is far larger than its cell, for a certificate walk
-// whose frontier overflowed.  Each lane takes one vertex x of the ring and
-// descends the bound tree greedily (at every level the node with the largest
-// bound at x, at the leaf the site with the largest P_j(x)); a site that
-// beats P_i at x cuts that vertex off.  The distinct sites found are applied
-// like any other candidates, and the search repeats on the new ring, up to
-// `rounds` times or until no vertex finds a site.  Every clip is by a site
-// that cuts the ring, so the ring still contains the cell; the walk that
-// follows certifies it, and the cell's result is the one any other clip
-// order gives.
+// whose frontier overflowed.  Four lanes take one vertex x of the ring and
+// descend the bound tree greedily (at every level the node with the largest
+// bound at x, a child a lane; at the leaf the site with the largest P_j(x));
+// a site that beats P_i at x cuts that vertex off.  The distinct sites found
+// are applied like any other candidates, and the search repeats on the new
+// ring, up to `rounds` times or until no vertex finds a site.  Every clip is
+// by a site that cuts the ring, so the ring still contains the cell; the walk
+// that follows certifies it, and the cell's result is the one any other clip
+// order gives.  A refinement is a chain of dependent loads that only a few
+// cells of an evaluation take but all others wait for: a lane a vertex, with
+// the children and sites one after the other, took 45 us at 4,096 sites and
+// 100 us at 65,536.
 template <int LPC>
 __device__ __noinline__ RegPoly refine_by_vertices(const CotGeo &g, const double *__restrict__ wt, int i, double2 si,
                                                    double wi, RegPoly P, FastScratch &S, int rounds)
 {
     const Seg<LPC> SG;
-    const int lane = SG.sl;
+    const int lane = SG.sl, sub = lane & 3;
     int top = g.nlev - 1;
     while (top > 0 && g.lev_w[top - 1] * g.lev_h[top - 1] <= (LPC < 16 ? 16 : LPC)) top--;
     const int tw = g.lev_w[top], ntop = tw * g.lev_h[top], toff = g.lev_off[top];
     const double phi_i = 0.5 * (__fma_rn(si.x, si.x, si.y * si.y) - wi);
+    // the larger value of the four lanes and its index (the lower on a tie)
+    const auto best4 = [&](double &v, int &k) {
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1) {
+            const double ov = SG.shfl_xor(v, o);
+            const int ok = SG.shfl_xor(k, o);
+            if (ov > v || (ov == v && ok < k)) {
+                v = ov;
+                k = ok;
+            }
+        }
+    };
     for (int r = 0; r < rounds && P.nv > 0; r++) {
-        int jl = -1;
-        if (lane < P.nv) {
-            const double x = si.x + P.x, y = si.y + P.y;
-            const double pi = __fma_rn(x, si.x, y * si.y) - phi_i;
-            int bu = -1, bv = -1;
-            double best = -INFINITY;
-            for (int q = 0; q < ntop; q++) {
-                const double ub = node_upper(g, toff + q, x, y);
-                if (ub > best) { best = ub; bu = q % tw; bv = q / tw; }
+        for (int v0 = 0; v0 < P.nv; v0 += LPC / 4) {
+            const int k = v0 + (lane >> 2);
+            const double x = si.x + SG.shfl(P.x, k & (LPC - 1)), y = si.y + SG.shfl(P.y, k & (LPC - 1));
+            int node = INT_MAX;
+            double ub = -INFINITY;
+            for (int q = sub; q < ntop; q += 4) {
+                const double u = node_upper(g, toff + q, x, y);
+                if (u > ub) {
+                    ub = u;
+                    node = q;
+                }
             }
-            for (int L = top; L > 0 && bu >= 0; L--) {
-                const int cw = g.lev_w[L - 1], ch = g.lev_h[L - 1], off = g.lev_off[L - 1];
-                int nu = -1, nw = -1;
-                best = -INFINITY;
-                for (int bb = 0; bb < 2; bb++)
-                    for (int aa = 0; aa < 2; aa++) {
-                        const int cu = 2 * bu + aa, cv = 2 * bv + bb;
-                        if (cu < cw && cv < ch) {
-                            const double ub = node_upper(g, off + cu + cv * cw, x, y);
-                            if (ub > best) { best = ub; nu = cu; nw = cv; }
-                        }
-                    }
-                bu = nu;
-                bv = nw;
+            best4(ub, node);
+            int bu = node == INT_MAX ? -1 : node % tw, bv = node == INT_MAX ? -1 : node / tw;
+            for (int L = top; L > 0; L--) {
+                const int cw = g.lev_w[L - 1], ch = g.lev_h[L - 1];
+                const int cu = 2 * bu + (sub & 1), cv = 2 * bv + (sub >> 1);
+                node = INT_MAX;
+                ub = -INFINITY;
+                if (bu >= 0 && cu < cw && cv < ch) {
+                    node = cu + cv * cw;
+                    ub = node_upper(g, g.lev_off[L - 1] + node, x, y);
+                    if (ub == -INFINITY) node = INT_MAX;  // empty
+                }
+                best4(ub, node);
+                bu = node == INT_MAX ? -1 : node % cw;
+                bv = node == INT_MAX ? -1 : node / cw;
             }
+            double bp = __fma_rn(x, si.x, y * si.y) - phi_i;
+            int jl = INT_MAX;
             if (bu >= 0) {
                 const int b = bu + bv * g.lev_w[0];
-                double bp = pi;
-                for (int j = g.bstart[b], e = g.bstart[b + 1]; j < e; j++) {
+                for (int j = g.bstart[b] + sub, e = g.bstart[b + 1]; j < e; j += 4) {
                     if (j == i) continue;
                     const double2 sj = g.xy[j];
                     const double pj = __fma_rn(x, sj.x, y * sj.y) - 0.5 * (__fma_rn(sj.x, sj.x, sj.y * sj.y) - wt[j]);
-                    if (pj > bp) { bp = pj; jl = j; }
+                    if (pj > bp) {
+                        bp = pj;
+                        jl = j;
+                    }
                 }
             }
+            best4(bp, jl);
+            if (sub == 0 && k < P.nv) S.fr[0][k] = jl == INT_MAX ? -1 : jl;
         }
+        SG.sync();
+        int jl = lane < P.nv ? S.fr[0][lane] : -1;
+        SG.sync();
         // one copy of each site
         for (int t = 0; t < LPC; t++) {
             const int o = SG.shfl(jl, t);
@@ -2820,7 +2890,8 @@ __device__ __forceinline__ float site_depth(const CotGeo &g, const double *__res
         dm = fmax(dm, side(al, bl, cl, S.X[q], S.Y[q]));
     }
     if (!(dm > 0.0)) return -1.0f;
-    return (float)(dm / sqrt(key));
+    // (the depth only orders the clips)
+    return fmaxf((float)dm * rsqrtf((float)key), FLT_MIN);
 }
 
 // (depth, index) order: deeper first, then the lower index.
@@ -2861,6 +2932,26 @@ __device__ __forceinline__ void warp_merge_top(float &td, int &tj, float cd, int
     if (deeper(rd, rj, td, tj)) { td = rd; tj = rj; }
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) cmpx(td, tj, m, (lane & m) == 0);
+}
+
+// The 32 deepest of a warp's list, deepest at lane 0 (-1 past its end): sorted
+// and merged 32 at a time.
+__device__ __forceinline__ void warp_deepest(const float *dep, const int *site, int n, float &td, int &tj, int lane)
+{
+    td = -1.0f;
+    tj = INT_MAX;
+    __syncwarp();
+    for (int base = 0; base < n; base += 32) {
+        float cd = base + lane < n ? dep[base + lane] : -1.0f;
+        int cj = base + lane < n ? site[base + lane] : INT_MAX;
+        warp_sort_deep(cd, cj, lane);
+        if (base == 0) {
+            td = cd;
+            tj = cj;
+        } else {
+            warp_merge_top(td, tj, cd, cj, lane);
+        }
+    }
 }
 
 template <bool KEEP>
@@ -2925,32 +3016,45 @@ __global__ void __launch_bounds__(32 * HEAVY_WARPS, 2) k_cells_heavy(const __gri
                     nk += __popc(m);
                 }
                 __syncwarp();
-                float td = -1.0f;
-                int tj = INT_MAX;
-                for (int k = 0; k < nk; k++) {
-                    const int b = H.kept[wp][k];
-                    const int s1 = g.bstart[b + 1];
-                    bool full = false;
-                    for (int j0 = g.bstart[b]; j0 < s1; j0 += 32) {
-                        const int j = j0 + lane;
-                        const float dj = (j < s1 && j != i) ? site_depth(g, a.wt, j, si, wi, S, nv) : -1.0f;
+                // their sites, a lane each, 32 buckets' ranges at a time
+                bool full = false;
+                for (int k0 = 0; k0 < nk && !full; k0 += 32) {
+                    int st = 0, cnt = 0;
+                    if (k0 + lane < nk) {
+                        const int b = H.kept[wp][k0 + lane];
+                        st = g.bstart[b];
+                        cnt = g.bstart[b + 1] - st;
+                    }
+                    const int inc = warp_incl_scan(cnt, lane);
+                    const int tot = __shfl_sync(FULLMASK, inc, 31);
+                    const int first = st - (inc - cnt);
+                    for (int base = 0; base < tot; base += 32) {
+                        const int t = base + lane;
+                        int k = 0;
+#pragma unroll
+                        for (int sft = 16; sft >= 1; sft >>= 1) {
+                            const int v = __shfl_sync(FULLMASK, inc, k + sft - 1);
+                            if (v <= t) k += sft;
+                        }
+                        const int j = __shfl_sync(FULLMASK, first, k & 31) + t;
+                        const float dj = (t < tot && j != i) ? site_depth(g, a.wt, j, si, wi, S, nv) : -1.0f;
                         const bool cut = dj > 0.0f;
                         const unsigned m = __ballot_sync(FULLMASK, cut);
-                        if (nc + __popc(m) > HEAVY_CCAP) { full = true; break; }
+                        if (nc + __popc(m) > HEAVY_CCAP) {
+                            full = true;
+                            break;
+                        }
                         if (cut) {
                             H.cut[wp][nc + __popc(m & lt)] = j;
                             H.dep[wp][nc + __popc(m & lt)] = dj;
                         }
                         nc += __popc(m);
-                        if (m != 0u) {
-                            float cd = cut ? dj : -1.0f;
-                            int cj = cut ? j : INT_MAX;
-                            warp_sort_deep(cd, cj, lane);
-                            warp_merge_top(td, tj, cd, cj, lane);
-                        }
                     }
-                    if (full) { ov = true; break; }
                 }
+                ov = ov || full;
+                float td;
+                int tj;
+                warp_deepest(H.dep[wp], H.cut[wp], nc, td, tj, lane);
                 H.tdep[wp][lane] = td;
                 H.tj[wp][lane] = tj;
                 if (lane == 0) {
@@ -2988,8 +3092,6 @@ __global__ void __launch_bounds__(32 * HEAVY_WARPS, 2) k_cells_heavy(const __gri
                 if (nv <= 0) break;
                 const int n0 = H.ncut[wp];
                 int nk = 0;
-                float td = -1.0f;
-                int tj = INT_MAX;
                 for (int base = 0; base < n0; base += 32) {
                     const int k = base + lane;
                     const int j = k < n0 ? H.cut[wp][k] : -1;
@@ -3001,14 +3103,11 @@ __global__ void __launch_bounds__(32 * HEAVY_WARPS, 2) k_cells_heavy(const __gri
                         H.dep[wp][nk + __popc(m & lt)] = dj;
                     }
                     nk += __popc(m);
-                    if (m != 0u) {
-                        float cd = cut ? dj : -1.0f;
-                        int cj = cut ? j : INT_MAX;
-                        warp_sort_deep(cd, cj, lane);
-                        warp_merge_top(td, tj, cd, cj, lane);
-                    }
                     __syncwarp();
                 }
+                float td;
+                int tj;
+                warp_deepest(H.dep[wp], H.cut[wp], nk, td, tj, lane);
                 H.tdep[wp][lane] = td;
                 H.tj[wp][lane] = tj;
                 if (lane == 0) H.ncut[wp] = nk;
