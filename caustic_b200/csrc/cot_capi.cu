@@ -78,7 +78,6 @@ struct CotProblemDev {
     CotGeo geo{};
     // per evaluation
     double *w = nullptr, *wt = nullptr, *d = nullptr, *mu = nullptr, *mut = nullptr, *fc = nullptr;
-    double *wbar = nullptr;
     int *blist = nullptr, *bcnt = nullptr;  // the bucket walk's leaf lists (solves only)
     double2 *rbuf = nullptr;  // ring vertices between the cell and integration kernels
     int *lbuf = nullptr;      // ring generators between the two ring-building kernels
@@ -242,7 +241,6 @@ static void free_sized_by_sites(CotProblemDev &P)
     keep.bstart = P.bstart;
     keep.tstat = P.tstat;
     keep.tdyn = P.tdyn;
-    keep.wbar = P.wbar;
     keep.blist = P.blist;
     keep.bcnt = P.bcnt;
     keep.gen = P.gen;
@@ -254,7 +252,7 @@ static void free_sized_by_grid(CotProblemDev &P)
 {
     if (P.b_grid) cudaFree(P.b_grid);
     P.b_grid = nullptr;
-    P.bstart = nullptr; P.tstat = P.tdyn = nullptr; P.wbar = nullptr; P.blist = P.bcnt = nullptr;
+    P.bstart = nullptr; P.tstat = P.tdyn = nullptr; P.blist = P.bcnt = nullptr;
     P.cap_nb = P.cap_nodes = 0;
 }
 
@@ -560,7 +558,6 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
         c.add(&P.bstart, P.cap_nb + 1);
         c.add(&P.tstat, P.cap_nodes);
         c.add(&P.tdyn, P.cap_nodes);
-        c.add(&P.wbar, P.cap_nb);
         c.add(&P.blist, P.cap_nb * COT_BLEAF);
         c.add(&P.bcnt, P.cap_nb);
         const cudaError_t e = c.alloc(&P.b_grid);
@@ -727,7 +724,6 @@ static CellsArgs cells_args(CotProblemDev &P, const double *w, const double *d, 
     a.d = d;
     a.tptr = tptr;
     a.wt = P.wt;
-    a.wbar = P.wbar;
     a.rbuf = P.rbuf;
     a.lbuf = P.lbuf;
     a.flist = P.flist;
@@ -1043,13 +1039,11 @@ static int report_progress(cot_handle *h, int phase, int iteration, int status, 
 static void launch_trial_body(cot_handle *h, cudaGraphConditionalHandle hc, double *tptr, CotCtx &c)
 {
     CotProblemDev &P = h->P;
-    launch_begin_iteration(P.S, c);
-    launch_direction(P.geo, P.S, P.Sv, P.Yv, P.mu, P.d, c);
+    launch_begin_direction(P.geo, P.S, P.Sv, P.Yv, P.mu, P.d, P.ticket, c);
     CellsArgs a = cells_args(P, P.w, P.d, tptr);
     launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, c);
     launch_reduce(P.geo, P.mut, P.fc, P.nv, P.wt, P.d, h->cfg.max_ring, P.partials, P.ticket, P.out, P.S, c);
-    launch_accept(P.geo, P.S, P.Sv, P.Yv, P.w, P.wt, P.mu, P.mut, P.d, P.partials, P.ticket, 0, c);
-    launch_reject_cond(hc, P.S, c);
+    launch_accept(P.geo, P.S, P.Sv, P.Yv, P.w, P.wt, P.mu, P.mut, P.d, P.partials, P.ticket, 0, &hc, c);
 }
 
 // The first point of a solve: its evaluation becomes the current point.
@@ -1060,7 +1054,7 @@ static void launch_first_point(cot_handle *h, CotCtx &c)
     launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, c);
     launch_reduce(P.geo, P.mut, P.fc, P.nv, P.wt, nullptr, h->cfg.max_ring, P.partials, P.ticket, P.out, nullptr, c);
     launch_init_from_eval(P.S, P.out, c);
-    launch_accept(P.geo, P.S, P.Sv, P.Yv, P.w, P.wt, P.mu, P.mut, P.d, P.partials, P.ticket, 1, c);
+    launch_accept(P.geo, P.S, P.Sv, P.Yv, P.w, P.wt, P.mu, P.mut, P.d, P.partials, P.ticket, 1, nullptr, c);
 }
 
 static double *step_ptr(CotProblemDev &P)
@@ -1289,8 +1283,7 @@ static int solve_device(cot_handle *h, const cot_solve_opts &o, CotSolver &out, 
     } else {
         // host-driven loop: one control-block read per trial
         while (true) {
-            launch_begin_iteration(P.S, h->c());
-            launch_direction(P.geo, P.S, P.Sv, P.Yv, P.mu, P.d, h->c());
+            launch_begin_direction(P.geo, P.S, P.Sv, P.Yv, P.mu, P.d, P.ticket, h->c());
             COT_CUDA_TRY(cudaMemcpyAsync(h->hS, P.S, ctl, cudaMemcpyDeviceToHost, s));
             COT_CUDA_TRY(cudaStreamSynchronize(s));
             int r = boundary_report();
@@ -1306,7 +1299,7 @@ static int solve_device(cot_handle *h, const cot_solve_opts &o, CotSolver &out, 
                 if (!hs.ls_active) break;
             }
             if (hs.accepted)
-                launch_accept(P.geo, P.S, P.Sv, P.Yv, P.w, P.wt, P.mu, P.mut, P.d, P.partials, P.ticket, 0, h->c());
+                launch_accept(P.geo, P.S, P.Sv, P.Yv, P.w, P.wt, P.mu, P.mut, P.d, P.partials, P.ticket, 0, nullptr, h->c());
             else
                 launch_reject(P.S, h->c());
             COT_CUDA_TRY(cudaGetLastError());

@@ -121,12 +121,36 @@ __device__ __forceinline__ double bseg_max(double v, unsigned m)
     return v;
 }
 
-// Trial weights of bucket b's sites and their mean phi (0 for an empty
-// bucket).  Block 0 also clears the cell kernels' counters.
-__global__ void k_bucket_phi(CotGeo g, const double *__restrict__ w, const int *__restrict__ perm,
-                             const double *__restrict__ d,
-                             const double *__restrict__ tptr, double *__restrict__ wt,
-                             double *__restrict__ wbar, int *counters, int ncounters)
+// Half the mean trial weight of bucket b's sites (0 for an empty bucket), the
+// same bits whichever segment asks.
+__device__ __forceinline__ double bucket_mean(const CotGeo &g, const double *__restrict__ w,
+                                              const int *__restrict__ perm, const double *__restrict__ d, double t,
+                                              int b, int sl, unsigned m, double *wt)
+{
+    const int s0 = g.bstart[b], s1 = g.bstart[b + 1];
+    double acc = 0.0;
+    for (int j = s0 + sl; j < s1; j += BSEG) {
+        const double wj = perm != nullptr ? w[perm[j]] : trial_weight(w, d, t, j);
+        if (wt != nullptr) wt[j] = wj;
+        acc = __dadd_rn(acc, wj);
+    }
+    acc = bseg_sum(acc, m);
+    return s1 > s0 ? 0.5 * acc / (double)(s1 - s0) : 0.0;
+}
+
+// Trial weights and weight bound of every bucket, one bucket per segment:
+// a_b = slope of w/2 across the neighbouring buckets (central difference of
+// their mean w/2 over their box centres, one-sided at the grid edges),
+// B_b = max_j w_j/2 - a_b.s_j.  A segment takes its neighbours' means itself:
+// five times the reads, all from L2, for one launch less an evaluation.
+// Block 0 also clears the cell kernels' counters.
+#define TREE_THREADS 128
+__global__ void __launch_bounds__(TREE_THREADS) k_bucket_bounds(const __grid_constant__ CotGeo g,
+                                                               const double *__restrict__ w,
+                                                               const int *__restrict__ perm,
+                                                               const double *__restrict__ d,
+                                                               const double *__restrict__ tptr,
+                                                               double *__restrict__ wt, int *counters, int ncounters)
 {
     if (blockIdx.x == 0 && (int)threadIdx.x < ncounters) counters[threadIdx.x] = 0;
     const int b = (blockIdx.x * blockDim.x + threadIdx.x) / BSEG;
@@ -134,29 +158,15 @@ __global__ void k_bucket_phi(CotGeo g, const double *__restrict__ w, const int *
     if (b >= g.bx * g.by) return;  // whole segments leave together
     const unsigned m = bseg_mask();
     const double t = (d != nullptr && tptr != nullptr) ? *tptr : 0.0;
-    const int s0 = g.bstart[b], s1 = g.bstart[b + 1];
-    double acc = 0.0;
-    for (int j = s0 + sl; j < s1; j += BSEG) {
-        const double wj = perm != nullptr ? w[perm[j]] : trial_weight(w, d, t, j);
-        wt[j] = wj;
-        acc = __dadd_rn(acc, wj);
-    }
-    acc = bseg_sum(acc, m);
-    if (sl == 0) wbar[b] = (s1 > s0) ? 0.5 * acc / (double)(s1 - s0) : 0.0;
-}
-
-// Weight bound of bucket b: a_b = slope of w/2 across the neighbouring
-// buckets (central difference of their mean w/2 over their box centres,
-// one-sided at the grid edges), B_b = max_j w_j/2 - a_b.s_j.  Called by a
-// whole segment (mask msk); every lane returns the bound.
-__device__ __forceinline__ double4 bucket_bound(const CotGeo &g, const double *__restrict__ wt,
-                                                const double *__restrict__ wbar, int b, int sl, unsigned msk)
-{
     const double4 st = g.tstat[b];
-    if (st.z < 0.0) return make_double4(0.0, 0.0, -INFINITY, 0.0);
+    const double pb = bucket_mean(g, w, perm, d, t, b, sl, m, wt);
+    if (st.z < 0.0) {
+        if (sl == 0) g.tdyn[b] = make_double4(0.0, 0.0, -INFINITY, 0.0);
+        return;
+    }
     const int u = b % g.bx, v = b / g.bx;
-    const double pb = wbar[b];
     double c[2];
+#pragma unroll
     for (int ax = 0; ax < 2; ax++) {
         int bp = -1, bm = -1;
         if (ax == 0) {
@@ -166,21 +176,15 @@ __device__ __forceinline__ double4 bucket_bound(const CotGeo &g, const double *_
             if (v + 1 < g.by && g.tstat[b + g.bx].z >= 0.0) bp = b + g.bx;
             if (v > 0 && g.tstat[b - g.bx].z >= 0.0) bm = b - g.bx;
         }
+        const double vp = bp >= 0 ? bucket_mean(g, w, perm, d, t, bp, sl, m, nullptr) : 0.0;
+        const double vm = bm >= 0 ? bucket_mean(g, w, perm, d, t, bm, sl, m, nullptr) : 0.0;
         const double mb = ax == 0 ? st.x : st.y;
-        double val;
-        if (bp >= 0 && bm >= 0) {
-            const double mp = ax == 0 ? g.tstat[bp].x : g.tstat[bp].y;
-            const double mm = ax == 0 ? g.tstat[bm].x : g.tstat[bm].y;
-            val = (wbar[bp] - wbar[bm]) / (mp - mm);
-        } else if (bp >= 0) {
-            const double mp = ax == 0 ? g.tstat[bp].x : g.tstat[bp].y;
-            val = (wbar[bp] - pb) / (mp - mb);
-        } else if (bm >= 0) {
-            const double mm = ax == 0 ? g.tstat[bm].x : g.tstat[bm].y;
-            val = (pb - wbar[bm]) / (mb - mm);
-        } else {
-            val = 0.0;
-        }
+        const double mp = bp >= 0 ? (ax == 0 ? g.tstat[bp].x : g.tstat[bp].y) : 0.0;
+        const double mm = bm >= 0 ? (ax == 0 ? g.tstat[bm].x : g.tstat[bm].y) : 0.0;
+        double val = 0.0;
+        if (bp >= 0 && bm >= 0) val = (vp - vm) / (mp - mm);
+        else if (bp >= 0) val = (vp - pb) / (mp - mb);
+        else if (bm >= 0) val = (pb - vm) / (mb - mm);
         if (!isfinite(val)) val = 0.0;
         c[ax] = val;
     }
@@ -190,20 +194,8 @@ __device__ __forceinline__ double4 bucket_bound(const CotGeo &g, const double *_
         const double2 s = g.xy[j];
         B = fmax(B, 0.5 * wt[j] - (c[0] * s.x + c[1] * s.y));
     }
-    B = bseg_max(B, msk);
-    return make_double4(c[0], c[1], B, 0.0);
-}
-
-// Bucket weight bounds, one bucket per segment.
-#define TREE_THREADS 256
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_build(CotGeo g, const double *__restrict__ wt,
-                                                            const double *__restrict__ wbar)
-{
-    const int b = (blockIdx.x * blockDim.x + threadIdx.x) / BSEG;
-    const int sl = threadIdx.x & (BSEG - 1);
-    if (b >= g.bx * g.by) return;  // whole segments leave together
-    const double4 bd = bucket_bound(g, wt, wbar, b, sl, bseg_mask());
-    if (sl == 0) g.tdyn[b] = bd;
+    B = bseg_max(B, m);
+    if (sl == 0) g.tdyn[b] = make_double4(c[0], c[1], B, 0.0);
 }
 
 // Fixed-order block sum and max over TREE_THREADS threads (every thread
@@ -238,12 +230,13 @@ __device__ __forceinline__ double tree_block_max(double v, double *sh)
 // buckets and sites under it: a = the mean weight slope of its non-empty
 // buckets, B = max_j w_j/2 - a.s_j over its sites, the exact value for that
 // a.  No level waits for the one below, and no bound is a bound of bounds.
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_levels(CotGeo g, const double *__restrict__ wt)
+// The first kernel of the rings does not read them, so it does this work too,
+// in its first `upper` blocks (13 us of a launch of its own at 65,536 sites, 33
+// at 262,144): the highest levels (the most sites a node) first.
+__device__ __forceinline__ void tree_node(const CotGeo &g, const double *__restrict__ wt, int upper)
 {
     __shared__ double sh[TREE_THREADS / 32];
-    // the highest levels (the most sites a node) first, so that they do not
-    // trail the many small nodes of level 1
-    const int node = g.lev_off[1] + (int)(gridDim.x - 1 - blockIdx.x);
+    const int node = g.lev_off[1] + (upper - 1 - (int)blockIdx.x);
     int L = 1;
     while (L + 1 < g.nlev && g.lev_off[L + 1] <= node) L++;
     const int q = node - g.lev_off[L], W = g.lev_w[L];
@@ -279,6 +272,12 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_levels(CotGeo g, const do
     }
     B = tree_block_max(B, sh);
     if (threadIdx.x == 0) g.tdyn[node] = make_double4(cx, cy, B, 0.0);
+}
+
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_levels(const __grid_constant__ CotGeo g,
+                                                             const double *__restrict__ wt, int upper)
+{
+    tree_node(g, wt, upper);
 }
 
 // ---------------------------------------------------------------------------
@@ -2407,10 +2406,15 @@ __global__ void __launch_bounds__(128, MINB) k_cells_fast(const __grid_constant_
 // else every cell.
 #define CST_CACHED 0x100
 #define CST_FAST 0x200  // k_rings_cached has the ring, k_certify is to prove it
+// The first `upper` blocks build the tree's levels (upper 0: they stand).
 template <int MINB>
-__global__ void __launch_bounds__(128, MINB) k_cells_first(CotGeo g, CellsArgs a)
+__global__ void __launch_bounds__(128, MINB) k_cells_first(const __grid_constant__ CotGeo g, CellsArgs a, int upper)
 {
     constexpr int LPC = 32;
+    if ((int)blockIdx.x < upper) {
+        tree_node(g, a.wt, upper);
+        return;
+    }
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FastScratch &S = reinterpret_cast<FastScratch *>(smem_raw)[threadIdx.x >> 5];
     PSTAT_INIT();
@@ -2592,12 +2596,16 @@ __device__ __forceinline__ void warp_append(bool want, int i, int *list, int *co
 // accepted when every vertex lies inside every other line and the domain,
 // every edge runs forward and every corner turns left.  Accepted rings go to
 // the ring buffers with CST_FAST, the other cells to flist.
-__global__ void __launch_bounds__(FAST_THREADS) k_rings_cached(const __grid_constant__ CotGeo g, CellsArgs a)
+__global__ void __launch_bounds__(FAST_THREADS) k_rings_cached(const __grid_constant__ CotGeo g, CellsArgs a, int upper)
 {
+    if ((int)blockIdx.x < upper) {
+        tree_node(g, a.wt, upper);
+        return;
+    }
     __shared__ double2 LAB[FAST_THREADS];
     __shared__ double LC[FAST_THREADS];
     const int sl = threadIdx.x & 7, t0 = threadIdx.x & ~7;
-    const int i = (blockIdx.x * FAST_THREADS + threadIdx.x) >> 3;
+    const int i = ((blockIdx.x - upper) * FAST_THREADS + threadIdx.x) >> 3;
     int m = i < g.n ? a.nbn[i] : 0;
     if (m < 3 || m > FAST_NV) m = 0;
     const bool act = sl < m;
@@ -2797,6 +2805,7 @@ __global__ void __launch_bounds__(FAST_THREADS) k_certify(const __grid_constant_
     warp_append(st >= 0 && !ok && sl == 0, i, a.flist, a.ovf_count + 15);
 }
 
+static_assert(TREE_THREADS == 128, "tree_node runs in blocks of the ring kernels");
 static_assert(FAST_NV <= COT_SEG_NV, "rings of these kernels fit the 8-lane integration");
 static_assert(COT_BLEAF <= 64, "a mask bit a listed leaf");
 
@@ -3966,16 +3975,11 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     // the overflowed walks' list size, [12]: k_cells_heavy's fetch counter,
     // [13]: the split integration list's size, [14], [15]: flist's sizes for
     // k_cells_first and k_cells_walk
-    const int segs = (nb * BSEG + 127) / 128;
-    k_bucket_phi<<<segs, 128, 0, s>>>(g, a.w, a.perm, a.d, a.tptr, a.wt, a.wbar, a.ovf_count, 16);
-    k_tree_build<<<(nb * BSEG + TREE_THREADS - 1) / TREE_THREADS, TREE_THREADS, 0, s>>>(g, a.wt, a.wbar);
-    c.launches += 2;
+    k_bucket_bounds<<<(nb * BSEG + TREE_THREADS - 1) / TREE_THREADS, TREE_THREADS, 0, s>>>(g, a.w, a.perm, a.d, a.tptr, a.wt,
+                                                                                           a.ovf_count, 16);
+    c.launches++;
     int upper = 0;  // nodes of levels 1..lmax
     for (int L = 1; L <= lmax; L++) upper += g.lev_w[L] * g.lev_h[L];
-    if (upper > 0) {
-        k_tree_levels<<<upper, TREE_THREADS, 0, s>>>(g, a.wt);
-        c.launches++;
-    }
     const int sms = num_sms > 0 ? num_sms : 148;
     // what needs each pixel's part of a cell: weighted centroids (the
     // reference leaves tiny parts out) and the render; plain centroids and
@@ -3999,6 +4003,10 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     const int blocks = std::min(want, sms * (lpc == 32 ? per_sm32 : (lpc == 16 ? per_sm16 : per_sm8)));
     bool timed = c.profile && c.ev != nullptr && c.ev_used + 2 <= c.ev_cap;
     if (timed) cudaEventRecord(c.ev[c.ev_used], s);
+    if (lpc != 32 && upper > 0) {
+        k_tree_levels<<<upper, TREE_THREADS, 0, s>>>(g, a.wt, upper);
+        c.launches++;
+    }
     if (lpc == 32) {
         const int bw = std::min(g.n, sms * (g_blocks_per_smw > 0 ? g_blocks_per_smw : WALK_MINB) * CELLS_WPB);
         const int bf = std::min(g.n, sms * (g_blocks_per_smf > 0 ? g_blocks_per_smf : FIRST_MINB) * CELLS_WPB);
@@ -4009,10 +4017,11 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
                           a.ring_xy == nullptr;
         if (!fast) a.flist = nullptr;
         if (fast) {
-            k_rings_cached<<<(g.n + FAST_THREADS / 8 - 1) / (FAST_THREADS / 8), FAST_THREADS, 0, s>>>(g, a);
+            k_rings_cached<<<upper + (g.n + FAST_THREADS / 8 - 1) / (FAST_THREADS / 8), FAST_THREADS, 0, s>>>(g, a, upper);
             c.launches++;
         }
-        k_cells_first<FIRST_MINB><<<(bf + CELLS_WPB - 1) / CELLS_WPB, 32 * CELLS_WPB, sm, s>>>(g, a);
+        const int lv = fast ? 0 : upper;
+        k_cells_first<FIRST_MINB><<<lv + (bf + CELLS_WPB - 1) / CELLS_WPB, 32 * CELLS_WPB, sm, s>>>(g, a, lv);
         if (a.bcnt != nullptr) {
             const int bb = std::min(nb, sms * (g_blocks_per_smb > 0 ? g_blocks_per_smb : WALK_MINB) * CELLS_WPB);
             k_bucket_walk<WALK_MINB><<<(bb + CELLS_WPB - 1) / CELLS_WPB, 32 * CELLS_WPB, sm, s>>>(g, a);

@@ -87,8 +87,6 @@ struct CotSolver {
     double c1, c2, t0, tol;
     double H0;
     double rho[COT_MAX_HIST];
-    double alpha[COT_MAX_HIST];
-    double delta[COT_BASIS];            // direction = sum delta_j * basis_j
     double G[COT_BASIS * COT_BASIS];    // Gram matrix of the basis
     // current point
     double f, gd;
@@ -138,7 +136,6 @@ struct CellsArgs {
     const double *d;       // direction (nullable)
     const double *tptr;    // device scalar step (nullable => 0)
     double *wt;            // trial weights out
-    double *wbar;          // per bucket mean w/2 (scratch)
     double *mu;            // per cell mass out
     double *fc;            // per cell objective out, without its -w_i nu_i term
     int *nv;               // per cell ring size out
@@ -210,15 +207,13 @@ void launch_reduce(const CotGeo &g, const double *mu, const double *fc, const in
 int reduce_blocks(int n);
 
 // Launchers implemented in cot_solver.cu.
-void launch_begin_iteration(CotSolver *S, CotCtx &c);
-void launch_direction(const CotGeo &g, const CotSolver *S, const double *Sv, const double *Yv,
-                      const double *mu, double *d, CotCtx &c);
+void launch_begin_direction(const CotGeo &g, CotSolver *S, const double *Sv, const double *Yv, const double *mu,
+                            double *d, unsigned int *ticket, CotCtx &c);
 void launch_accept(const CotGeo &g, CotSolver *S, double *Sv, double *Yv, double *w,
                    const double *wt, double *mu, const double *mut, const double *d,
-                   double *partials, unsigned int *ticket, int initial, CotCtx &c);
+                   double *partials, unsigned int *ticket, int initial, const cudaGraphConditionalHandle *loop,
+                   CotCtx &c);
 void launch_reject(CotSolver *S, CotCtx &c);
-void launch_loop_cond(cudaGraphConditionalHandle hc, const CotSolver *S, CotCtx &c);
-void launch_reject_cond(cudaGraphConditionalHandle hc, CotSolver *S, CotCtx &c);
 void launch_init_from_eval(CotSolver *S, const CotEvalOut *out, CotCtx &c);
 void configure_cells_kernels();
 

@@ -6,8 +6,8 @@
 // iteration, ot_op.cuh:298-337).  Here the two-loop runs on the Gram matrix of
 // the basis {s_0..s_{m-1}, y_0..y_{m-1}, g} (the vector-free form of the
 // recursion): after each accepted step one pass over N computes the 5m+1 new
-// dot products, one device thread runs the recursion on the (2m+1)^2 matrix,
-// and one pass forms d = sum_j delta_j b_j.  Every reduction is a fixed-order
+// dot products, and one launch runs the recursion on the (2m+1)^2 matrix and
+// forms d = sum_j delta_j b_j.  Every reduction is a fixed-order
 // tree (per-block partials summed in block order by the last block), so a
 // solve is bit-reproducible run to run.  Line-search decisions are taken by
 // one device thread as well; the host only reads a flag.
@@ -84,75 +84,85 @@ __device__ double block_reduce(double v, double *sh)
 
 #define COT_F_NOISE 1e-12  // relative noise of the objective the line search tolerates
 
-// Line-search decision for the trial just reduced (one thread).
+// Line-search decision for the trial just reduced (one thread).  The control
+// block's fields are read together first and written together last: one after
+// the other, each waiting for the store before it, they took longer than the
+// reduction.
 __device__ void ls_decide(CotSolver *S, const CotEvalOut &o)
 {
-    S->evals++;
-    S->last = o;
-    S->accepted = 0;
-    if (S->mode == COT_SOLVE_REFERENCE) {
+    const int mode = S->mode, stop_nonempty = S->stop_nonempty, final_eval = S->final_eval, max_ls = S->max_ls;
+    const int evals = S->evals, rejects = S->ring_rejects, trials = S->trials;
+    const double t = S->t, t0 = S->t0, f = S->f, f_lo = S->f_lo, gd = S->gd, c1 = S->c1, c2 = S->c2;
+    const double hi = S->hi, lo = S->lo;
+    const bool bad = o.overflow > 0;
+    bool accepted = false, active = true;
+    double nt = t, nhi = hi, nlo = lo, nf_lo = f_lo;
+    int ntrials = trials, nfinal = final_eval;
+    bool count_reject = false;
+    if (mode == COT_SOLVE_REFERENCE) {
         // ot_op.cuh:360-426
-        if (o.overflow > 0) {
-            S->ring_rejects++;
-            S->t *= 0.5;
-        } else if (o.f < S->f) {
-            S->accepted = 1;
-            S->ls_active = 0;
-            return;
+        if (bad) {
+            count_reject = true;
+            nt = t * 0.5;
+        } else if (o.f < f) {
+            accepted = true;
         } else {
-            S->t *= 0.5;
+            nt = t * 0.5;
         }
-        if (S->t <= 1e-4 * S->t0) S->ls_active = 0;  // restart
-        return;
-    }
-    // a solve that only has to give every cell mass takes the first trial
-    // point where none is empty
-    if (S->stop_nonempty && o.empty == 0 && o.overflow == 0) {
-        S->accepted = 1;
-        S->ls_active = 0;
-        return;
-    }
-    // strong Wolfe: bracket by doubling, zoom by bisection
-    if (S->final_eval) {
-        S->accepted = 1;
-        S->ls_active = 0;
-        return;
-    }
-    double t = S->t;
-    bool bad = o.overflow > 0;
-    if (bad) S->ring_rejects++;
-    // approximate Wolfe (Hager and Zhang): near convergence the objective's
-    // evaluation noise (rounding in every cell's terms, about 1e-16 of |f|
-    // per cell) exceeds the decrease a step can still make, and comparisons
-    // of f stop telling steps apart.  A change of f within COT_F_NOISE |f|
-    // is then not held against the step, provided the slope at the trial
-    // point g(t).d <= (2 c1 - 1) g.d: the directional derivative decides.
-    const bool approx = o.f <= S->f + COT_F_NOISE * fabs(S->f) && o.gtd <= (2.0 * S->c1 - 1.0) * S->gd;
-    if (bad || (!approx && (!(o.f <= S->f + S->c1 * t * S->gd) || o.f >= S->f_lo))) {
-        S->hi = t;
-    } else if (fabs(o.gtd) <= S->c2 * fabs(S->gd)) {
-        S->accepted = 1;
-        S->ls_active = 0;
-        return;
-    } else if (o.gtd > 0.0) {
-        S->hi = t;
+        if (!accepted && nt <= 1e-4 * t0) active = false;  // restart
+    } else if (stop_nonempty && o.empty == 0 && !bad) {
+        // a solve that only has to give every cell mass takes the first trial
+        // point where none is empty
+        accepted = true;
+    } else if (final_eval) {
+        accepted = true;
     } else {
-        // a step taken on the approximate conditions may sit a rounding
-        // above f_lo: it moves the bracket's low end but never raises f_lo
-        S->lo = t;
-        S->f_lo = fmin(S->f_lo, o.f);
-    }
-    S->trials++;
-    if (S->trials >= S->max_ls) {
-        if (S->lo > 0.0) {
-            S->t = S->lo;
-            S->final_eval = 1;
+        // strong Wolfe: bracket by doubling, zoom by bisection
+        count_reject = bad;
+        // approximate Wolfe (Hager and Zhang): near convergence the objective's
+        // evaluation noise (rounding in every cell's terms, about 1e-16 of |f|
+        // per cell) exceeds the decrease a step can still make, and comparisons
+        // of f stop telling steps apart.  A change of f within COT_F_NOISE |f|
+        // is then not held against the step, provided the slope at the trial
+        // point g(t).d <= (2 c1 - 1) g.d: the directional derivative decides.
+        const bool approx = o.f <= f + COT_F_NOISE * fabs(f) && o.gtd <= (2.0 * c1 - 1.0) * gd;
+        if (bad || (!approx && (!(o.f <= f + c1 * t * gd) || o.f >= f_lo))) {
+            nhi = t;
+        } else if (fabs(o.gtd) <= c2 * fabs(gd)) {
+            accepted = true;
+        } else if (o.gtd > 0.0) {
+            nhi = t;
         } else {
-            S->ls_active = 0;  // failed
+            // a step taken on the approximate conditions may sit a rounding
+            // above f_lo: it moves the bracket's low end but never raises f_lo
+            nlo = t;
+            nf_lo = fmin(f_lo, o.f);
         }
-        return;
+        if (!accepted) {
+            ntrials = trials + 1;
+            if (ntrials >= max_ls) {
+                if (nlo > 0.0) {
+                    nt = nlo;
+                    nfinal = 1;
+                } else {
+                    active = false;  // failed
+                }
+            } else {
+                nt = isinf(nhi) ? 2.0 * t : 0.5 * (nlo + nhi);
+            }
+        }
     }
-    S->t = isinf(S->hi) ? 2.0 * t : 0.5 * (S->lo + S->hi);
+    S->evals = evals + 1;
+    S->last = o;
+    S->accepted = accepted ? 1 : 0;
+    if (accepted || !active) S->ls_active = 0;
+    S->ring_rejects = rejects + (count_reject ? 1 : 0);
+    S->t = nt;
+    S->hi = nhi;
+    S->lo = nlo;
+    S->f_lo = nf_lo;
+    S->trials = ntrials;
+    S->final_eval = nfinal;
 }
 
 // One pass over the cells: objective, gradient statistics, directional
@@ -164,7 +174,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_eval(int n, const double
                                                             int max_ring, double *partials, unsigned int *ticket,
                                                             CotEvalOut *out, CotSolver *S)
 {
-    __shared__ double sh[33];
+    __shared__ double sh[8], red[7][RED_THREADS / 32];
     __shared__ bool last;
     if (S != nullptr && (S->done || !S->ls_active)) return;
     double f = 0.0, gtd = 0.0, mx = 0.0, gn = 0.0, emp = 0.0, ovf = 0.0, mnv = 0.0;
@@ -181,21 +191,35 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_eval(int n, const double
         ovf += (nv[i] > max_ring) ? 1.0 : 0.0;
         mnv = fmax(mnv, (double)nv[i]);
     }
-    double v[RED_VALS];
-    v[0] = block_reduce<false>(f, sh);
-    v[1] = block_reduce<false>(gtd, sh);
-    v[2] = block_reduce<true>(mx, sh);
-    v[3] = block_reduce<false>(gn, sh);
-    v[4] = block_reduce<false>(emp, sh);
-    v[5] = block_reduce<false>(ovf, sh);
-    v[6] = block_reduce<true>(mnv, sh);
-    v[7] = 0.0;
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < RED_VALS; k++) partials[blockIdx.x * RED_VALS + k] = v[k];
-        __threadfence();
-        unsigned int tk = atomicAdd(ticket, 1u);
-        last = (tk == gridDim.x - 1);
+    // warps' sums in shared memory, added in warp order by a thread a value
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    f = wsum(f);
+    gtd = wsum(gtd);
+    mx = wmax(mx);
+    gn = wsum(gn);
+    emp = wsum(emp);
+    ovf = wsum(ovf);
+    mnv = wmax(mnv);
+    if (lane == 0) {
+        red[0][wid] = f;
+        red[1][wid] = gtd;
+        red[2][wid] = mx;
+        red[3][wid] = gn;
+        red[4][wid] = emp;
+        red[5][wid] = ovf;
+        red[6][wid] = mnv;
     }
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const int k = threadIdx.x;
+        const bool top = k == 2 || k == 6;
+        double r = top ? -INFINITY : 0.0;
+        for (int w = 0; w < RED_THREADS / 32; w++) r = top ? fmax(r, red[k][w]) : r + red[k][w];
+        partials[blockIdx.x * RED_VALS + k] = r;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
@@ -233,107 +257,93 @@ void launch_reduce(const CotGeo &g, const double *mu, const double *fc, const in
 }
 
 // ---------------------------------------------------------------------------
-// iteration control (single thread)
+// the start of an iteration
 // ---------------------------------------------------------------------------
 // Two-loop recursion on the Gram matrix (ot_op.cuh:291-351): delta gives
-// d = sum_j delta_j basis_j; then the descent safeguard.  One warp: the
-// (2m+1)^2 matrix is staged in shared memory and every row product is a
-// warp-wide dot product.
-__global__ void __launch_bounds__(32) k_begin_iteration(CotSolver *S)
+// d = sum_j delta_j basis_j; then the descent safeguard.  Every block runs the
+// recursion for itself (its first warp, the (2m+1)^2 matrix in shared memory)
+// and forms its part of d; the block that finishes last, when all have read
+// the control block, writes the iteration's start into it.  The recursion
+// keeps r = G delta in the lanes and updates it with every change of delta, so
+// a step is a shuffle and a fused multiply-add and not a dot product; as a
+// kernel of its own, with dot products, it took 12 us and its launch.
+__global__ void __launch_bounds__(RED_THREADS) k_begin_direction(int n, CotSolver *S, const double *__restrict__ Sv,
+                                                                 const double *__restrict__ Yv,
+                                                                 const double *__restrict__ mu,
+                                                                 const double *__restrict__ nu, double *__restrict__ d,
+                                                                 unsigned int *ticket)
 {
     __shared__ double G[COT_BASIS * COT_BASIS];
     __shared__ double dl[COT_BASIS];
-    __shared__ double rh[COT_MAX_HIST], alpha[COT_MAX_HIST];
-    const int lane = threadIdx.x;
+    __shared__ double gd_s;
+    __shared__ bool reset_s, last;
     // only at an iteration boundary: inside a device-driven loop this kernel
     // also runs before every further trial of a line search
     if (S->done || !S->need_begin) return;
     const int m = S->m, B = 2 * m + 1, gi = 2 * m;
     const int k = S->k;
-    // the control block's arrays once into shared memory: the recursion
-    // below is a chain of 2m dependent steps
-    for (int q = lane; q < B * B; q += 32) G[q] = S->G[(q / B) * COT_BASIS + q % B];
-    for (int c = lane; c < B; c += 32) dl[c] = (c == gi) ? -1.0 : 0.0;
-    for (int c = lane; c < m; c += 32) rh[c] = S->rho[c];
-    __syncwarp();
-    auto gdot = [&](int row) -> double {
-        double r = 0.0;
-        for (int c = lane; c < B; c += 32) r += G[row * B + c] * dl[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(FULLMASK, r, o);
-        return r;
-    };
-    const int cnt = k < m ? k : m;
-    const bool skip = (S->mode == COT_SOLVE_REFERENCE) && S->restart;
+    for (int q = threadIdx.x; q < B * B; q += blockDim.x) G[q] = S->G[(q / B) * COT_BASIS + q % B];
+    const int lane = threadIdx.x & 31;
+    const double rho = lane < m ? S->rho[lane] : 0.0;
     const double H0 = S->H0;
-    if (!skip) {
-        for (int i = 1; i <= cnt; i++) {
-            const int idx = ((k - i) % m + m) % m;
-            const double a = gdot(idx) * rh[idx];
-            __syncwarp();
-            if (lane == 0) {
-                alpha[i - 1] = a;
-                dl[m + idx] -= a;
+    const bool skip = (S->mode == COT_SOLVE_REFERENCE) && S->restart;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        constexpr int Q = (COT_BASIS + 31) / 32;
+        double x[Q], r[Q];  // delta and G delta, entry c in lane c % 32
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int c = lane + 32 * q;
+            x[q] = c == gi ? -1.0 : 0.0;
+            r[q] = c < B ? -G[c * B + gi] : 0.0;
+        }
+        const auto at = [&](int c) {
+            double v = r[0];
+#pragma unroll
+            for (int q = 1; q < Q; q++)
+                if (c >= 32 * q) v = r[q];
+            return __shfl_sync(FULLMASK, v, c & 31);
+        };
+        const auto add = [&](int c, double v) {  // delta_c += v
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                if (lane + 32 * q == c) x[q] += v;
+                if (lane + 32 * q < B) r[q] += v * G[(lane + 32 * q) * B + c];
             }
-            __syncwarp();
+        };
+        const int cnt = k < m ? k : m;
+        if (!skip) {
+            double alpha = 0.0;  // of step i in lane i - 1
+            for (int i = 1; i <= cnt; i++) {
+                const int idx = ((k - i) % m + m) % m;
+                const double a = at(idx) * __shfl_sync(FULLMASK, rho, idx);
+                if (lane == i - 1) alpha = a;
+                add(m + idx, -a);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                x[q] *= H0;
+                r[q] *= H0;
+            }
+            for (int i = cnt; i > 0; i--) {
+                const int idx = ((k - i) % m + m) % m;
+                const double beta = __shfl_sync(FULLMASK, rho, idx) * at(m + idx);
+                add(idx, __shfl_sync(FULLMASK, alpha, i - 1) - beta);
+            }
         }
-        for (int c = lane; c < B; c += 32) dl[c] *= H0;
-        __syncwarp();
-        for (int i = cnt; i > 0; i--) {
-            const int idx = ((k - i) % m + m) % m;
-            const double beta = rh[idx] * gdot(m + idx);
-            __syncwarp();
-            if (lane == 0) dl[idx] += alpha[i - 1] - beta;
-            __syncwarp();
+        double gd = at(gi);
+        const bool reset = !(gd < 0.0);  // not a descent direction: steepest descent
+        if (reset) gd = -G[gi * B + gi];
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int c = lane + 32 * q;
+            if (c < B) dl[c] = reset ? (c == gi ? -1.0 : 0.0) : x[q];
+        }
+        if (lane == 0) {
+            gd_s = gd;
+            reset_s = reset;
         }
     }
-    double gd = gdot(gi);
-    __syncwarp();
-    const bool reset = !(gd < 0.0);  // not a descent direction: steepest descent
-    if (reset) {
-        for (int c = lane; c < B; c += 32) dl[c] = (c == gi) ? -1.0 : 0.0;
-        gd = -G[gi * B + gi];
-    }
-    __syncwarp();
-    for (int c = lane; c < COT_BASIS; c += 32) S->delta[c] = c < B ? dl[c] : 0.0;
-    if (lane != 0) return;
-    if (!skip)
-        for (int i = 1; i <= cnt; i++) S->alpha[((k - i) % m + m) % m] = alpha[i - 1];
-    if (reset) {
-        S->k = 0;
-        S->H0 = 1.0;
-    }
-    S->need_begin = 0;
-    S->eval_mark = S->evals;
-    S->gnorm_stale = sqrt(S->gnorm2);
-    S->empty_stale = S->empty;
-    S->gd = gd;
-    S->t = S->t0;
-    S->lo = 0.0;
-    S->hi = INFINITY;
-    S->f_lo = S->f;
-    S->trials = 0;
-    S->ls_active = 1;
-    S->accepted = 0;
-    S->final_eval = 0;
-}
-
-void launch_begin_iteration(CotSolver *S, CotCtx &c)
-{
-    k_begin_iteration<<<1, 32, 0, c.s>>>(S);
-    c.launches++;
-}
-
-// d = sum_j delta_j basis_j
-__global__ void k_direction(int n, const CotSolver *__restrict__ S, const double *__restrict__ Sv,
-                            const double *__restrict__ Yv, const double *__restrict__ mu,
-                            const double *__restrict__ nu, double *__restrict__ d)
-{
-    // only right after k_begin_iteration (no trial evaluated since)
-    if (S->done || S->evals != S->eval_mark || !S->ls_active) return;
-    __shared__ double dl[COT_BASIS];
-    const int m = S->m;
-    for (int c = threadIdx.x; c < 2 * m + 1; c += blockDim.x) dl[c] = S->delta[c];
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double r = dl[2 * m] * (mu[i] - nu[i]);
@@ -344,67 +354,132 @@ __global__ void k_direction(int n, const CotSolver *__restrict__ S, const double
         }
         d[i] = r;
     }
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last || threadIdx.x != 0) return;
+    *ticket = 0u;
+    const int evals = S->evals, empty = S->empty;
+    const double gnorm2 = S->gnorm2, t0 = S->t0, f = S->f;
+    if (reset_s) {
+        S->k = 0;
+        S->H0 = 1.0;
+    }
+    S->need_begin = 0;
+    S->eval_mark = evals;
+    S->gnorm_stale = sqrt(gnorm2);
+    S->empty_stale = empty;
+    S->gd = gd_s;
+    S->t = t0;
+    S->lo = 0.0;
+    S->hi = INFINITY;
+    S->f_lo = f;
+    S->trials = 0;
+    S->ls_active = 1;
+    S->accepted = 0;
+    S->final_eval = 0;
 }
 
-void launch_direction(const CotGeo &g, const CotSolver *S, const double *Sv, const double *Yv, const double *mu,
-                      double *d, CotCtx &c)
+void launch_begin_direction(const CotGeo &g, CotSolver *S, const double *Sv, const double *Yv, const double *mu,
+                            double *d, unsigned int *ticket, CotCtx &c)
 {
-    int blocks = (g.n + 255) / 256;
-    if (blocks > 4 * 148) blocks = 4 * 148;
-    k_direction<<<blocks, 256, 0, c.s>>>(g.n, S, Sv, Yv, mu, g.nu, d);
+    int blocks = (g.n + RED_THREADS - 1) / RED_THREADS;
+    if (blocks > 2 * 148) blocks = 2 * 148;
+    k_begin_direction<<<blocks, RED_THREADS, 0, c.s>>>(g.n, S, Sv, Yv, mu, g.nu, d, ticket);
     c.launches++;
+}
+
+// Line search gave up (ot_op.cuh:413-425): keep the point, drop the history.
+__device__ __forceinline__ void reject(CotSolver *S)
+{
+    if (S->done || S->accepted || S->ls_active) return;
+    const int mode = S->mode, k = S->k, restarts = S->restarts, iter = S->iter, max_iter = S->max_iter;
+    S->need_begin = 1;
+    if (mode == COT_SOLVE_REFERENCE) {
+        S->restart = 1;
+    } else if (k == 0) {
+        S->failed = 1;
+        S->done = 1;
+        return;
+    }
+    S->k = 0;
+    S->H0 = 1.0;
+    S->restarts = restarts + 1;
+    S->iter = iter + 1;
+    if (iter + 1 >= max_iter) S->done = 1;
+}
+
+// Condition of the device-driven trial loop (a WHILE node of a CUDA graph):
+// go on until the solve is done or reaches the iteration where the host
+// wants to look (a progress report).
+__device__ __forceinline__ void loop_condition(cudaGraphConditionalHandle hc, const CotSolver *S)
+{
+    cudaGraphSetConditional(hc, (!S->done && S->iter < S->pause_iter) ? 1u : 0u);
 }
 
 // Accept the trial: s_h = t d, y_h = mu_t - mu, w = w_t, mu = mu_t, then the
 // new Gram entries s_h.y_j, y_h.s_j, y_h.y_j, g.s_j, g.y_j, g.g; the last
 // block updates the matrix, the history scalars (ot_op.cuh:434-466) and the
 // stop test (ot_op.cuh:468-476, 510).
-#define ACC_PER 4
+// LOOP: the end of a pass of the device-driven trial loop.  A pass whose trial
+// was not accepted ends here too (the rejection, where the line search gave
+// up), and the loop's condition is set.
+template <bool LOOP>
 __global__ void __launch_bounds__(RED_THREADS) k_accept(int n, CotSolver *S, double *Sv, double *Yv, double *w,
                                                        const double *__restrict__ wt, double *mu,
                                                        const double *__restrict__ mut, const double *__restrict__ nu,
                                                        const double *__restrict__ d, double *partials,
-                                                       unsigned int *ticket, int initial)
+                                                       unsigned int *ticket, int initial,
+                                                       cudaGraphConditionalHandle hc)
 {
     constexpr int NW = RED_THREADS / 32;
     __shared__ double red[(5 * COT_MAX_HIST + 1) * NW];
     __shared__ double tot[5 * COT_MAX_HIST + 1];
     __shared__ bool last;
-    if (S->done) return;
-    if (!initial && !S->accepted) return;
-    const int m = S->m;
-    const int h = S->k % m;
+    // (a rejection may raise `done` while blocks of the same launch read it:
+    // they leave either way)
+    if (S->done || (!initial && !S->accepted)) {
+        if (LOOP && blockIdx.x == 0 && threadIdx.x == 0) {
+            reject(S);
+            loop_condition(hc, S);
+        }
+        return;
+    }
+    const int m = S->m, k0 = S->k;
     const double t = S->t;
+    const int h = k0 % m;
     const int nvals = 5 * m + 1;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int per = (n + gridDim.x - 1) / gridDim.x;
     int b0 = blockIdx.x * per, b1 = min(n, b0 + per);
-    // new vectors (each thread later reads back only what it wrote)
-    for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
-        double mt = mut[i];
+    // the new vectors; the pair and the gradient of this thread's first
+    // ACC_REG elements stay in registers across the m passes below
+    constexpr int ACC_REG = 4;
+    double csn[ACC_REG], cyn[ACC_REG], cg[ACC_REG];
+    const auto take = [&](int i, double &sn, double &yn, double &g) {
+        const double mt = mut[i];
+        sn = yn = 0.0;
         if (!initial) {
-            Sv[(size_t)h * n + i] = __dmul_rn(t, d[i]);
-            Yv[(size_t)h * n + i] = mt - mu[i];
+            sn = __dmul_rn(t, d[i]);
+            yn = mt - mu[i];
+            Sv[(size_t)h * n + i] = sn;
+            Yv[(size_t)h * n + i] = yn;
             w[i] = wt[i];
         }
         mu[i] = mt;
-    }
-    int cnt = initial ? 0 : (S->k + 1 < m ? S->k + 1 : m);  // slots that hold pairs after this update
-    // the new pair and the gradient of this thread's first ACC_REG elements
-    // stay in registers across the m passes below (same sums, same order)
-    constexpr int ACC_REG = 4;
-    double csn[ACC_REG], cyn[ACC_REG], cg[ACC_REG];
+        g = mt - nu[i];
+    };
 #pragma unroll
     for (int q = 0; q < ACC_REG; q++) {
         const int i = b0 + threadIdx.x + q * blockDim.x;
         csn[q] = cyn[q] = cg[q] = 0.0;
-        if (i < b1) {
-            csn[q] = Sv[(size_t)h * n + i];
-            cyn[q] = Yv[(size_t)h * n + i];
-            cg[q] = mu[i] - nu[i];
-        }
+        if (i < b1) take(i, csn[q], cyn[q], cg[q]);
     }
     const int brest = b0 + threadIdx.x + ACC_REG * blockDim.x;
+    for (int i = brest; i < b1; i += blockDim.x) {
+        double sn, yn, g;
+        take(i, sn, yn, g);
+    }
+    int cnt = initial ? 0 : (k0 + 1 < m ? k0 + 1 : m);  // slots that hold pairs after this update
     // all 5m+1 sums in one sweep: per-warp partials in shared memory, summed
     // in warp order, then block partials summed in block order by the last
     // block (the order of a per-value block reduction, in one barrier)
@@ -416,7 +491,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_accept(int n, CotSolver *S, dou
             for (int q = 0; q < ACC_REG; q++) {
                 const int i = b0 + threadIdx.x + q * blockDim.x;
                 if (i < b1) {
-                    const double sj = Sv[(size_t)j * n + i], yj = Yv[(size_t)j * n + i];
+                    const double sj = j == h ? csn[q] : Sv[(size_t)j * n + i];
+                    const double yj = j == h ? cyn[q] : Yv[(size_t)j * n + i];
                     sy += csn[q] * yj;
                     ys += cyn[q] * sj;
                     yy += cyn[q] * yj;
@@ -475,88 +551,79 @@ __global__ void __launch_bounds__(RED_THREADS) k_accept(int n, CotSolver *S, dou
     __threadfence();
     for (int v = threadIdx.x; v < nvals; v += blockDim.x) tot[v] = sum_partials<false>(partials + v, gridDim.x, nvals);
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    *ticket = 0u;
     const int gi = 2 * m;
     double *G = S->G;
-    for (int j = 0; j < m; j++) {
-        int age = ((h - j) % m + m) % m;
-        bool valid = cnt > 0 && age < cnt;
-        if (!valid) continue;
+    // a thread a slot for the matrix
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const int age = ((h - j) % m + m) % m;
+        if (cnt == 0 || age >= cnt) continue;
         if (!initial) {
             G[h * COT_BASIS + (m + j)] = G[(m + j) * COT_BASIS + h] = tot[5 * j + 0];
-            G[(m + h) * COT_BASIS + j] = G[j * COT_BASIS + (m + h)] = tot[5 * j + 1];
+            if (j != h) G[(m + h) * COT_BASIS + j] = G[j * COT_BASIS + (m + h)] = tot[5 * j + 1];
             G[(m + h) * COT_BASIS + (m + j)] = G[(m + j) * COT_BASIS + (m + h)] = tot[5 * j + 2];
         }
         G[gi * COT_BASIS + j] = G[j * COT_BASIS + gi] = tot[5 * j + 3];
         G[gi * COT_BASIS + (m + j)] = G[(m + j) * COT_BASIS + gi] = tot[5 * j + 4];
     }
+    if (threadIdx.x != 0) return;
+    // the control block's fields are read together before the first is written
+    const CotEvalOut o = S->last;
+    const int mode = S->mode, iter = S->iter, max_iter = S->max_iter, stop_nonempty = S->stop_nonempty;
+    const int empty_stale = S->empty_stale, pause = S->pause_iter;
+    const double tol = S->tol, gnorm_stale = S->gnorm_stale;
+    *ticket = 0u;
     G[gi * COT_BASIS + gi] = tot[5 * m];
     // current point
-    S->f = S->last.f;
-    S->maxrel = S->last.maxrel;
-    S->gnorm2 = S->last.gnorm2;
-    S->empty = S->last.empty;
+    S->f = o.f;
+    S->maxrel = o.maxrel;
+    S->gnorm2 = o.gnorm2;
+    S->empty = o.empty;
+    bool done = stop_nonempty && o.empty == 0, converged = false;
+    int it = iter;
     if (initial) {
         // a Wolfe-mode solve whose start already meets the tolerance stops at
         // its first evaluation (as the oracle's restatement does); the
         // reference mode always takes an iteration, as direct_ot does
-        if (S->mode == COT_SOLVE_WOLFE && S->maxrel <= S->tol) {
-            S->converged = 1;
-            S->done = 1;
-        }
-        if (S->stop_nonempty && S->empty == 0) S->done = 1;
-        return;
-    }
-    double ys = G[(m + h) * COT_BASIS + h];
-    double yy = G[(m + h) * COT_BASIS + (m + h)];
-    if (S->mode == COT_SOLVE_REFERENCE) {
-        S->rho[h] = 1.0 / ys;
-        S->H0 = (yy > 1e-5) ? ys / yy : 1.0;
-        S->k++;
-        S->restart = 0;
-    } else if (ys > 0.0) {
-        S->rho[h] = 1.0 / ys;
-        S->H0 = ys / yy;
-        S->k++;
-    }
-    S->iter++;
-    S->need_begin = 1;
-    if (S->mode == COT_SOLVE_REFERENCE) {
-        if (S->gnorm_stale < S->tol && S->empty_stale == 0) { S->converged = 1; S->done = 1; }
+        converged = mode == COT_SOLVE_WOLFE && o.maxrel <= tol;
     } else {
-        if (S->maxrel <= S->tol) { S->converged = 1; S->done = 1; }
+        const double ys = tot[5 * h + 1], yy = tot[5 * h + 2];
+        if (mode == COT_SOLVE_REFERENCE) {
+            S->rho[h] = 1.0 / ys;
+            S->H0 = (yy > 1e-5) ? ys / yy : 1.0;
+            S->k = k0 + 1;
+            S->restart = 0;
+            converged = gnorm_stale < tol && empty_stale == 0;
+        } else {
+            if (ys > 0.0) {
+                S->rho[h] = 1.0 / ys;
+                S->H0 = ys / yy;
+                S->k = k0 + 1;
+            }
+            converged = o.maxrel <= tol;
+        }
+        it = iter + 1;
+        S->iter = it;
+        S->need_begin = 1;
+        done = done || it >= max_iter;
     }
-    if (S->stop_nonempty && S->empty == 0) S->done = 1;
-    if (S->iter >= S->max_iter) S->done = 1;
+    if (converged) S->converged = 1;
+    done = done || converged;
+    if (done) S->done = 1;
+    if (LOOP) cudaGraphSetConditional(hc, (!done && it < pause) ? 1u : 0u);
 }
 
 void launch_accept(const CotGeo &g, CotSolver *S, double *Sv, double *Yv, double *w, const double *wt, double *mu,
                    const double *mut, const double *d, double *partials, unsigned int *ticket, int initial,
-                   CotCtx &c)
+                   const cudaGraphConditionalHandle *loop, CotCtx &c)
 {
     int nb = reduce_blocks(g.n);
-    k_accept<<<nb, RED_THREADS, 0, c.s>>>(g.n, S, Sv, Yv, w, wt, mu, mut, g.nu, d, partials, ticket, initial);
+    if (loop != nullptr)
+        k_accept<true><<<nb, RED_THREADS, 0, c.s>>>(g.n, S, Sv, Yv, w, wt, mu, mut, g.nu, d, partials, ticket, initial,
+                                                    *loop);
+    else
+        k_accept<false><<<nb, RED_THREADS, 0, c.s>>>(g.n, S, Sv, Yv, w, wt, mu, mut, g.nu, d, partials, ticket, initial,
+                                                     cudaGraphConditionalHandle{});
     c.launches++;
-}
-
-// Line search gave up (ot_op.cuh:413-425): keep the point, drop the history.
-__device__ __forceinline__ void reject(CotSolver *S)
-{
-    if (S->done || S->accepted || S->ls_active) return;
-    S->need_begin = 1;
-    if (S->mode == COT_SOLVE_REFERENCE) {
-        S->restart = 1;
-    } else if (S->k == 0) {
-        S->failed = 1;
-        S->done = 1;
-        return;
-    }
-    S->k = 0;
-    S->H0 = 1.0;
-    S->restarts++;
-    S->iter++;
-    if (S->iter >= S->max_iter) S->done = 1;
 }
 
 __global__ void k_reject(CotSolver *S) { reject(S); }
@@ -564,34 +631,6 @@ __global__ void k_reject(CotSolver *S) { reject(S); }
 void launch_reject(CotSolver *S, CotCtx &c)
 {
     k_reject<<<1, 1, 0, c.s>>>(S);
-    c.launches++;
-}
-
-// Condition of the device-driven trial loop (a WHILE node of a CUDA graph):
-// go on until the solve is done or reaches the iteration where the host
-// wants to look (a progress report).
-__global__ void k_loop_cond(cudaGraphConditionalHandle hc, const CotSolver *S)
-{
-    cudaGraphSetConditional(hc, (!S->done && S->iter < S->pause_iter) ? 1u : 0u);
-}
-
-void launch_loop_cond(cudaGraphConditionalHandle hc, const CotSolver *S, CotCtx &c)
-{
-    k_loop_cond<<<1, 1, 0, c.s>>>(hc, S);
-    c.launches++;
-}
-
-// The end of a pass of the device-driven trial loop: reject (if the line
-// search just gave up) and the loop condition, in one launch.
-__global__ void k_reject_cond(cudaGraphConditionalHandle hc, CotSolver *S)
-{
-    reject(S);
-    cudaGraphSetConditional(hc, (!S->done && S->iter < S->pause_iter) ? 1u : 0u);
-}
-
-void launch_reject_cond(cudaGraphConditionalHandle hc, CotSolver *S, CotCtx &c)
-{
-    k_reject_cond<<<1, 1, 0, c.s>>>(hc, S);
     c.launches++;
 }
 
