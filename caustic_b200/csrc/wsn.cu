@@ -17,7 +17,6 @@
 #include <cutlass/gemm/collective/collective_builder.hpp>
 #include <cutlass/epilogue/collective/collective_builder.hpp>
 #include <cutlass/epilogue/fusion/operations.hpp>
-#include <cutlass/epilogue/thread/activation.h>
 #include <cutlass/util/packed_stride.hpp>
 
 #include <algorithm>
@@ -88,6 +87,22 @@ WS_GEMM_CONFIG(GemmCR32, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor
 // A[M,K], B[K,N] both row-major         (input gradient: dcols = dZ W)
 WS_GEMM_CONFIG(GemmRR, cutlass::layout::RowMajor, cutlass::layout::RowMajor, 128, 128)
 
+// max(v, 0) as k_bias_act takes it: a NaN becomes 0 (CUTLASS's ReLu keeps it).
+template <class V>
+struct ReluMax {
+    CUTLASS_HOST_DEVICE V operator()(V v) const { return fmaxf(v, 0.f); }
+};
+template <class V, int N>
+struct ReluMax<cutlass::Array<V, N>> {
+    CUTLASS_HOST_DEVICE cutlass::Array<V, N> operator()(cutlass::Array<V, N> const &v) const
+    {
+        cutlass::Array<V, N> r;
+        CUTLASS_PRAGMA_UNROLL
+        for (int i = 0; i < N; i++) r[i] = fmaxf(v[i], 0.f);
+        return r;
+    }
+};
+
 // The forward layer: y[M,N] (bf16) = relu(A[M,K] W[N,K]^T + bias), the sums of
 // GemmRC (same K blocks, same order) with the bias, the ReLU and the rounding
 // in the epilogue, so the fp32 result is never written.  NT columns a tile: as
@@ -97,8 +112,7 @@ struct GemmAct {
     using ElemAB = cutlass::bfloat16_t;
     using Tile = cute::Shape<cute::_128, cute::Int<NT>, cute::_64>;
     using Cluster = cute::Shape<cute::_1, cute::_1, cute::_1>;
-    using Fusion = cutlass::epilogue::fusion::LinCombPerColBiasEltAct<cutlass::epilogue::thread::ReLu, ElemAB, float,
-                                                                      float, void>;
+    using Fusion = cutlass::epilogue::fusion::LinCombPerColBiasEltAct<ReluMax, ElemAB, float, float, void>;
     using Epilogue = typename cutlass::epilogue::collective::CollectiveBuilder<
         cutlass::arch::Sm100, cutlass::arch::OpClassTensorOp, Tile, Cluster,
         cutlass::epilogue::collective::EpilogueTileAuto, float, float, void, cutlass::layout::RowMajor, 8, ElemAB,
@@ -170,9 +184,10 @@ inline bool wide(int C, int per, long long pieces, std::initializer_list<const v
 
 // im2col of one or two sources: channels [0, C0) from in0 (half the
 // resolution where UP: a nearest 2x upsampling read in place), the rest from
-// in1 (a skip connection), as the concatenated tensor would give.
+// in1 (a skip connection), as the concatenated tensor would give.  dh: the
+// rows of an image that this launch takes, from y0 on.
 template <bool UP>
-__global__ void __launch_bounds__(T) k_im2col16(unsigned total, int H, int W, int c0, int c1, FastDiv dk, FastDiv dc,
+__global__ void __launch_bounds__(T) k_im2col16(unsigned total, int H, int W, int y0, int c0, int c1, FastDiv dk, FastDiv dc,
                                                 FastDiv dw, FastDiv dh, const uint4 *__restrict__ in0,
                                                 const uint4 *__restrict__ in1, uint4 *__restrict__ cols)
 {
@@ -182,6 +197,7 @@ __global__ void __launch_bounds__(T) k_im2col16(unsigned total, int H, int W, in
         dc.divmod(k, tap, c);
         dw.divmod(row, t, x);
         dh.divmod(t, b, y);
+        y += y0;
         const int dy = (int)(tap * 11u >> 5), dx = (int)tap - 3 * dy;  // tap / 3, tap % 3 for tap < 9
         const int yy = (int)y + dy - 1, xx = (int)x + dx - 1;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -232,14 +248,15 @@ __device__ __forceinline__ float4 unpack4(uint2 v)
 
 // dz = dy where the layer's output y is positive (y null: everywhere; bf16, for the GEMMs), and
 // the column sums of that: a block's rows in a fixed order into part[block][C].
-// A thread takes 4 channels of every T / (C / 4)-th row.
+// A thread takes 4 channels of every T / w-th row, w pieces of 4 channels a
+// block: all C / 4, or T of them from the block's y on.
 __global__ void __launch_bounds__(T) k_act_back_sum(long long M, int Cn, int rows_per, const float4 *__restrict__ dy,
                                                     const uint2 *__restrict__ y, uint2 *__restrict__ dz,
                                                     float4 *__restrict__ part)
 {
     extern __shared__ float4 sh[];
-    const int c4 = Cn / 4, lanes = T / c4;
-    const int c = threadIdx.x % c4, lane = threadIdx.x / c4;
+    const int c4 = Cn / 4, w0 = blockIdx.y * T, w = min(c4 - w0, T), lanes = T / w;
+    const int at = threadIdx.x % w, c = w0 + at, lane = threadIdx.x / w;
     const long long r0 = (long long)blockIdx.x * rows_per, r1 = min(M, r0 + rows_per);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (lane < lanes) {
@@ -263,7 +280,7 @@ __global__ void __launch_bounds__(T) k_act_back_sum(long long M, int Cn, int row
     __syncthreads();
     if (lane == 0) {
         for (int l = 1; l < lanes; l++) {
-            const float4 v = sh[l * c4 + c];
+            const float4 v = sh[l * w + at];
             acc.x += v.x;
             acc.y += v.y;
             acc.z += v.z;
@@ -657,7 +674,7 @@ WS_API int ws_im2col(int B, int H, int W, int C, const void *in, void *cols, voi
     if (n > 0 && wide(C, 8, n / 8, {in, cols})) {
         const unsigned c8 = C / 8, total = (unsigned)(n / 8);
         k_im2col16<false><<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
-            total, H, W, (int)c8, 0, FastDiv(9 * c8), FastDiv(c8), FastDiv(W), FastDiv(H),
+            total, H, W, 0, (int)c8, 0, FastDiv(9 * c8), FastDiv(c8), FastDiv(W), FastDiv(H),
             static_cast<const uint4 *>(in), nullptr, static_cast<uint4 *>(cols));
         return last_error();
     }
@@ -668,12 +685,24 @@ WS_API int ws_im2col(int B, int H, int W, int C, const void *in, void *cols, voi
 
 WS_API int ws_im2col_up(int B, int H, int W, int C0, const void *up, int C1, const void *skip, void *cols, void *stream)
 {
-    const long long n = (long long)B * H * W * 9 * (C0 + C1);
-    if (n <= 0 || H % 2 || W % 2 || C0 % 8 || !wide(C1, 8, n / 8, {up, skip, cols})) return WS_EINVAL;
-    const unsigned c8 = (C0 + C1) / 8, total = (unsigned)(n / 8);
-    k_im2col16<true><<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
-        total, H, W, C0 / 8, C1 / 8, FastDiv(9 * c8), FastDiv(c8), FastDiv(W), FastDiv(H),
-        static_cast<const uint4 *>(up), static_cast<const uint4 *>(skip), static_cast<uint4 *>(cols));
+    if (B <= 0 || H <= 0 || W <= 0 || H % 2 || W % 2 || C0 <= 0 || C0 % 8 || C1 <= 0 || !wide(C1, 8, 0, {up, skip, cols}))
+        return WS_EINVAL;
+    // launches of at most 2^30 pieces: all images, a few, or bands of one's rows
+    const unsigned c0 = C0 / 8, c1 = C1 / 8, c8 = c0 + c1;
+    const long long row = (long long)W * 9 * c8, most = 1ll << 30;
+    if (row > most) return WS_EINVAL;
+    const int band = (int)std::min<long long>(H, most / row);
+    const int images = band < H ? 1 : (int)std::min<long long>(B, most / (row * H));
+    for (int b = 0; b < B; b += images)
+        for (int y = 0; y < H; y += band) {
+            const int ni = std::min(images, B - b), ny = std::min(band, H - y);
+            const unsigned total = (unsigned)(row * ny * ni);
+            k_im2col16<true><<<grid16(total), T, 0, static_cast<cudaStream_t>(stream)>>>(
+                total, H, W, y, c0, c1, FastDiv(9 * c8), FastDiv(c8), FastDiv(W), FastDiv(ny),
+                static_cast<const uint4 *>(up) + (size_t)b * (H / 2) * (W / 2) * c0,
+                static_cast<const uint4 *>(skip) + (size_t)b * H * W * c1,
+                static_cast<uint4 *>(cols) + ((size_t)b * H + y) * row);
+        }
     return last_error();
 }
 
@@ -692,14 +721,15 @@ WS_API size_t ws_act_back_sum_workspace(int C) { return (size_t)kSms * 4 * C * s
 WS_API int ws_act_back_sum(long long M, int C, const float *dy, const void *y, void *dz, float *gb, void *workspace,
                            size_t workspace_bytes, void *stream)
 {
-    if (M <= 0 || C <= 0 || !dy || !dz || !workspace || C % 8 || C > 1024) return WS_EINVAL;
+    if (M <= 0 || C <= 0 || !dy || !dz || !workspace || C % 8) return WS_EINVAL;
     if (!wide(C, 4, M * (C / 4), {dy, y, dz, workspace}) || workspace_bytes < ws_act_back_sum_workspace(C))
         return WS_EINVAL;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     float *part = static_cast<float *>(workspace);
     const int rows_per = (int)std::max<long long>((M + 4 * kSms - 1) / (4 * kSms), 32);
     const int blocks = (int)((M + rows_per - 1) / rows_per);
-    k_act_back_sum<<<blocks, T, T * sizeof(float4), s>>>(M, C, rows_per, reinterpret_cast<const float4 *>(dy),
+    const dim3 grid((unsigned)blocks, (unsigned)((C / 4 + T - 1) / T));
+    k_act_back_sum<<<grid, T, T * sizeof(float4), s>>>(M, C, rows_per, reinterpret_cast<const float4 *>(dy),
                                                          static_cast<const uint2 *>(y), static_cast<uint2 *>(dz),
                                                          reinterpret_cast<float4 *>(part));
     if (gb) k_sum_slices<<<(C + 31) / 32, dim3(32, 8), 0, s>>>(C, blocks, part, gb);

@@ -370,6 +370,9 @@ class WarmStartNet:
         if not self._sides:
             self._sides = [torch.cuda.Stream(device=self.dev) for _ in range(4)]
         self._held = []
+        # as forward(): the launches go to the caller's current stream, which
+        # the side streams wait for and are joined to
+        self._stream = torch.cuda.current_stream(self.dev).cuda_stream
         try:
             return self._backward(dpred)
         finally:

@@ -63,7 +63,7 @@ WS_API int ws_layer(int M, int N, int K, const void *A, const void *Wt, const fl
 /* The backward of such a layer's bias and ReLU from dy[M][C] (fp32) and its
  * output y (NULL: no ReLU): dz = dy where y > 0 (bf16, for the GEMMs), and
  * gb[C] += the column sums of the masked dy (fp32, in a fixed order; NULL: no
- * bias).  C a multiple of 8, at most 1024; workspace:
+ * bias).  C a multiple of 8; workspace:
  * ws_act_back_sum_workspace() bytes of device scratch. */
 WS_API int ws_act_back_sum(long long M, int C, const float *dy, const void *y, void *dz, float *gb, void *workspace,
                            size_t workspace_bytes, void *stream);
