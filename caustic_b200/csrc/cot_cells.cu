@@ -2717,6 +2717,11 @@ __global__ void __launch_bounds__(FAST_THREADS) k_certify(const __grid_constant_
     }
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) ru = fmaxf(ru, __shfl_xor_sync(FULLMASK, ru, o));
+    // squares of a ring (or a domain) this small vanish in single precision
+    if (ok && !(ru > 1e-30f && ru < 1e30f)) {
+        ok = false;
+        bc = 0;
+    }
     ru = sqrtf(ru) * 1.00001f;
     const double rr = (double)ru + 1e-13 * (fabs(mx) + fabs(my));
     const double r2 = rr * rr;

@@ -46,3 +46,19 @@ def test_jacobian_of_cached_rings(gpu):
     a, b = warm.mass_jacobian(w), solver_for(p).mass_jacobian(w)
     assert np.array_equal(a.indptr, b.indptr) and np.array_equal(a.indices, b.indices)
     assert np.array_equal(a.data, b.data)
+
+
+def test_domain_too_small_for_squares_in_single_precision(gpu):
+    """A domain 2^-90 across: the short path's single-precision tests see only
+    zeros there and leave every cell to the others."""
+    p = problems.make(4, g=129, res=200)
+    k = 2.0 ** -90
+    small = problems.SDOTProblem("small", p.xy * k, p.nu * k * k, p.picture, p.size, np.asarray(p.proj_domain) * k)
+    rng = np.random.default_rng(5)
+    s = solver_for(small)
+    w = np.zeros(p.n)
+    for amp in (0.0, 0.05, 1.0):
+        w = w + rng.normal(0.0, amp / p.n, p.n)
+        _, mu, _, _ = s.eval(w * k * k)
+        _, mu0, _, _ = solver_for(small).eval(w * k * k)
+        assert np.array_equal(mu, mu0), amp
