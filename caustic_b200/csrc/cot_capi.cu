@@ -1796,7 +1796,7 @@ static int newton_alloc(cot_handle *h)
     c.add(&P.nb_pa, N);
     c.add(&P.nb_pb, N);
     c.add(&P.nb_q, N);
-    c.add(&P.nb_part, (size_t)std::max(6 * pcg_blocks + 48, 256 * 5));
+    c.add(&P.nb_part, (size_t)std::max(6 * pcg_blocks + 48, 5 * reduce_blocks((int)N)));
     c.add(&P.nb_tau, 1);
     c.add(&P.pcg, 1);
     c.add(&P.nst, 1);

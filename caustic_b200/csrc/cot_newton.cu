@@ -129,31 +129,34 @@ __global__ void __launch_bounds__(NST_THREADS) k_newton_stats(int n, const doubl
         sh[4][wid] = mnv;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double r[NST_VALS] = {0.0, INFINITY, 0.0, 0.0, 0.0};
-        for (int k = 0; k < NST_THREADS / 32; k++) {
-            r[0] += sh[0][k];
-            r[1] = fmin(r[1], sh[1][k]);
-            r[2] = nmax_keep_nan(r[2], sh[2][k]);
-            r[3] += sh[3][k];
-            r[4] = fmax(r[4], sh[4][k]);
-        }
-        for (int k = 0; k < NST_VALS; k++) partials[(size_t)blockIdx.x * NST_VALS + k] = r[k];
+    // a thread a value for the warps, then a warp a value for the blocks (their
+    // partials, never NaN but in the sums, in one fixed order)
+    const auto join = [](int k, double x, double y) {
+        return k == 1 ? fmin(x, y) : (k == 2 || k == 4 ? fmax(x, y) : x + y);
+    };
+    if (threadIdx.x < NST_VALS) {
+        const int k = threadIdx.x;
+        double r = sh[k][0];
+        for (int w = 1; w < NST_THREADS / 32; w++) r = join(k, r, sh[k][w]);
+        partials[(size_t)k * gridDim.x + blockIdx.x] = r;
         __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
     __threadfence();
-    double r[NST_VALS] = {0.0, INFINITY, 0.0, 0.0, 0.0};
-    for (unsigned b = 0; b < gridDim.x; b++) {
-        const double *p = partials + (size_t)b * NST_VALS;
-        r[0] += __ldcg(p + 0);
-        r[1] = fmin(r[1], __ldcg(p + 1));
-        r[2] = nmax_keep_nan(r[2], __ldcg(p + 2));
-        r[3] += __ldcg(p + 3);
-        r[4] = fmax(r[4], __ldcg(p + 4));
+    if (wid < NST_VALS) {
+        double r = wid == 1 ? INFINITY : 0.0;
+#pragma unroll 5
+        for (unsigned b = lane; b < gridDim.x; b += 32) r = join(wid, r, __ldcg(partials + (size_t)wid * gridDim.x + b));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r = join(wid, r, __shfl_xor_sync(0xffffffffu, r, o));
+        if (lane == 0) sh[wid][0] = r;
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double r[NST_VALS] = {sh[0][0], sh[1][0], sh[2][0], sh[3][0], sh[4][0]};
     NewtonEvalStats o;
     o.gnorm2 = r[0];
     o.minmu = r[1];
@@ -167,8 +170,7 @@ __global__ void __launch_bounds__(NST_THREADS) k_newton_stats(int n, const doubl
 void launch_newton_stats(int n, const double *mu, const double *nu, const int *nv, double *partials,
                          unsigned int *ticket, NewtonEvalStats *out, CotCtx &c)
 {
-    const int blocks = std::min(reduce_blocks(n), 256);
-    k_newton_stats<<<blocks, NST_THREADS, 0, c.s>>>(n, mu, nu, nv, partials, ticket, out);
+    k_newton_stats<<<reduce_blocks(n), NST_THREADS, 0, c.s>>>(n, mu, nu, nv, partials, ticket, out);
     c.launches++;
 }
 

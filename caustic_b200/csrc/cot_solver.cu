@@ -14,20 +14,19 @@
 #include "cot_common.cuh"
 #include "../../include/causticot.h"
 #include <math.h>
+#include <algorithm>
 
 namespace cot {
 
 #define FULLMASK 0xffffffffu
 #define RED_THREADS 256
-#define RED_VALS 8
 
-int reduce_blocks(int n)
-{
-    int b = (n + RED_THREADS * 4 - 1) / (RED_THREADS * 4);
-    if (b < 1) b = 1;
-    if (b > 1024) b = 1024;
-    return b;
-}
+// Blocks of the reductions: a cell a thread up to 296 blocks (two an SM),
+// whose sums a warp adds in at most ten loads a lane.  With four cells a thread
+// and a thread that added the blocks one after the other, k_reduce_eval took
+// 11 us at 4,096 sites (4 blocks) and 23 at 262,144 (256 blocks); now 7 and
+// 12.
+int reduce_blocks(int n) { return std::max(1, std::min((n + RED_THREADS - 1) / RED_THREADS, 2 * 148)); }
 
 __device__ __forceinline__ double wsum(double v)
 {
@@ -42,26 +41,25 @@ __device__ __forceinline__ double wmax(double v)
     return v;
 }
 
-// Sum (or max) of stride-separated partials in block order, with the loads
-// issued ahead in groups (L2 reads: partials of other blocks are never taken
-// from a stale L1 line).
+// Sum (or max) of the blocks' partials of one value by a warp: lane l blocks l,
+// l + 32, ..., then the lanes, always in that order (L2 reads: partials of other
+// blocks are never taken from a stale L1 line).  lane_partials is a lane's part.
 template <bool MAX>
-__device__ __forceinline__ double sum_partials(const double *p, unsigned nblocks, size_t stride)
+__device__ __forceinline__ double lane_partials(const double *p, unsigned nblocks)
 {
-    double r = 0.0;
-    unsigned b = 0;
-    for (; b + 8 <= nblocks; b += 8) {
-        double v[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) v[q] = __ldcg(p + (size_t)(b + q) * stride);
-#pragma unroll
-        for (int q = 0; q < 8; q++) r = MAX ? fmax(r, v[q]) : r + v[q];
-    }
-    for (; b < nblocks; b++) {
-        const double v = __ldcg(p + (size_t)b * stride);
+    double r = MAX ? -INFINITY : 0.0;
+#pragma unroll 5
+    for (unsigned b = threadIdx.x & 31; b < nblocks; b += 32) {
+        const double v = __ldcg(p + b);
         r = MAX ? fmax(r, v) : r + v;
     }
     return r;
+}
+template <bool MAX>
+__device__ __forceinline__ double warp_partials(const double *p, unsigned nblocks)
+{
+    const double r = lane_partials<MAX>(p, nblocks);
+    return MAX ? wmax(r) : wsum(r);
 }
 
 // Fixed-order block reduction of one value (sum or max).  All threads call it.
@@ -215,7 +213,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_eval(int n, const double
         const bool top = k == 2 || k == 6;
         double r = top ? -INFINITY : 0.0;
         for (int w = 0; w < RED_THREADS / 32; w++) r = top ? fmax(r, red[k][w]) : r + red[k][w];
-        partials[blockIdx.x * RED_VALS + k] = r;
+        partials[k * gridDim.x + blockIdx.x] = r;
         __threadfence();
     }
     __syncthreads();
@@ -223,11 +221,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_eval(int n, const double
     __syncthreads();
     if (!last) return;
     __threadfence();
-    // one thread per value, each summing the blocks in order
-    if (threadIdx.x < 7) {
-        const int k = threadIdx.x;
-        sh[k] = (k == 2 || k == 6) ? sum_partials<true>(partials + k, gridDim.x, RED_VALS)
-                                   : sum_partials<false>(partials + k, gridDim.x, RED_VALS);
+    // a warp a value
+    if (wid < 7) {
+        const double *p = partials + wid * gridDim.x;
+        const double r = (wid == 2 || wid == 6) ? warp_partials<true>(p, gridDim.x) : warp_partials<false>(p, gridDim.x);
+        if (lane == 0) sh[wid] = r;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -431,8 +429,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_accept(int n, CotSolver *S, dou
                                                        unsigned int *ticket, int initial,
                                                        cudaGraphConditionalHandle hc)
 {
-    constexpr int NW = RED_THREADS / 32;
-    __shared__ double red[(5 * COT_MAX_HIST + 1) * NW];
+    constexpr int NW = RED_THREADS / 32, SLOTS = (COT_MAX_HIST + NW - 1) / NW;
+    __shared__ double sn_s[RED_THREADS], yn_s[RED_THREADS], g_s[RED_THREADS], red[NW];
     __shared__ double tot[5 * COT_MAX_HIST + 1];
     __shared__ bool last;
     // (a rejection may raise `done` while blocks of the same launch read it:
@@ -451,94 +449,77 @@ __global__ void __launch_bounds__(RED_THREADS) k_accept(int n, CotSolver *S, dou
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int per = (n + gridDim.x - 1) / gridDim.x;
     int b0 = blockIdx.x * per, b1 = min(n, b0 + per);
-    // the new vectors; the pair and the gradient of this thread's first
-    // ACC_REG elements stay in registers across the m passes below
-    constexpr int ACC_REG = 4;
-    double csn[ACC_REG], cyn[ACC_REG], cg[ACC_REG];
-    const auto take = [&](int i, double &sn, double &yn, double &g) {
-        const double mt = mut[i];
-        sn = yn = 0.0;
-        if (!initial) {
-            sn = __dmul_rn(t, d[i]);
-            yn = mt - mu[i];
-            Sv[(size_t)h * n + i] = sn;
-            Yv[(size_t)h * n + i] = yn;
-            w[i] = wt[i];
-        }
-        mu[i] = mt;
-        g = mt - nu[i];
-    };
+    const int cnt = initial ? 0 : (k0 + 1 < m ? k0 + 1 : m);  // slots that hold pairs after this update
+    const auto held = [&](int j) { return j < m && ((h - j) % m + m) % m < cnt; };
+    // 256 cells at a time: a thread a cell for the new vectors, which go to
+    // shared memory, then a warp a slot for the dot products with its pair, so
+    // that the slots' loads and sums run side by side (all threads on one slot
+    // after the other took 30 us for ten of them at 4,096 sites, this 12)
+    double acc[SLOTS][5], gg = 0.0;
 #pragma unroll
-    for (int q = 0; q < ACC_REG; q++) {
-        const int i = b0 + threadIdx.x + q * blockDim.x;
-        csn[q] = cyn[q] = cg[q] = 0.0;
-        if (i < b1) take(i, csn[q], cyn[q], cg[q]);
-    }
-    const int brest = b0 + threadIdx.x + ACC_REG * blockDim.x;
-    for (int i = brest; i < b1; i += blockDim.x) {
-        double sn, yn, g;
-        take(i, sn, yn, g);
-    }
-    int cnt = initial ? 0 : (k0 + 1 < m ? k0 + 1 : m);  // slots that hold pairs after this update
-    // all 5m+1 sums in one sweep: per-warp partials in shared memory, summed
-    // in warp order, then block partials summed in block order by the last
-    // block (the order of a per-value block reduction, in one barrier)
-    for (int j = 0; j < m; j++) {
-        double sy = 0.0, ys = 0.0, yy = 0.0, gs = 0.0, gy = 0.0;
-        const int age = ((h - j) % m + m) % m;
-        if (cnt > 0 && age < cnt) {
-#pragma unroll
-            for (int q = 0; q < ACC_REG; q++) {
-                const int i = b0 + threadIdx.x + q * blockDim.x;
-                if (i < b1) {
-                    const double sj = j == h ? csn[q] : Sv[(size_t)j * n + i];
-                    const double yj = j == h ? cyn[q] : Yv[(size_t)j * n + i];
-                    sy += csn[q] * yj;
-                    ys += cyn[q] * sj;
-                    yy += cyn[q] * yj;
-                    gs += cg[q] * sj;
-                    gy += cg[q] * yj;
-                }
+    for (int s = 0; s < SLOTS; s++)
+        for (int v = 0; v < 5; v++) acc[s][v] = 0.0;
+    for (int base = b0; base < b1; base += RED_THREADS) {
+        const int i = base + threadIdx.x;
+        double sn = 0.0, yn = 0.0, g = 0.0;
+        if (i < b1) {
+            const double mt = mut[i];
+            if (!initial) {
+                sn = __dmul_rn(t, d[i]);
+                yn = mt - mu[i];
+                Sv[(size_t)h * n + i] = sn;
+                Yv[(size_t)h * n + i] = yn;
+                w[i] = wt[i];
             }
-            for (int i = brest; i < b1; i += blockDim.x) {
-                double sj = Sv[(size_t)j * n + i], yj = Yv[(size_t)j * n + i];
-                double sn = Sv[(size_t)h * n + i], yn = Yv[(size_t)h * n + i];
-                double g = mu[i] - nu[i];
-                sy += sn * yj;
-                ys += yn * sj;
-                yy += yn * yj;
-                gs += g * sj;
-                gy += g * yj;
-            }
-            sy = wsum(sy);
-            ys = wsum(ys);
-            yy = wsum(yy);
-            gs = wsum(gs);
-            gy = wsum(gy);
+            mu[i] = mt;
+            g = mt - nu[i];
         }
-        if (lane == 0) {
-            red[(5 * j + 0) * NW + wid] = sy;
-            red[(5 * j + 1) * NW + wid] = ys;
-            red[(5 * j + 2) * NW + wid] = yy;
-            red[(5 * j + 3) * NW + wid] = gs;
-            red[(5 * j + 4) * NW + wid] = gy;
-        }
-    }
-    double gg = 0.0;
-#pragma unroll
-    for (int q = 0; q < ACC_REG; q++)
-        if (b0 + threadIdx.x + q * blockDim.x < b1) gg += cg[q] * cg[q];
-    for (int i = brest; i < b1; i += blockDim.x) {
-        double g = mu[i] - nu[i];
+        sn_s[threadIdx.x] = sn;
+        yn_s[threadIdx.x] = yn;
+        g_s[threadIdx.x] = g;
         gg += g * g;
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < SLOTS; s++) {
+            const int j = wid + NW * s;
+            if (!held(j)) continue;
+            double sj[NW], yj[NW];
+#pragma unroll
+            for (int q = 0; q < NW; q++) {
+                const int c = lane + 32 * q;
+                const bool in = base + c < b1;
+                sj[q] = j == h ? sn_s[c] : (in ? Sv[(size_t)j * n + base + c] : 0.0);
+                yj[q] = j == h ? yn_s[c] : (in ? Yv[(size_t)j * n + base + c] : 0.0);
+            }
+#pragma unroll
+            for (int q = 0; q < NW; q++) {
+                const int c = lane + 32 * q;
+                acc[s][0] += sn_s[c] * yj[q];
+                acc[s][1] += yn_s[c] * sj[q];
+                acc[s][2] += yn_s[c] * yj[q];
+                acc[s][3] += g_s[c] * sj[q];
+                acc[s][4] += g_s[c] * yj[q];
+            }
+        }
+        __syncthreads();
     }
     gg = wsum(gg);
-    if (lane == 0) red[5 * m * NW + wid] = gg;
+    if (lane == 0) red[wid] = gg;
+#pragma unroll
+    for (int s = 0; s < SLOTS; s++) {
+        const int j = wid + NW * s;
+        if (j >= m) continue;
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            const double r = wsum(acc[s][v]);
+            if (lane == 0) partials[(size_t)(5 * j + v) * gridDim.x + blockIdx.x] = r;
+        }
+    }
     __syncthreads();
-    for (int v = threadIdx.x; v < nvals; v += blockDim.x) {
+    if (threadIdx.x == 0) {
         double r = 0.0;
-        for (int k = 0; k < NW; k++) r += red[v * NW + k];
-        partials[(size_t)blockIdx.x * nvals + v] = r;
+        for (int k = 0; k < NW; k++) r += red[k];
+        partials[(size_t)5 * m * gridDim.x + blockIdx.x] = r;
     }
     __threadfence();
     __syncthreads();
@@ -549,7 +530,20 @@ __global__ void __launch_bounds__(RED_THREADS) k_accept(int n, CotSolver *S, dou
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int v = threadIdx.x; v < nvals; v += blockDim.x) tot[v] = sum_partials<false>(partials + v, gridDim.x, nvals);
+    // a warp a value, four values' loads at once
+    for (int v0 = wid; v0 < nvals; v0 += 4 * NW) {
+        double r[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int v = v0 + NW * q;
+            r[q] = v < nvals ? lane_partials<false>(partials + (size_t)v * gridDim.x, gridDim.x) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            r[q] = wsum(r[q]);
+            if (lane == 0 && v0 + NW * q < nvals) tot[v0 + NW * q] = r[q];
+        }
+    }
     __syncthreads();
     const int gi = 2 * m;
     double *G = S->G;
@@ -705,8 +699,8 @@ __global__ void k_fresnel_energy(int n, const double *__restrict__ cen, const do
     energy[i] = lam[i] * (t1 * t2);
 }
 
-// Fixed-order sum of x: block partials in block order; every block of the
-// scale kernel re-reduces the partials identically.
+// Fixed-order sum of x: block partials, which every block of the scale kernel
+// adds in the same order.
 __global__ void __launch_bounds__(RED_THREADS) k_sum_partials(int n, const double *__restrict__ x, double *partials)
 {
     __shared__ double sh[33];
@@ -725,8 +719,7 @@ __global__ void k_scale_to_total(int n, const double *__restrict__ energy, const
                                  double *__restrict__ nu)
 {
     if (eval->overflow > 0) return;
-    double s = 0.0;
-    for (int k = 0; k < nparts; k++) s += partials[k];
+    const double s = warp_partials<false>(partials, nparts);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) nu[i] = energy[i] / s * total;
 }
@@ -755,39 +748,43 @@ __global__ void k_aa_store(int n, const double *__restrict__ w, const double *__
     fh[i] = w[i] + alpha * g;
 }
 
-// row[j] = G_h . G_j for j < cnt (fixed order: block partials, last block sums)
+// row[j] = G_h . G_j for j < cnt (fixed order: warps' and blocks' partials, the
+// last block sums)
 __global__ void __launch_bounds__(RED_THREADS) k_aa_gram_row(int n, const double *__restrict__ G, int h, int cnt,
                                                             double *partials, unsigned int *ticket, double *row)
 {
-    __shared__ double sh[33];
+    constexpr int NW = RED_THREADS / 32;
+    __shared__ double red[COT_MAX_HIST][NW];
     __shared__ bool last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int per = (n + gridDim.x - 1) / gridDim.x;
     int b0 = blockIdx.x * per, b1 = min(n, b0 + per);
     const double *gh = G + (size_t)h * n;
+#pragma unroll 4
     for (int j = 0; j < cnt; j++) {
         const double *gj = G + (size_t)j * n;
         double v = 0.0;
         for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) v += gh[i] * gj[i];
-        v = block_reduce<false>(v, sh);
-        if (threadIdx.x == 0) partials[(size_t)blockIdx.x * COT_MAX_HIST + j] = v;
+        v = wsum(v);
+        if (lane == 0) red[j][wid] = v;
     }
-    if (threadIdx.x == 0) {
-        __threadfence();
-        unsigned int t = atomicAdd(ticket, 1u);
-        last = (t == gridDim.x - 1);
+    __syncthreads();
+    if ((int)threadIdx.x < cnt) {
+        double r = 0.0;
+        for (int k = 0; k < NW; k++) r += red[threadIdx.x][k];
+        partials[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = r;
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (threadIdx.x == 0) {
-        volatile double *p = partials;
-        for (int j = 0; j < cnt; j++) {
-            double r = 0.0;
-            for (unsigned b = 0; b < gridDim.x; b++) r += p[(size_t)b * COT_MAX_HIST + j];
-            row[j] = r;
-        }
-        *ticket = 0u;
+    for (int j = wid; j < cnt; j += NW) {
+        const double r = warp_partials<false>(partials + (size_t)j * gridDim.x, gridDim.x);
+        if (lane == 0) row[j] = r;
     }
+    if (threadIdx.x == 0) *ticket = 0u;
 }
 
 void launch_aa_store_gram(int n, const double *w, const double *mu, const double *nu, double alpha, double *G,
