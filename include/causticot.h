@@ -171,7 +171,8 @@ COT_API int cot_solve(cot_handle *h, double *w_inout, const cot_solve_opts *opts
  * handle's stream (which must not be the legacy default stream): handle k's
  * solve is one branch of the graph -- its first evaluation, then its own
  * device-driven trial loop -- and the branches run concurrently, so many
- * small instances share the GPU instead of queueing.  w_inout[k]: host array
+ * small instances share the GPU instead of queueing.  The first handle keeps
+ * the graph for the next batch of the same handles and problems.  w_inout[k]: host array
  * of handle k's n weights (start in, result out).  stats (nullable): count
  * entries; their ms is the time of the whole batch.  Progress callbacks are
  * not called.  COT_ENOTCONV when some solve stopped before the tolerance

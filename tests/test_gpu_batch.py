@@ -63,3 +63,32 @@ def test_autotune_and_batched_config_instances(gpu):
     ws, st, sec = batch.solve(probs[:3], cells_per_warp=res.cells_per_warp, bucket_size=res.bucket_size,
                               max_iter=40)
     assert sec > 0 and all(x.iterations <= 40 for x in st)
+
+
+def test_further_batches_of_the_same_handles(gpu):
+    """The batch's graph is kept: other starts and iteration limits, a new
+    problem in one handle, a longer history and a part of the handles give what
+    a solve by itself gives."""
+    probs = uneven()
+    sol = solvers_for(probs)
+
+    def check(pick, history, max_iter, scale):
+        w0 = [scale * np.sin(np.arange(probs[k].n)) / probs[k].n for k in pick]
+        wb, sb = capi.solve_batch([sol[k] for k in pick], w0, history=history, max_iter=max_iter, tol=1e-9)
+        for k, w, w_start, st in zip(pick, wb, w0, sb):
+            one = solvers_for([probs[k]])[0]
+            w1, s1 = one.solve(w_start, history=history, max_iter=max_iter, tol=1e-9)
+            assert np.array_equal(w, w1) and (st.iterations, st.f) == (s1.iterations, s1.f)
+
+    check(range(6), 7, 9, 0.0)
+    check(range(6), 7, 9, 0.1)
+    check(range(6), 5, 14, 0.1)
+    check(range(6), 12, 14, 0.0)   # the history's buffers grow
+    probs[3] = problems.make(1, instance=9, g=24, res=80)
+    p = probs[3]
+    sol[3].set_problem(p.xy, p.nu, p.picture, p.size, p.proj_domain)
+    check(range(6), 7, 9, 0.1)
+    check((0, 2, 4), 7, 9, 0.1)
+    sol[4].close()                 # a handle of a kept graph goes, another takes its place
+    sol[4] = solvers_for([probs[4]])[0]
+    check((0, 2, 4), 7, 9, 0.1)
