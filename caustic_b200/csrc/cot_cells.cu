@@ -3342,15 +3342,19 @@ __device__ __forceinline__ CellAcc integrate_pixels(PixScratch<8> &P, int nv, co
     }
     // the pixel columns and rows that each edge spans, from the cell's first
     // ones, 7 bits each (a larger one counts as 127); lower bounds as they are,
-    // upper ones from 127 down.  Widened by far more than their rounding: an
-    // edge a rounding short of a pixel line is the side of its pixel.
+    // upper ones from 127 down.  An edge a rounding short of a pixel line is the
+    // side of its pixel, so the ranges are widened by more than they and the
+    // pixels' sides can be off: five roundings (1.1e-16 each) of the site's and
+    // the domain's coordinates, in pixels.
+    const double ex = 1e-9 + 1e-15 * (fabs(si.x) + fabs(g.pd0) + g.nx * g.xs) * g.ixs;
+    const double ey = 1e-9 + 1e-15 * (fabs(si.y) + fabs(g.pd2) + g.ny * g.ys) * g.iys;
     for (int k = sl; k < nv; k += 8) {
         const int kn = (k + 1 == nv) ? 0 : k + 1;
         const auto at = [](double v, int o) { return (unsigned)min(max((int)floor(v) - o, 0), 127); };
-        const unsigned c0 = at((si.x + fmin(P.X[k], P.X[kn]) - g.pd0) * g.ixs - 1e-9, lx);
-        const unsigned c1 = at((si.x + fmax(P.X[k], P.X[kn]) - g.pd0) * g.ixs + 1e-9, lx);
-        const unsigned w0 = at((si.y + fmin(P.Y[k], P.Y[kn]) - g.pd2) * g.iys - 1e-9, ly);
-        const unsigned w1 = at((si.y + fmax(P.Y[k], P.Y[kn]) - g.pd2) * g.iys + 1e-9, ly);
+        const unsigned c0 = at((si.x + fmin(P.X[k], P.X[kn]) - g.pd0) * g.ixs - ex, lx);
+        const unsigned c1 = at((si.x + fmax(P.X[k], P.X[kn]) - g.pd0) * g.ixs + ex, lx);
+        const unsigned w0 = at((si.y + fmin(P.Y[k], P.Y[kn]) - g.pd2) * g.iys - ey, ly);
+        const unsigned w1 = at((si.y + fmax(P.Y[k], P.Y[kn]) - g.pd2) * g.iys + ey, ly);
         P.EB[k] = c0 | (127u - c1) << 8 | w0 << 16 | (127u - w1) << 24;
     }
     __syncwarp();

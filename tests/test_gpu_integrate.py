@@ -81,3 +81,38 @@ def test_pixel_parts_of_large_and_small_cells(gpu, g, res):
     flat.set_problem(p.xy, area, np.ones(res * res), p.size, p.proj_domain)
     img = flat.render(w)
     assert np.abs(img * res * res - 1.0).max() < 1e-9
+
+
+@pytest.mark.parametrize("offset,width,k", [(3.0e3, 0.7, 4), (1.0e4, 1.9, 8), (1.0e5, 0.7, 4), (-1.0e5, 1.9, 5)])
+def test_pixel_parts_of_aligned_cells_far_from_the_origin(gpu, offset, width, k):
+    """Weighted centroids and the render where a cell's sides lie on pixel
+    lines up to the coordinates' rounding, which is far above a pixel's own."""
+    gx, gy = 32, 24
+    nx, ny = k * gx, k * gy
+    pd = np.array([offset, offset + width, 0.5 * offset, 0.5 * offset + width * gy / gx])
+    X, Y = np.meshgrid(pd[0] + (np.arange(gx) + 0.5) * (pd[1] - pd[0]) / gx,
+                       pd[2] + (np.arange(gy) + 0.5) * (pd[3] - pd[2]) / gy)
+    rng = np.random.default_rng(k)
+    nu = rng.uniform(0.5, 1.5, gx * gy)
+    pic = rng.uniform(0.1, 1.0, nx * ny)
+    s = capi.Solver()
+    s.set_problem(np.column_stack([X.ravel(), Y.ravel()]), nu / nu.sum(), pic / pic.sum(), (nx, ny), pd)
+    xy, ex = s.centroids(np.zeros(gx * gy), weighted=True)
+    img = s.render(np.zeros(gx * gy))
+    # each cell is k x k whole pixels
+    rho = pic.reshape(gy, k, gx, k)
+    at = (np.arange(k) + 0.5) / k
+    mass = rho.sum((1, 3))
+    wx = (np.arange(gx) + (rho * at).sum((1, 3)) / mass) * width / gx
+    wy = (np.arange(gy)[:, None] + (rho * at[:, None, None]).sum((1, 3)) / mass) * width / gx
+    # four sides a pixel, each at most four units in the last place of a
+    # coordinate off its line
+    ulp = np.spacing(np.abs(pd).max())
+    rel = 16.0 * ulp / (width / nx)
+    tol = rel * width / gx + 4.0 * ulp
+    assert ex.all()
+    assert np.abs(xy[:, 0] - pd[0] - wx.ravel()).max() <= tol
+    assert np.abs(xy[:, 1] - pd[2] - wy.ravel()).max() <= tol
+    want = np.repeat(np.repeat(nu.reshape(gy, gx) / nu.sum() / k ** 2, k, 0), k, 1)
+    got = np.asarray(img).reshape(ny, nx)
+    assert np.abs(got / want - 1.0).max() <= rel
