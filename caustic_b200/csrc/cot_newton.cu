@@ -308,7 +308,11 @@ __device__ __forceinline__ bool pcg_reduce(double v0, double v1, double2 &out, i
                 ok = __all_sync(0xffffffffu, ok);
                 a0 = hsum32(a0);
                 if (TWO) a1 = hsum32(a1);
+                // each lane's fence after the slots that it read, then the warp's
+                // barrier: what the blocks wrote before their totals is ordered
+                // before lane 0's result (votes and shuffles order no memory)
                 __threadfence();
+                __syncwarp();
                 if (lane == 0 && ok) {
                     if (a0 != a0) a0 = __longlong_as_double(0x7ff8000000000000ll);
                     if (a1 != a1) a1 = __longlong_as_double(0x7ff8000000000000ll);
