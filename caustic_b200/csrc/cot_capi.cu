@@ -788,8 +788,9 @@ extern "C" int cot_eval(cot_handle *h, const double *w, double *f_total, double 
     // other in the staging vectors; small ones come back in one copy
     double *stage = P.tmp + 8;
     double *dmu = mu, *dg = g, *df = f_cell;
+    const bool host = mem != COT_MEM_DEVICE;  // as query_weights takes it
     size_t used = 0;
-    if (mem == COT_MEM_HOST) {
+    if (host) {
         const auto place = [&](double *want) { return want ? stage + N * used++ : nullptr; };
         dmu = place(mu);
         dg = place(g);
@@ -799,7 +800,7 @@ extern "C" int cot_eval(cot_handle *h, const double *w, double *f_total, double 
                                          reinterpret_cast<CotEvalOut *>(P.tmp), dmu, dg, df);
     h->ctx.launches++;
     COT_CUDA_TRY(cudaGetLastError());
-    if (mem == COT_MEM_HOST && P.n <= COT_STAGE_N) {
+    if (host && P.n <= COT_STAGE_N) {
         COT_CUDA_TRY(cudaMemcpyAsync(h->hQ, P.tmp, (8 + N * used) * sizeof(double), cudaMemcpyDeviceToHost, s));
         COT_CUDA_TRY(cudaStreamSynchronize(s));
         if (mu) std::memcpy(mu, h->hQ + (dmu - P.tmp), N * sizeof(double));
@@ -807,7 +808,7 @@ extern "C" int cot_eval(cot_handle *h, const double *w, double *f_total, double 
         if (f_cell) std::memcpy(f_cell, h->hQ + (df - P.tmp), N * sizeof(double));
     } else {
         COT_CUDA_TRY(cudaMemcpyAsync(h->hQ, P.tmp, sizeof o, cudaMemcpyDeviceToHost, s));
-        if (mem == COT_MEM_HOST) {
+        if (host) {
             if (mu) COT_CUDA_TRY(cudaMemcpyAsync(mu, dmu, N * sizeof(double), cudaMemcpyDeviceToHost, s));
             if (g) COT_CUDA_TRY(cudaMemcpyAsync(g, dg, N * sizeof(double), cudaMemcpyDeviceToHost, s));
             if (f_cell) COT_CUDA_TRY(cudaMemcpyAsync(f_cell, df, N * sizeof(double), cudaMemcpyDeviceToHost, s));
