@@ -147,6 +147,7 @@ class WarmStartNet:
         self._ws_bytes = 0
         self._sides = []  # side streams of backward(), and what runs on them
         self._held = []
+        self._tape = self._tape_stream = None  # what backward() reads, and the stream that wrote it
 
     def layers(self):
         for pair in self.enc:
@@ -311,7 +312,8 @@ class WarmStartNet:
         Returns fp32 [B, H*W] (N * w up to a constant)."""
         torch = self.torch
         L = load()
-        self._stream = torch.cuda.current_stream(self.dev).cuda_stream
+        stream = torch.cuda.current_stream(self.dev)
+        self._stream = stream.cuda_stream
         Bn, H, W, _ = x.shape
         tape = []
         skips = []
@@ -361,6 +363,7 @@ class WarmStartNet:
         pred = d[:, 0].contiguous().view(Bn, hh * ww)
         if keep:
             self._tape = (tape, Bn, H, W)
+            self._tape_stream = stream
         return pred
 
     def backward(self, dpred):
@@ -370,16 +373,24 @@ class WarmStartNet:
         if not self._sides:
             self._sides = [torch.cuda.Stream(device=self.dev) for _ in range(4)]
         self._held = []
-        # as forward(): the launches go to the caller's current stream, which
-        # the side streams wait for and are joined to
-        self._stream = torch.cuda.current_stream(self.dev).cuda_stream
+        # the launches go to the caller's current stream, which waits for
+        # forward()'s and which the side streams wait for and are joined to
+        cur, fwd, tape = torch.cuda.current_stream(self.dev), self._tape_stream, self._tape
+        if fwd is not None and fwd != cur:
+            cur.wait_stream(fwd)
+        self._stream = cur.cuda_stream
         try:
             return self._backward(dpred)
         finally:
-            cur = torch.cuda.current_stream(self.dev)
             for s in self._sides:
                 cur.wait_stream(s)
+            if fwd is not None and fwd != cur:
+                # the tape's memory goes back to forward()'s stream, which
+                # also runs the optimiser's step
+                fwd.wait_stream(cur)
+                self._stream = fwd.cuda_stream
             self._held = []
+            del tape
 
     def _backward(self, dpred):
         torch = self.torch

@@ -1,0 +1,53 @@
+"""Ways of calling the network that its fused layers have to bear: streams of
+the caller's choice, a trace set late, layers that are not plain."""
+import numpy as np
+import pytest
+
+from caustic_b200 import warmstart
+from test_gpu_warmstart_fused import build
+
+pytestmark = pytest.mark.gpu
+
+SHAPE = (4, 32, 32)
+
+
+def inputs(torch, seed=0):
+    B, H, W = SHAPE
+    rng = np.random.default_rng(seed)
+    x = torch.from_numpy(rng.normal(size=(B, H, W, warmstart.IN_CH)).astype(np.float32)).cuda().to(torch.bfloat16)
+    g = torch.from_numpy(rng.normal(size=(B, H * W)).astype(np.float32)).cuda()
+    return x, g
+
+
+def gradients(net):
+    return [t for c in net.layers() for t in (c.gw, c.gb) if t is not None]
+
+
+def test_backward_on_another_stream(gpu):
+    """The tape is forward()'s memory: backward() on another stream waits for
+    it, and gives it back only when it has been read."""
+    import torch
+
+    x, g = inputs(torch)
+    net = build(torch, 3, 32, 5)
+    net.zero_grad()
+    net.forward(x, keep=True)
+    want_dx = net.backward(g)
+    torch.cuda.synchronize()
+    want = [t.clone() for t in gradients(net)]
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    net.zero_grad()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(100_000_000)  # forward() is far from done when backward() is called
+        net.forward(x, keep=True)
+        sizes = [t.numel() * t.element_size() for e in net._tape[0] for t in e[1:3] if t is not None]
+    with torch.cuda.stream(b):
+        torch.cuda._sleep(100_000_000)  # and backward() when forward()'s stream allocates again
+        dx = net.backward(g)
+    with torch.cuda.stream(a):
+        over = [torch.full((n,), 0x7f, dtype=torch.uint8, device="cuda") for n in sizes]
+    torch.cuda.synchronize()
+    assert len(over) == len(sizes) and torch.equal(dx, want_dx)
+    for u, v in zip(gradients(net), want):
+        assert torch.equal(u, v)
