@@ -271,10 +271,12 @@ class WarmStartNet:
                       ws.data_ptr() if need else None, need, side.cuda_stream), "weight gradient")
         dcols = torch.empty(M, K, dtype=torch.float32, device=self.dev)
         self._gemm(GEMM_RR, M, K, c.cout, dz, c.w16, dcols)
-        if c.k == 1:
-            return dcols
-        dx = torch.empty(M, c.cin, dtype=torch.float32, device=self.dev)
-        _ok(L.ws_col2im(Bn, H, W, c.cin, dcols.data_ptr(), dx.data_ptr(), self._stream), "col2im")
+        dx = dcols
+        if c.k != 1:
+            dx = torch.empty(M, c.cin, dtype=torch.float32, device=self.dev)
+            _ok(L.ws_col2im(Bn, H, W, c.cin, dcols.data_ptr(), dx.data_ptr(), self._stream), "col2im")
+        if self.trace is not None:  # set after the forward pass
+            self.trace.append((c, dy.clone(), dz.clone(), dx.clone()))
         return dx
 
     def _conv_bwd(self, c: Conv, dy, cols, pre, Bn, H, W):

@@ -51,3 +51,22 @@ def test_backward_on_another_stream(gpu):
     assert len(over) == len(sizes) and torch.equal(dx, want_dx)
     for u, v in zip(gradients(net), want):
         assert torch.equal(u, v)
+
+
+def test_a_trace_set_after_the_forward_pass_is_recorded(gpu):
+    import torch
+
+    x, g = inputs(torch, 1)
+    got = []
+    for late in (False, True):
+        net = build(torch, 3, 32, 5)
+        net.zero_grad()
+        net.trace = None if late else []
+        net.forward(x, keep=True)
+        net.trace = []
+        net.backward(g)
+        got.append(([list(net.layers()).index(e[0]) for e in net.trace], [e[1:] for e in net.trace]))
+    assert got[0][0] == got[1][0] and len(got[0][0]) == 11
+    for u, v in zip(got[0][1], got[1][1]):
+        for p, q in zip(u, v):
+            assert torch.equal(p, q)
