@@ -65,7 +65,7 @@ def test_a_trace_set_after_the_forward_pass_is_recorded(gpu):
         net.forward(x, keep=True)
         net.trace = []
         net.backward(g)
-        got.append(([list(net.layers()).index(e[0]) for e in net.trace], [e[1:] for e in net.trace]))
+        got.append(([[c is e[0] for c in net.layers()].index(True) for e in net.trace], [e[1:] for e in net.trace]))
     assert got[0][0] == got[1][0] and len(got[0][0]) == 11
     for u, v in zip(got[0][1], got[1][1]):
         for p, q in zip(u, v):
