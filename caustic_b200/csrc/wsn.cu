@@ -708,7 +708,8 @@ WS_API int ws_im2col_up(int B, int H, int W, int C0, const void *up, int C1, con
 
 WS_API int ws_layer(int M, int N, int K, const void *A, const void *Wt, const float *bias, void *y, void *stream)
 {
-    if (M <= 0 || N <= 0 || K <= 0 || !A || !Wt || !bias || !y || K % 8 || N % 8) return WS_EINVAL;
+    if (M <= 0 || N <= 0 || K <= 0 || !A || !Wt || !bias || !y || K % 8 || !wide(N, 8, 0, {A, Wt, bias, y}))
+        return WS_EINVAL;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int rows = (M + 127) / 128;
     if (N > 64 && rows * ((N + 127) / 128) >= kSms) return GemmAct<128>::run(M, N, K, A, Wt, bias, y, s);

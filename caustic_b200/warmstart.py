@@ -320,9 +320,11 @@ class WarmStartNet:
         tape = []
         skips = []
         h, hh, ww = x.contiguous(), H, W
-        # a trace wants every layer's pre-activations and gradients: the layers
-        # run launch by launch then
-        fused = self.trace is None
+        # a trace wants every layer's pre-activations and gradients, and ws_layer
+        # has a ReLU and reads aligned biases: the layers run launch by launch
+        # where that does not fit
+        fused = self.trace is None and not any(
+            not c.relu or c.b.data_ptr() & 15 for pair in self.enc + self.dec for c in pair)
         for l in range(self.levels):
             for c in self.enc[l]:
                 if fused:

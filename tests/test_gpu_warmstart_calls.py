@@ -70,3 +70,47 @@ def test_a_trace_set_after_the_forward_pass_is_recorded(gpu):
     for u, v in zip(got[0][1], got[1][1]):
         for p, q in zip(u, v):
             assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("what", ["no relu", "bias off a 16-byte boundary"])
+def test_layers_that_the_fused_launch_does_not_take(gpu, what):
+    """They run launch by launch, as a trace makes them."""
+    import torch
+
+    x, g = inputs(torch, 2)
+    out = []
+    for traced in (True, False):
+        net = build(torch, 3, 32, 5)
+        if what == "no relu":
+            net.enc[1][0].relu = net.dec[0][1].relu = False
+        else:
+            c = net.dec[0][0]
+            room = torch.zeros(c.cout + 1, device="cuda")
+            room[1:].copy_(c.b)
+            c.b = room[1:]
+        net.trace = [] if traced else None
+        net.zero_grad()
+        pred = net.forward(x, keep=True)
+        dx = net.backward(g)
+        torch.cuda.synchronize()
+        out.append([pred, dx] + gradients(net))
+    for u, v in zip(*out):
+        assert torch.equal(u, v)
+
+
+def test_layer_refuses_addresses_that_its_vectors_do_not_fit(gpu):
+    import torch
+
+    L = warmstart.load()
+    a, w = (torch.zeros(64, 72, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    y = torch.zeros(64, 64, dtype=torch.bfloat16, device="cuda")
+    b = torch.zeros(64 + 4, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    assert L.ws_layer(64, 64, 72, a.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), s) == 0
+    assert L.ws_layer(64, 64, 72, a.data_ptr(), w.data_ptr(), b.data_ptr() + 16, y.data_ptr(), s) == 0
+    for args in ((a.data_ptr(), w.data_ptr(), b.data_ptr() + 4, y.data_ptr()),
+                 (a.data_ptr() + 8, w.data_ptr(), b.data_ptr(), y.data_ptr()),
+                 (a.data_ptr(), w.data_ptr() + 2, b.data_ptr(), y.data_ptr()),
+                 (a.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr() + 2)):
+        assert L.ws_layer(64, 64, 72, *args, s) == -1  # WS_EINVAL, before any launch
+    torch.cuda.synchronize()
