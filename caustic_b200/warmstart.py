@@ -84,6 +84,14 @@ def _p(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
+WS_EINVAL = -1
+
+
+class _NotFused(Exception):
+    """A layer that the fused launches do not take: no ReLU, a bias off a 16-byte
+    boundary, rows of more patches than one launch holds."""
+
+
 def _ok(rc, what):
     if rc != 0:
         raise RuntimeError(f"{what} failed with code {rc}")
@@ -242,11 +250,16 @@ class WarmStartNet:
             _ok(L.ws_im2col(Bn, H, W, c.cin, x.data_ptr(), cols.data_ptr(), self._stream), "im2col")
         else:
             cs = skip.shape[-1]
-            _ok(L.ws_im2col_up(Bn, H, W, c.cin - cs, x.data_ptr(), cs, skip.data_ptr(), cols.data_ptr(), self._stream),
-                "im2col_up")
+            rc = L.ws_im2col_up(Bn, H, W, c.cin - cs, x.data_ptr(), cs, skip.data_ptr(), cols.data_ptr(), self._stream)
+            if rc == WS_EINVAL:
+                raise _NotFused
+            _ok(rc, "im2col_up")
         y = torch.empty(M, c.cout, dtype=torch.bfloat16, device=self.dev)
-        _ok(L.ws_layer(M, c.cout, 9 * c.cin, cols.data_ptr(), c.w16.data_ptr(), c.b.data_ptr(), y.data_ptr(),
-                       self._stream), "layer")
+        rc = L.ws_layer(M, c.cout, 9 * c.cin, cols.data_ptr(), c.w16.data_ptr(), c.b.data_ptr(), y.data_ptr(),
+                        self._stream) if c.relu else WS_EINVAL
+        if rc == WS_EINVAL:
+            raise _NotFused
+        _ok(rc, "layer")
         return y, cols
 
     def _layer_bwd(self, c: Conv, dy, cols, y, Bn, H, W):
@@ -312,6 +325,16 @@ class WarmStartNet:
     def forward(self, x, keep: bool = False):
         """x: bf16 [B, H, W, 8] with H, W divisible by 2**(levels-1).
         Returns fp32 [B, H*W] (N * w up to a constant)."""
+        # a trace wants every layer's pre-activations and gradients, and not
+        # every layer fits ws_layer: they run launch by launch then
+        if self.trace is None:
+            try:
+                return self._forward(x, keep, True)
+            except _NotFused:
+                pass
+        return self._forward(x, keep, False)
+
+    def _forward(self, x, keep, fused):
         torch = self.torch
         L = load()
         stream = torch.cuda.current_stream(self.dev)
@@ -320,11 +343,6 @@ class WarmStartNet:
         tape = []
         skips = []
         h, hh, ww = x.contiguous(), H, W
-        # a trace wants every layer's pre-activations and gradients, and ws_layer
-        # has a ReLU and reads aligned biases: the layers run launch by launch
-        # where that does not fit
-        fused = self.trace is None and not any(
-            not c.relu or c.b.data_ptr() & 15 for pair in self.enc + self.dec for c in pair)
         for l in range(self.levels):
             for c in self.enc[l]:
                 if fused:
