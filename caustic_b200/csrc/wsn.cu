@@ -88,9 +88,16 @@ WS_GEMM_CONFIG(GemmCR32, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor
 WS_GEMM_CONFIG(GemmRR, cutlass::layout::RowMajor, cutlass::layout::RowMajor, 128, 128)
 
 // max(v, 0) as k_bias_act takes it: a NaN becomes 0 (CUTLASS's ReLu keeps it).
+// A positive value that bf16 rounds to 0 (at most half its smallest, 2^-133)
+// becomes -0: the backward pass reads the ReLU's mask from the output, and such
+// a value passes its gradient on.
+__host__ __device__ __forceinline__ float relu_marked(float v)
+{
+    return v > 0.f ? (v > 0x1p-134f ? v : -0.f) : 0.f;
+}
 template <class V>
 struct ReluMax {
-    CUTLASS_HOST_DEVICE V operator()(V v) const { return fmaxf(v, 0.f); }
+    CUTLASS_HOST_DEVICE V operator()(V v) const { return relu_marked(v); }
 };
 template <class V, int N>
 struct ReluMax<cutlass::Array<V, N>> {
@@ -98,7 +105,7 @@ struct ReluMax<cutlass::Array<V, N>> {
     {
         cutlass::Array<V, N> r;
         CUTLASS_PRAGMA_UNROLL
-        for (int i = 0; i < N; i++) r[i] = fmaxf(v[i], 0.f);
+        for (int i = 0; i < N; i++) r[i] = relu_marked(v[i]);
         return r;
     }
 };
@@ -246,8 +253,9 @@ __device__ __forceinline__ float4 unpack4(uint2 v)
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// dz = dy where the layer's output y is positive (y null: everywhere; bf16, for the GEMMs), and
-// the column sums of that: a block's rows in a fixed order into part[block][C].
+// dz = dy where the layer's output y is positive or -0 (relu_marked; y null:
+// everywhere; bf16, for the GEMMs), and the column sums of that: a block's rows
+// in a fixed order into part[block][C].
 // A thread takes 4 channels of every T / w-th row, w pieces of 4 channels a
 // block: all C / 4, or T of them from the block's y on.
 __global__ void __launch_bounds__(T) k_act_back_sum(long long M, int Cn, int rows_per, const float4 *__restrict__ dy,
@@ -264,10 +272,12 @@ __global__ void __launch_bounds__(T) k_act_back_sum(long long M, int Cn, int row
             float4 g = dy[r * c4 + c];
             if (y != nullptr) {
                 const float4 v = unpack4(y[r * c4 + c]);
-                g.x = v.x > 0.f ? g.x : 0.f;
-                g.y = v.y > 0.f ? g.y : 0.f;
-                g.z = v.z > 0.f ? g.z : 0.f;
-                g.w = v.w > 0.f ? g.w : 0.f;
+                // (the bits less one: below the sign bit for these alone)
+                const auto on = [](float u) { return (int)(__float_as_uint(u) - 1u) >= 0; };
+                g.x = on(v.x) ? g.x : 0.f;
+                g.y = on(v.y) ? g.y : 0.f;
+                g.z = on(v.z) ? g.z : 0.f;
+                g.w = on(v.w) ? g.w : 0.f;
             }
             dz[r * c4 + c] = pack4(g);
             acc.x += g.x;

@@ -56,12 +56,13 @@ WS_API int ws_im2col_up(int B, int H, int W, int C0, const void *up, int C1, con
                         void *stream);
 
 /* A layer in one launch: y[M][N] = relu(A[M][K] Wt[N][K]^T + bias) in bf16, the
- * values of ws_gemm (WS_GEMM_RC) followed by ws_bias_act.  K and N multiples
- * of 8; A, Wt, bias and y 16-byte aligned (WS_EINVAL otherwise). */
+ * values of ws_gemm (WS_GEMM_RC) followed by ws_bias_act, but -0 for a positive
+ * value that rounds to 0 (ws_act_back_sum's mark).  K and N multiples of 8; A,
+ * Wt, bias and y 16-byte aligned (WS_EINVAL otherwise). */
 WS_API int ws_layer(int M, int N, int K, const void *A, const void *Wt, const float *bias, void *y, void *stream);
 
 /* The backward of such a layer's bias and ReLU from dy[M][C] (fp32) and its
- * output y (NULL: no ReLU): dz = dy where y > 0 (bf16, for the GEMMs), and
+ * output y (NULL: no ReLU): dz = dy where y > 0 or -0 (bf16, for the GEMMs), and
  * gb[C] += the column sums of the masked dy (fp32, in a fixed order; NULL: no
  * bias).  C a multiple of 8; workspace:
  * ws_act_back_sum_workspace() bytes of device scratch. */

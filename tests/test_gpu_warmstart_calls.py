@@ -114,3 +114,31 @@ def test_layer_refuses_addresses_that_its_vectors_do_not_fit(gpu):
                  (a.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr() + 2)):
         assert L.ws_layer(64, 64, 72, *args, s) == -1  # WS_EINVAL, before any launch
     torch.cuda.synchronize()
+
+
+def test_gradients_pass_positive_values_below_the_smallest_bf16(gpu):
+    """Pre-activations that are positive in fp32 and round to 0 in bf16 pass
+    their gradient on, as the fp32 mask of the single launches has it."""
+    import torch
+
+    x, g = inputs(torch, 3)
+    out = []
+    for traced in (True, False):
+        net = build(torch, 2, 16, 5)
+        for c, r in ((net.enc[0][0], 0), (net.enc[1][1], 8), (net.dec[0][1], 1)):
+            # rows of no weights: their pre-activations are the biases
+            tiny = torch.tensor([1e-41, 2.0 ** -134, 5e-41, 0.0, -1e-41, 2.0 ** -133, 1.5e-38], device="cuda")
+            c.w[r:r + 7] = 0.0
+            c.w16[r:r + 7] = 0.0
+            c.b[r:r + 7] = tiny
+        net.trace = [] if traced else None
+        net.zero_grad()
+        pred = net.forward(x, keep=True)
+        dx = net.backward(g)
+        torch.cuda.synchronize()
+        assert float(net.enc[0][0].gb[0].abs()) > 0.0 or not traced
+        out.append([pred, dx] + gradients(net))
+    for u, v in zip(*out):
+        # the biases' gradients are fp32 sums in another order
+        assert torch.equal(u, v) if u.dim() > 1 else float((u - v).norm()) <= 1e-5 * float(u.norm())
+        assert torch.equal(u != 0, v != 0)
