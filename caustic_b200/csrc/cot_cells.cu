@@ -3813,6 +3813,11 @@ __global__ void __launch_bounds__(128, MINB) k_cells(CotGeo g, CellsArgs a, int 
                 a.nv[i] = MAXV + 1;
                 a.mu[i] = 0.0;
                 a.fc[i] = 0.0;
+                if (a.cen != nullptr) {
+                    a.exist[i] = 0;
+                    a.cen[2 * (size_t)i] = si.x;
+                    a.cen[2 * (size_t)i + 1] = si.y;
+                }
             }
             __syncwarp();
             continue;

@@ -298,8 +298,9 @@ typedef int (*cot_progress_fn)(void *user, int phase, int iteration, int status,
 COT_API int cot_set_progress(cot_handle *h, cot_progress_fn fn, void *user, int every);
 
 /* Density-weighted (weighted=1) or plain centroids of the cells at w and
- * the exist flags.  Replaces compute_center (basic_function.cuh:1056-1191,
- * ot_op.cuh:539-546). */
+ * the exist flags (an empty cell's centroid is its site; a cell of more than 256
+ * vertices counts as empty).  Replaces compute_center
+ * (basic_function.cuh:1056-1191, ot_op.cuh:539-546). */
 COT_API int cot_centroids(cot_handle *h, const double *w, double *xy, unsigned char *exist,
                   int weighted, int mem);
 

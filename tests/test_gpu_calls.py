@@ -24,3 +24,22 @@ def test_evaluation_takes_any_other_flag_as_host(gpu, n_side):
                        out[2].ctypes.data, 2)
     assert rc == 0 and val.value == f
     assert np.array_equal(out[0], mu) and np.array_equal(out[1], g) and np.array_equal(out[2], fc)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_centroid_of_a_cell_beyond_the_largest_ring(gpu, weighted):
+    """300 neighbours: more vertices than a ring holds.  The cell counts as
+    empty, whatever an earlier call found for it."""
+    th = 2 * np.pi * np.arange(300) / 300
+    # (radii that differ a little, or all the other cells' sides meet in one point)
+    r = 0.2 + 1e-6 * np.random.default_rng(0).uniform(-1.0, 1.0, 300)
+    xy = np.vstack([[[0.4, 0.45]], np.column_stack([0.4 + r * np.cos(th), 0.45 + r * np.sin(th)])])
+    n = len(xy)
+    s = capi.Solver()
+    s.set_problem(xy, np.ones(n) / n, np.ones(64 * 64) / 4096.0, (64, 64), np.array([0.0, 1.0, 0.0, 1.0]))
+    w = np.zeros(n)
+    w[0] = 3.0  # the whole domain
+    c, ex = s.centroids(w, weighted=weighted)
+    assert ex[0] and not ex[1:].any() and np.abs(c[0] - 0.5).max() < 1e-12
+    c, ex = s.centroids(np.zeros(n), weighted=weighted)
+    assert ex[1:].all() and not ex[0] and np.array_equal(c[0], xy[0])
