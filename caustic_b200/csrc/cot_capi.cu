@@ -52,9 +52,10 @@ struct cot_handle;
 
 struct CotProblemDev {
     // the groups' blocks: sites and pixels, bucket grid, and what the first
-    // call that needs it makes (and keeps): a history longer than COT_HIST0,
-    // the Newton solve, the render
-    void *b_sites = nullptr, *b_grid = nullptr, *b_hist = nullptr, *b_newton = nullptr, *b_image = nullptr;
+    // call that needs it makes (and keeps): the history, the centroids, the
+    // Anderson solve, the Newton solve, the render
+    void *b_sites = nullptr, *b_grid = nullptr, *b_hist = nullptr, *b_points = nullptr, *b_aa = nullptr;
+    void *b_newton = nullptr, *b_image = nullptr;
     int n = 0;
     int nb = 0;
     int nodes = 0;
@@ -119,7 +120,6 @@ struct CotProblemDev {
     unsigned int *nticket = nullptr;
 };
 
-#define COT_HIST0 10                      // L-BFGS (or Anderson) memory that every problem has room for
 #define COT_TMP(n) (8 + 3 * (size_t)(n))  // an evaluation's scalars, then three vectors
 #define COT_STAGE_N 4096                  // sites up to which an evaluation's host vectors go through pinned memory
 
@@ -247,7 +247,7 @@ using namespace cot;
 // the Newton and Anderson solves and the queries, which are sized by them too).
 static void free_sized_by_sites(CotProblemDev &P)
 {
-    void *blocks[] = {P.b_sites, P.b_hist, P.b_newton, P.b_image, P.cubtmp};
+    void *blocks[] = {P.b_sites, P.b_hist, P.b_points, P.b_aa, P.b_newton, P.b_image, P.cubtmp};
     for (void *p : blocks)
         if (p) cudaFree(p);
     // the grid's group is the other function's
@@ -486,21 +486,7 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
         c.add(&P.bpart, build_partials_doubles());
         c.add(&P.bticket, 2);
         c.add(&P.bstat, 256);
-        c.add(&P.Sv, COT_HIST0 * N);
-        c.add(&P.Yv, COT_HIST0 * N);
-        c.add(&P.pcen, 4 * N);
-        c.add(&P.pex, 2 * N);
-        c.add(&P.aa_src, 2 * N);
-        c.add(&P.aa_inl, 3 * N);
-        c.add(&P.aa_insl, 3 * N);
-        c.add(&P.aa_hgt, N);
-        c.add(&P.aa_lam, N);
-        c.add(&P.aa_energy, N);
-        c.add(&P.aa_row, COT_MAX_HIST);
-        c.add(&P.aa_coef, COT_MAX_HIST);
-        c.add(&P.aa_step, 1);
         cudaError_t e = c.alloc(&P.b_sites);
-        if (e == cudaSuccess) P.hist_alloc = COT_HIST0;
         if (e == cudaSuccess) e = cudaMemsetAsync(P.bticket, 0, 2 * sizeof(unsigned int), s);
         if (e == cudaSuccess) e = cudaMemsetAsync(P.hticket, 0, COT_HSPLIT_CAP * sizeof(unsigned int), s);
         if (e != cudaSuccess) {
@@ -677,6 +663,18 @@ static int need_hperm(cot_handle *h, CotProblemDev &P)
     COT_CUDA_TRY(cudaStreamSynchronize(h->stream));
     P.hperm_valid = true;
     return COT_OK;
+}
+
+// Room for the centroids and exist flags.
+static int need_points(cot_handle *h, const char *what)
+{
+    CotProblemDev &P = h->P;
+    if (P.b_points) return COT_OK;
+    Carve c;
+    c.add(&P.pcen, 4 * P.cap_n);
+    c.add(&P.pex, 2 * P.cap_n);
+    const cudaError_t e = c.alloc(&P.b_points);
+    return e == cudaSuccess ? COT_OK : fail(h, COT_ENOMEM, what, cudaGetErrorString(e));
 }
 
 // The weights of a query as a device vector in caller order: device arrays
@@ -899,6 +897,7 @@ extern "C" int cot_centroids(cot_handle *h, const double *w, double *xy, unsigne
     size_t N = (size_t)P.n;
     int r;
     const double *dw;
+    if ((r = need_points(h, "cot_centroids: device allocation")) != COT_OK) return r;
     if ((r = query_weights(h, w, mem, &dw)) != COT_OK) return r;
     CellsArgs a = cells_args(P, dw, nullptr, nullptr, true);
     a.cen = P.pcen;
@@ -1140,20 +1139,40 @@ static int need_history(cot_handle *h, int m)
 {
     CotProblemDev &P = h->P;
     if (P.hist_alloc >= m) return COT_OK;
-    void *old = P.b_hist;
+    // the shorter one goes first: both at once may not fit
+    if (P.b_hist) cudaFree(P.b_hist);
+    P.b_hist = nullptr;
+    P.Sv = P.Yv = nullptr;
+    P.hist_alloc = 0;
     // sized for the buffers' capacity: a later problem that fits them reuses these
-    Carve hc;
-    hc.add(&P.Sv, (size_t)m * P.cap_n);
-    hc.add(&P.Yv, (size_t)m * P.cap_n);
-    const cudaError_t e = hc.alloc(&P.b_hist);
-    if (e != cudaSuccess) {
-        P.b_hist = old;  // the shorter history stays
-        return fail(h, COT_ENOMEM, "solve: history allocation", cudaGetErrorString(e));
-    }
-    if (old) cudaFree(old);
+    Carve c;
+    c.add(&P.Sv, (size_t)m * P.cap_n);
+    c.add(&P.Yv, (size_t)m * P.cap_n);
+    const cudaError_t e = c.alloc(&P.b_hist);
+    if (e != cudaSuccess) return fail(h, COT_ENOMEM, "solve: history allocation", cudaGetErrorString(e));
     P.hist_alloc = m;
     P.gen = ++g_problem_gen;  // a graph that captured the old history buffers is stale
     return COT_OK;
+}
+
+// Room for the Anderson solve's vectors.
+static int need_aa(cot_handle *h)
+{
+    CotProblemDev &P = h->P;
+    if (P.b_aa) return COT_OK;
+    const size_t N = P.cap_n;
+    Carve c;
+    c.add(&P.aa_src, 2 * N);
+    c.add(&P.aa_inl, 3 * N);
+    c.add(&P.aa_insl, 3 * N);
+    c.add(&P.aa_hgt, N);
+    c.add(&P.aa_lam, N);
+    c.add(&P.aa_energy, N);
+    c.add(&P.aa_row, COT_MAX_HIST);
+    c.add(&P.aa_coef, COT_MAX_HIST);
+    c.add(&P.aa_step, 1);
+    const cudaError_t e = c.alloc(&P.b_aa);
+    return e == cudaSuccess ? COT_OK : fail(h, COT_ENOMEM, "cot_solve_aarl: device allocation", cudaGetErrorString(e));
 }
 
 // History buffers and the device control block of a solve from the weights
@@ -1597,10 +1616,11 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
         }
         hgt[p] = in->height[i];
     }
-    // device workspace of this call
     // the Anderson history takes the L-BFGS history's place, which is free
     // again when its phase begins
-    if ((r = need_history(h, std::max(M, o.history))) != COT_OK) return r;
+    if ((r = need_history(h, in->lbfgs_prepass ? std::max(M, o.history) : M)) != COT_OK) return r;
+    if ((r = need_points(h, "cot_solve_aarl: device allocation")) != COT_OK) return r;
+    if ((r = need_aa(h)) != COT_OK) return r;
     double *dsrc = P.aa_src, *dinl = P.aa_inl, *dinsl = P.aa_insl, *dhgt = P.aa_hgt, *lam = P.aa_lam;
     double *energy = P.aa_energy, *cen = P.pcen, *G = P.Sv, *F = P.Yv, *row = P.aa_row, *coef = P.aa_coef;
     double *step = P.aa_step;

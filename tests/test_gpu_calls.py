@@ -43,3 +43,35 @@ def test_centroid_of_a_cell_beyond_the_largest_ring(gpu, weighted):
     assert ex[0] and not ex[1:].any() and np.abs(c[0] - 0.5).max() < 1e-12
     c, ex = s.centroids(np.zeros(n), weighted=weighted)
     assert ex[1:].all() and not ex[0] and np.array_equal(c[0], xy[0])
+
+
+def test_memory_is_taken_by_the_calls_that_need_it(gpu):
+    """A handle that evaluates holds no history, centroids or Anderson vectors;
+    a longer history takes the shorter one's place."""
+    import torch
+
+    def used():
+        torch.cuda.synchronize()
+        free, total = torch.cuda.mem_get_info()
+        return total - free
+
+    p = problems.make(4, g=512, res=256)  # 262,144 sites
+    w = np.random.default_rng(2).normal(0.0, 0.05 / p.n, p.n)
+    warm = solver_for(problems.make(1, g=16, res=32))  # the context, the kernels
+    warm.eval(np.zeros(256))
+    warm.close()
+    n0 = used()
+    s = solver_for(p)
+    s.eval(w)
+    base = used() - n0
+    mb = 1 << 20
+    # per site: rings 640, neighbour caches 136, vectors and lists 140, the sort
+    # 24, its share of a bucket of 16 with its leaf list 22
+    assert base <= 980 * p.n + 24 * mb, base / p.n
+    s.centroids(w)
+    pts = used() - n0 - base
+    assert pts <= p.n * 34 + 4 * mb
+    for m in (10, 20, 32):
+        s.solve(np.zeros(p.n), mode=capi.SOLVE_WOLFE, tol=1e-12, history=m, max_iter=1)
+        hist = used() - n0 - base - pts
+        assert 16 * m * p.n <= hist <= 16 * m * p.n + 16 * mb, (m, hist / p.n)
