@@ -62,3 +62,23 @@ def test_domain_too_small_for_squares_in_single_precision(gpu):
         _, mu, _, _ = s.eval(w * k * k)
         _, mu0, _, _ = solver_for(small).eval(w * k * k)
         assert np.array_equal(mu, mu0), amp
+
+
+@pytest.mark.parametrize("n,width", [(16384, 0.01), (45000, 0.0005)])  # 8 lanes a cell, and 4
+def test_clustered_sites_have_the_bits_of_a_cold_evaluation(gpu, n, width):
+    """Half of the sites in a few buckets: leaves of more sites than the short
+    path looks through go to the warp kernels."""
+    rng = np.random.default_rng(n)
+    xy = rng.uniform(0.0, 1.0, (n, 2))
+    xy[: n // 2] = np.clip(0.5 + width * rng.normal(size=(n // 2, 2)), 0.0, 1.0)
+    nu = rng.uniform(0.5, 1.5, n)
+    pic = problems.gaussian_mixture(rng, 6, 128, 128)
+    p = problems.SDOTProblem("clustered", xy, nu / nu.sum(), pic, (128, 128))
+    s = solver_for(p)
+    for amp in (0.0, 1e-3, 0.0):
+        w = amp * width * width / n * rng.normal(size=n)
+        f, mu, g, fc = s.eval(w)
+        fresh = solver_for(p)
+        f0, mu0, g0, fc0 = fresh.eval(w)
+        assert np.array_equal(mu, mu0) and np.array_equal(fc, fc0) and f == f0, amp
+        fresh.close()
