@@ -903,6 +903,7 @@ extern "C" int cot_centroids(cot_handle *h, const double *w, double *xy, unsigne
     a.cen = P.pcen;
     a.exist = P.pex;
     a.weighted = weighted ? 1 : 0;
+    a.rings_only = weighted ? 0 : 1;
     launch_eval(P.geo, a, h->cfg.cells_per_warp, h->num_sms, h->c());
     const bool host = mem != COT_MEM_DEVICE;
     double *xy_out = host ? P.pcen + 2 * N : xy;

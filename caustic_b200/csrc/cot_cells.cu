@@ -3501,7 +3501,8 @@ constexpr int PIX_WARP_SMEM =
 // weighted centroids and the render.  The cells of the split list take
 // COT_SPLIT warps (each every eighth row of pixels), those of the heavy list
 // one, first; the others share one with three more.
-template <int MINB>
+// L = 32: those have a warp each as well.
+template <int MINB, int L>
 __global__ void __launch_bounds__(128, MINB) k_integrate_pixels(const __grid_constant__ CotGeo g, CellsArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -3546,11 +3547,13 @@ __global__ void __launch_bounds__(128, MINB) k_integrate_pixels(const __grid_con
         int f = 0;
         if (lane == 0) f = atomicAdd(fetch, 1);
         f = __shfl_sync(FULLMASK, f, 0);
-        if (f >= (g.n + 3) / 4 + nh + np) break;
-        if (f < nh + np) {
+        if (f >= (L == 32 ? g.n : (g.n + 3) / 4) + nh + np) break;
+        if (L == 32 || f < nh + np) {
             const int slot = f / COT_SPLIT, part = f < np ? f % COT_SPLIT : 0;
-            const int i = f < np ? a.hsplit[slot] : a.hlist[f - np];
+            const int i = f < np ? a.hsplit[slot] : (f < nh + np ? a.hlist[f - np] : f - nh - np);
+            if (f >= nh + np && (nh > 0 || np > 0) && a.cstate[i] == CST_HEAVY) continue;
             const int nv = a.nv[i];
+            if (nv > COT_RCAP) continue;  // the large-ring pass
             if (lane < nv) {
                 const double2 v = a.rbuf[ring_at(i, lane)];
                 S.X[lane] = v.x;
@@ -3559,7 +3562,8 @@ __global__ void __launch_bounds__(128, MINB) k_integrate_pixels(const __grid_con
             __syncwarp();
             const auto ring = [&](int k) { return make_double2(S.X[k], S.Y[k]); };
             const double2 si = g.xy[i];
-            CellAcc acc = pixels_whole(S, nv, geo(i, nv, ring), si, part, f < np ? COT_SPLIT : 1);
+            CellAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+            if (nv >= 3) acc = pixels_whole(S, nv, geo(i, nv, ring), si, part, f < np ? COT_SPLIT : 1);
             if (lane == 0) {
                 bool last = true;
                 if (f < np) {
@@ -3983,6 +3987,15 @@ static size_t cells_smem(int maxv, int warps)
 #ifndef COT_SEG_MIN_N
 #define COT_SEG_MIN_N 4096
 #endif
+// Sites up to which weighted centroids and the render do with four launches: a
+// walk of the whole tree a cell, no bucket lists and no k_cells_heavy, and a
+// warp a cell in the integration.  The launches in a row are what these calls
+// wait for there (a render of 256 sites on 64^2 88 us against 105 with all of
+// them, of 2,304 on 128^2 126 against 145, of 4,096 on 256^2 240 against 243;
+// of a first point with many hidden cells at 4,096 sites 398 against 363).
+#ifndef COT_PIX_SEG_MIN_N
+#define COT_PIX_SEG_MIN_N 4096
+#endif
 // Sites from which the cells whose last ring stands take a few lanes each
 // (k_rings_cached, k_certify), and up to which k_certify takes 8 of them: its
 // two launches cost about what they save at 16,384 sites, and below 8 lanes
@@ -4039,11 +4052,12 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     const int lpc = (pixels || points || cells_per_warp < 2) ? 32 : (cells_per_warp == 2 ? 16 : 8);
     // the bucket walk's lists exist only on the path that runs it: every
     // other path walks in full
-    if (lpc != 32) a.blist = a.bcnt = nullptr;
+    const bool few = pixels && g.n <= COT_PIX_SEG_MIN_N;
+    if (lpc != 32 || few) a.blist = a.bcnt = nullptr;
     // the heavy integration list (ovf_list2, which only the 16- and 8-lane
     // paths use otherwise) on the two-kernel path
     a.hlist = lpc != 32 ? nullptr : a.ovf_list2;
-    if (lpc != 32) a.wlist = nullptr;
+    if (lpc != 32 || few) a.wlist = nullptr;
     if (lpc != 32) a.hsplit = nullptr;
     const int per_sm32 = g_blocks_per_sm32 > 0 ? g_blocks_per_sm32 : CELLS_MINB;
     const int per_sm16 = g_blocks_per_sm16 > 0 ? g_blocks_per_sm16 : CELLS_MINB;
@@ -4092,11 +4106,13 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
         // the cells whose walk overflowed, a block each (an empty list
         // returns at once)
         const size_t hsm = sizeof(FastScratch) + sizeof(HeavyShared);
-        if (a.keep_labels)
-            k_cells_heavy<true><<<2 * sms, 32 * HEAVY_WARPS, hsm, s>>>(g, a);
-        else
-            k_cells_heavy<false><<<2 * sms, 32 * HEAVY_WARPS, hsm, s>>>(g, a);
-        c.launches++;
+        if (a.wlist != nullptr) {
+            if (a.keep_labels)
+                k_cells_heavy<true><<<2 * sms, 32 * HEAVY_WARPS, hsm, s>>>(g, a);
+            else
+                k_cells_heavy<false><<<2 * sms, 32 * HEAVY_WARPS, hsm, s>>>(g, a);
+            c.launches++;
+        }
     } else if (lpc == 16) {
         launch_fast<16>(g, a, 0, blocks, s);
         launch_fast<32>(g, a, 1, sms, s);
@@ -4108,10 +4124,19 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     }
     if (pixels) {
         const int per = g_blocks_per_smp > 0 ? g_blocks_per_smp : PIX_MINB;
-        const int bp = std::min((g.n + CELLS_WPB - 1) / CELLS_WPB, sms * per);
-        k_integrate_pixels<PIX_MINB><<<bp, 32 * CELLS_WPB, PIX_WARP_SMEM * CELLS_WPB, s>>>(g, a);
+        // warps for the cells and for eight parts of each that can be split, as
+        // far as they are resident (a warp a cell left most of the GPU idle
+        // where few cells are all large: 1,024 sites on 1024^2 243 us of this
+        // kernel, now 166)
+        const long long split = std::min<long long>(g.n, (long long)g.nx * g.ny / (COT_SPLIT_PIX / 4));
+        const long long warps = (few ? g.n : (g.n + 3) / 4) + COT_SPLIT * split;
+        const int bp = (int)std::min<long long>((warps + CELLS_WPB - 1) / CELLS_WPB, (long long)sms * per);
+        if (few)
+            k_integrate_pixels<PIX_MINB, 32><<<bp, 32 * CELLS_WPB, PIX_WARP_SMEM * CELLS_WPB, s>>>(g, a);
+        else
+            k_integrate_pixels<PIX_MINB, 8><<<bp, 32 * CELLS_WPB, PIX_WARP_SMEM * CELLS_WPB, s>>>(g, a);
         c.launches++;
-    } else {
+    } else if (!a.rings_only) {
         const int per_smi = g_blocks_per_smi > 0 ? g_blocks_per_smi : 8;
         const int bi = std::min((g.n + CELLS_WPB - 1) / CELLS_WPB, sms * per_smi);
         if (a.hlist != nullptr && g.n > COT_SEG_MIN_N)
@@ -4168,7 +4193,8 @@ void configure_cells_kernels()
                                                       sm8) == cudaSuccess && nb > 0)
         g_blocks_per_sm8 = nb;
     const int smi = INT_WARP_SMEM * CELLS_WPB, smp = PIX_WARP_SMEM * CELLS_WPB;
-    cudaFuncSetAttribute(k_integrate_pixels<PIX_MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp);
+    cudaFuncSetAttribute(k_integrate_pixels<PIX_MINB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp);
+    cudaFuncSetAttribute(k_integrate_pixels<PIX_MINB, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp);
     cudaFuncSetAttribute(k_integrate<INT_MINB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi);
     cudaFuncSetAttribute(k_integrate<INT_MINB, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smi);
     cudaFuncSetAttribute(k_cells_first<FIRST_MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
@@ -4195,7 +4221,7 @@ void configure_cells_kernels()
         nb > 0)
         g_blocks_per_smi = nb;
     nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_integrate_pixels<PIX_MINB>, 32 * CELLS_WPB, smp) ==
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_integrate_pixels<PIX_MINB, 8>, 32 * CELLS_WPB, smp) ==
             cudaSuccess &&
         nb > 0)
         g_blocks_per_smp = nb;

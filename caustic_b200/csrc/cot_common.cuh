@@ -165,6 +165,7 @@ struct CellsArgs {
     double *ring_xy;       // optional fixed-stride ring dump (nullable)
     int *ring_lab;
     int ring_cap;
+    int rings_only;        // 1: no masses and objective (plain centroids alone)
     // Newton solve only (zero elsewhere): the mass Jacobian's rows
     int keep_labels;       // 1: the final ring's edge generators stay in lbuf
     double *hbig_val;      // rows of rings above COT_RCAP vertices, COT_HBIG_W entries a slot (nullable)

@@ -116,3 +116,27 @@ def test_pixel_parts_of_aligned_cells_far_from_the_origin(gpu, offset, width, k)
     want = np.repeat(np.repeat(nu.reshape(gy, gx) / nu.sum() / k ** 2, k, 0), k, 1)
     got = np.asarray(img).reshape(ny, nx)
     assert np.abs(got / want - 1.0).max() <= rel
+
+
+@pytest.mark.parametrize("gx,gy,nx,ny", [(1, 1, 20, 30), (3, 2, 7, 9), (64, 64, 100, 90), (241, 17, 300, 31), (9, 7, 900, 700)])
+def test_pixel_parts_at_the_sizes_where_the_form_changes(gpu, gx, gy, nx, ny):
+    """Weighted centroids and the render up to 4,096 sites, a warp a cell, and
+    just above, four cells a warp; cells that all go to eight warps."""
+    rng = np.random.default_rng(gx + nx)
+    xy = problems.jittered_grid(rng, gx, gy)
+    n = gx * gy
+    nu = rng.uniform(0.5, 1.5, n)
+    p = problems.SDOTProblem("form", xy, nu / nu.sum(), rng.uniform(0.1, 1.0, nx * ny), (nx, ny))
+    s = solver_for(p)
+    for w in (np.zeros(n), rng.normal(0.0, 1.0 / n, n)):  # the second hides some cells
+        c = O.cells(p.xy, w, O.proj_corner(p.xy, p.proj_domain))
+        oxy, oex = O.centers(c, p.picture, p.size, p.proj_domain, weighting=True)
+        for _ in range(2):  # without and with the cells of the call before
+            got, ex = s.centroids(w, weighted=True)
+            assert np.array_equal(ex, oex) and np.abs(got[ex] - oxy[ex]).max() < 1e-10
+        oxy, oex = O.centers(c, p.picture, p.size, p.proj_domain, weighting=False)
+        got, ex = s.centroids(w, weighted=False)
+        assert np.array_equal(ex, oex) and np.abs(got[ex] - oxy[ex]).max() < 1e-10
+        # the picture of the cells' masses: each cell's whole mass arrives
+        img = s.render(w)
+        assert abs(img.sum() - p.nu[ex].sum()) < 1e-10
