@@ -121,7 +121,11 @@ struct CotProblemDev {
 };
 
 #define COT_TMP(n) (8 + 3 * (size_t)(n))  // an evaluation's scalars, then three vectors
-#define COT_STAGE_N 4096                  // sites up to which an evaluation's host vectors go through pinned memory
+// Sites up to which an evaluation's host results come back through pinned
+// memory in one copy: an evaluation of 1,024 sites 83 us against 109 straight to
+// the caller's arrays, of 4,096 111 against 137, of 16,384 (with the limit there)
+// 141 against 178.  The limit is a handle's share of pinned memory, 96 KB.
+#define COT_STAGE_N 4096
 
 // Counters that one body of the trial graph adds per execution.
 struct BodyCounts {
@@ -150,7 +154,7 @@ struct cot_handle {
     cot::NewtonEvalStats *hN = nullptr;  // pinned copies of the Newton solve's trial statistics
     cot::PcgState *hP = nullptr;         // and of its inner solve's state
     unsigned char *hB = nullptr;         // pinned copy of the set-up's input statistics
-    double *hQ = nullptr;                // pinned vectors of small evaluations
+    double *hQ = nullptr;                // pinned results of small evaluations
     unsigned char *pinned = nullptr;     // the block that holds these five
     // the device-driven trial loop's graph, kept while the problem, its
     // buffers and the stream stay the same (instantiating it costs more than
@@ -678,19 +682,13 @@ static int need_points(cot_handle *h, const char *what)
 }
 
 // The weights of a query as a device vector in caller order: device arrays
-// are read in place, host arrays go to the staging vector (small ones through
-// pinned memory, which the caller's call does not wait for).
+// are read in place, host arrays go to the staging vector.
 static int query_weights(cot_handle *h, const double *w, int mem, const double **dev)
 {
     CotProblemDev &P = h->P;
     *dev = w;
     if (mem == COT_MEM_DEVICE) return COT_OK;
-    const double *src = w;
-    if (P.n <= COT_STAGE_N) {
-        std::memcpy(h->hQ, w, (size_t)P.n * sizeof(double));
-        src = h->hQ;
-    }
-    COT_CUDA_TRY(cudaMemcpyAsync(P.tmp, src, (size_t)P.n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    COT_CUDA_TRY(cudaMemcpyAsync(P.tmp, w, (size_t)P.n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     *dev = P.tmp;
     return COT_OK;
 }
