@@ -36,10 +36,6 @@ namespace cot {
 #define COT_REFINE_PASSES 3  // ring refinements before a walk that overflows scans every bucket
 #define COT_REFINE_ROUNDS 4  // point-location rounds of one refinement
 #define COT_DEFERRED (-3)    // ring size of a cell handed to k_cells_heavy
-#ifndef COT_DEFER_LEAVES
-#define COT_DEFER_LEAVES 12  // surviving leaf buckets above which a walk is handed to k_cells_heavy (25 cold iterations at
-                             // 4,096 sites with 24, 16, 12, 8: 5.33, 5.19, 5.01, 5.10 ms; at 65,536 sites 5.65, 5.56, 5.57, 5.55)
-#endif
 #ifndef COT_DEFER_PASS
 #define COT_DEFER_PASS 1  // refinement passes before a walk is handed to k_cells_heavy (1, 2, 3 measured 134.9, 134.8, 134.3 M cell-evals/s: 65,536 sites, 1024² target)
 #endif
@@ -2206,7 +2202,7 @@ __device__ __forceinline__ RegPoly cell_walk(const CotGeo &g, const CellsArgs &a
             // many surviving leaves: applied in bucket order, their sites
             // would cost a real clip nearly each; k_cells_heavy tests them
             // with a block and clips the deepest first
-            if (!brute && ncur > COT_DEFER_LEAVES && a.wlist != nullptr) {
+            if (!brute && ncur > a.defer && a.wlist != nullptr) {
                 if (lane < P.nv) {
                     a.rbuf[ring_at(i, lane)] = make_double2(P.x, P.y);
                     a.lbuf[ring_at(i, lane)] = P.l;
@@ -3980,6 +3976,19 @@ static size_t cells_smem(int maxv, int warps)
 #ifndef INT_MINB
 #define INT_MINB 6  // k_integrate: 80 registers (8 blocks: 2043 us at 262,144 sites against 2072, but 724 against 718 at 65,536)
 #endif
+// Surviving leaf buckets above which a walk is handed to k_cells_heavy.  A block
+// a cell is done with a long walk sooner than a warp, but starts when the walk is
+// over and holds eight warps.  Few sites: all walks run at once, and the two ends
+// one after the other cost more than one long walk (no limit but the frontier's).
+// Many: the blocks fill the GPU, the more leaves a warp takes the better.
+// Cold solves, ms, with 12, 16, 24, 48, 96 leaves: 20 to 100 iterations of 4,096
+// sites 16.8 17.1 17.5 17.5 16.0, 6,400 8.0 8.2 8.4 8.6 7.5, 10,000 8.9 8.9 9.2 9.7
+// 8.8 and 8.7 8.8 9.1 9.7 9.3, 14,400 10.0 9.8 10.0 10.6 10.5, 25,600 14.9 14.2 13.9
+// 14.6 14.7, 40,000 19.8 18.6 17.7 18.2 18.5, 65,536 39.3 36.5 33.6 33.1 33.6, 90,000
+// 25.4 23.0 21.1 20.5 20.7, 262,144 69.9 56.7 45.9 39.6 38.2.
+#ifndef COT_DEFER
+#define COT_DEFER(n) ((n) <= 8192 ? COT_FRMAX : std::min(std::max((n) / 1800, 20), COT_FRMAX))
+#endif
 // sites above which four cells share a warp of the integration: at 4,096 a
 // warp a cell still fits the GPU at once (148 x 32 warps) and each cell is
 // done sooner (two evaluations at 1,024 sites 325 against 334 us, 25
@@ -4044,6 +4053,7 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     int upper = 0;  // nodes of levels 1..lmax
     for (int L = 1; L <= lmax; L++) upper += g.lev_w[L] * g.lev_h[L];
     const int sms = num_sms > 0 ? num_sms : 148;
+    a.defer = COT_DEFER(g.n);
     // what needs each pixel's part of a cell: weighted centroids (the
     // reference leaves tiny parts out) and the render; plain centroids and
     // solid angles need the rings alone

@@ -159,6 +159,7 @@ struct CellsArgs {
     double splat_scale;    // gray_multiple of the render
     double2 *rbuf;         // ring vertices of the solve's path, at ring_at(cell, vertex)
     int *lbuf;             // their edge generators between the ring kernels
+    int defer;             // leaves of a walk from which k_cells_heavy takes it (launch_eval sets it)
     int *flist;            // cells that the thread-per-cell ring kernels leave to the others
                            // (two-kernel path only; nullable)
     int *cstate;           // per cell: ring size (+ cached flag) after phase 1, -1 = finished
