@@ -52,8 +52,9 @@ struct cot_handle;
 
 struct CotProblemDev {
     // the groups' blocks: sites and pixels, bucket grid, and what the first
-    // call that needs it makes (and keeps): the history, the centroids, the
-    // Anderson solve, the Newton solve, the render
+    // call that needs it makes (and keeps): a history, the centroids, the
+    // Anderson solve (up to COT_EARLY_N sites with the sites), the Newton solve,
+    // the render
     void *b_sites = nullptr, *b_grid = nullptr, *b_hist = nullptr, *b_points = nullptr, *b_aa = nullptr;
     void *b_newton = nullptr, *b_image = nullptr;
     int n = 0;
@@ -120,6 +121,13 @@ struct CotProblemDev {
     unsigned int *nticket = nullptr;
 };
 
+// Sites up to which a handle's problem has room for a history of this many pairs,
+// the centroids and the Anderson vectors from the start: 282 bytes a site in the
+// block that is made anyway (36 MB at the limit).  The first solve at 65,536 sites
+// takes 0.97 ms instead of 1.27, the first centroids 0.62 instead of 0.97.  Above,
+// the first call that needs them makes them.
+#define COT_EARLY_N 131072
+#define COT_EARLY_HIST 10
 #define COT_TMP(n) (8 + 3 * (size_t)(n))  // an evaluation's scalars, then three vectors
 // Sites up to which an evaluation's host results come back through pinned
 // memory in one copy: an evaluation of 1,024 sites 83 us against 109 straight to
@@ -437,14 +445,80 @@ extern "C" int cot_last_error(cot_handle *h, char *buf, size_t n)
 }
 
 
+// What the solves and the centroids need besides: one problem's history of m
+// pairs, its centroids and exist flags (sorted and in caller order), the
+// Anderson solve's vectors.  Sized for the buffers' capacity: a later problem
+// that fits them reuses these.
+static void add_history(Carve &c, CotProblemDev &P, int m)
+{
+    c.add(&P.Sv, (size_t)m * P.cap_n);
+    c.add(&P.Yv, (size_t)m * P.cap_n);
+}
+static void add_points(Carve &c, CotProblemDev &P)
+{
+    c.add(&P.pcen, 4 * P.cap_n);
+    c.add(&P.pex, 2 * P.cap_n);
+}
+static void add_aa(Carve &c, CotProblemDev &P)
+{
+    const size_t N = P.cap_n;
+    c.add(&P.aa_src, 2 * N);
+    c.add(&P.aa_inl, 3 * N);
+    c.add(&P.aa_insl, 3 * N);
+    c.add(&P.aa_hgt, N);
+    c.add(&P.aa_lam, N);
+    c.add(&P.aa_energy, N);
+    c.add(&P.aa_row, COT_MAX_HIST);
+    c.add(&P.aa_coef, COT_MAX_HIST);
+    c.add(&P.aa_step, 1);
+}
+
+static int need_history(cot_handle *h, int m)
+{
+    CotProblemDev &P = h->P;
+    if (P.hist_alloc >= m) return COT_OK;
+    // the shorter one goes first: both at once may not fit
+    if (P.b_hist) cudaFree(P.b_hist);
+    P.b_hist = nullptr;
+    P.Sv = P.Yv = nullptr;
+    P.hist_alloc = 0;
+    Carve c;
+    add_history(c, P, m);
+    const cudaError_t e = c.alloc(&P.b_hist);
+    if (e != cudaSuccess) return fail(h, COT_ENOMEM, "solve: history allocation", cudaGetErrorString(e));
+    P.hist_alloc = m;
+    P.gen = ++g_problem_gen;  // a graph that captured the old history buffers is stale
+    return COT_OK;
+}
+
+static int need_points(cot_handle *h, const char *what)
+{
+    CotProblemDev &P = h->P;
+    if (P.pcen) return COT_OK;
+    Carve c;
+    add_points(c, P);
+    const cudaError_t e = c.alloc(&P.b_points);
+    return e == cudaSuccess ? COT_OK : fail(h, COT_ENOMEM, what, cudaGetErrorString(e));
+}
+
+static int need_aa(cot_handle *h)
+{
+    CotProblemDev &P = h->P;
+    if (P.aa_src) return COT_OK;
+    Carve c;
+    add_aa(c, P);
+    const cudaError_t e = c.alloc(&P.b_aa);
+    return e == cudaSuccess ? COT_OK : fail(h, COT_ENOMEM, "cot_solve_aarl: device allocation", cudaGetErrorString(e));
+}
+
 // Build the device problem (the kernels are in cot_build.cu): input checks
 // and sums, the bucket grid over the sites' box, the stable sort of the
 // sites by bucket (then caller index), the static bound tree, and the
 // density scaled to sum(nu) per unit area.  The host reads only the box and
 // the sums.  Inputs are host arrays (copied in first) or device arrays
-// (read in place) per mem.
+// (read in place) per mem.  kept: the handle's own problem, not one call's.
 static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, const double *nu_in,
-                         const double *dens_in, int n, int nx, int ny, const double pd[4], int mem)
+                         const double *dens_in, int n, int nx, int ny, const double pd[4], int mem, bool kept = true)
 {
     cudaStream_t s = h->stream;
     const size_t npix = (size_t)nx * ny;
@@ -490,7 +564,13 @@ static int build_problem(cot_handle *h, CotProblemDev &P, const double *xy_in, c
         c.add(&P.bpart, build_partials_doubles());
         c.add(&P.bticket, 2);
         c.add(&P.bstat, 256);
+        if (kept && N <= COT_EARLY_N) {
+            add_history(c, P, COT_EARLY_HIST);
+            add_points(c, P);
+            add_aa(c, P);
+        }
         cudaError_t e = c.alloc(&P.b_sites);
+        if (e == cudaSuccess && P.Sv) P.hist_alloc = COT_EARLY_HIST;
         if (e == cudaSuccess) e = cudaMemsetAsync(P.bticket, 0, 2 * sizeof(unsigned int), s);
         if (e == cudaSuccess) e = cudaMemsetAsync(P.hticket, 0, COT_HSPLIT_CAP * sizeof(unsigned int), s);
         if (e != cudaSuccess) {
@@ -667,18 +747,6 @@ static int need_hperm(cot_handle *h, CotProblemDev &P)
     COT_CUDA_TRY(cudaStreamSynchronize(h->stream));
     P.hperm_valid = true;
     return COT_OK;
-}
-
-// Room for the centroids and exist flags.
-static int need_points(cot_handle *h, const char *what)
-{
-    CotProblemDev &P = h->P;
-    if (P.b_points) return COT_OK;
-    Carve c;
-    c.add(&P.pcen, 4 * P.cap_n);
-    c.add(&P.pex, 2 * P.cap_n);
-    const cudaError_t e = c.alloc(&P.b_points);
-    return e == cudaSuccess ? COT_OK : fail(h, COT_ENOMEM, what, cudaGetErrorString(e));
 }
 
 // The weights of a query as a device vector in caller order: device arrays
@@ -929,7 +997,7 @@ static int source_masses_impl(cot_handle *h, const double *points_xy, int n, con
     // unweighted cells inside the sample domain, one "pixel" of unit density
     std::vector<double> one(n, 1.0), dens(1, 1.0);
     CotProblemDev Q;
-    int r = build_problem(h, Q, points_xy, one.data(), dens.data(), n, 1, 1, sd, COT_MEM_HOST);
+    int r = build_problem(h, Q, points_xy, one.data(), dens.data(), n, 1, 1, sd, COT_MEM_HOST, false);
     if (r != COT_OK) free_problem(Q);
     if (r != COT_OK) return r;
     cudaStream_t s = h->stream;
@@ -1131,47 +1199,6 @@ static int build_trial_graph(cot_handle *h, double *tptr, cudaGraphExec_t *exec,
         return COT_ECUDA;
     }
     return COT_OK;
-}
-
-// Room for a history of m pairs.
-static int need_history(cot_handle *h, int m)
-{
-    CotProblemDev &P = h->P;
-    if (P.hist_alloc >= m) return COT_OK;
-    // the shorter one goes first: both at once may not fit
-    if (P.b_hist) cudaFree(P.b_hist);
-    P.b_hist = nullptr;
-    P.Sv = P.Yv = nullptr;
-    P.hist_alloc = 0;
-    // sized for the buffers' capacity: a later problem that fits them reuses these
-    Carve c;
-    c.add(&P.Sv, (size_t)m * P.cap_n);
-    c.add(&P.Yv, (size_t)m * P.cap_n);
-    const cudaError_t e = c.alloc(&P.b_hist);
-    if (e != cudaSuccess) return fail(h, COT_ENOMEM, "solve: history allocation", cudaGetErrorString(e));
-    P.hist_alloc = m;
-    P.gen = ++g_problem_gen;  // a graph that captured the old history buffers is stale
-    return COT_OK;
-}
-
-// Room for the Anderson solve's vectors.
-static int need_aa(cot_handle *h)
-{
-    CotProblemDev &P = h->P;
-    if (P.b_aa) return COT_OK;
-    const size_t N = P.cap_n;
-    Carve c;
-    c.add(&P.aa_src, 2 * N);
-    c.add(&P.aa_inl, 3 * N);
-    c.add(&P.aa_insl, 3 * N);
-    c.add(&P.aa_hgt, N);
-    c.add(&P.aa_lam, N);
-    c.add(&P.aa_energy, N);
-    c.add(&P.aa_row, COT_MAX_HIST);
-    c.add(&P.aa_coef, COT_MAX_HIST);
-    c.add(&P.aa_step, 1);
-    const cudaError_t e = c.alloc(&P.b_aa);
-    return e == cudaSuccess ? COT_OK : fail(h, COT_ENOMEM, "cot_solve_aarl: device allocation", cudaGetErrorString(e));
 }
 
 // History buffers and the device control block of a solve from the weights

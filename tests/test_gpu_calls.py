@@ -75,3 +75,16 @@ def test_memory_is_taken_by_the_calls_that_need_it(gpu):
         s.solve(np.zeros(p.n), mode=capi.SOLVE_WOLFE, tol=1e-12, history=m, max_iter=1)
         hist = used() - n0 - base - pts
         assert 16 * m * p.n <= hist <= 16 * m * p.n + 16 * mb, (m, hist / p.n)
+
+
+def test_a_history_longer_than_the_first_room(gpu):
+    """Small problems have room for ten pairs from the start; a longer history
+    moves, a shorter one after it stays, and results do not change."""
+    p = problems.make(1, g=24, res=96)
+    runs = []
+    for order in ((10, 24, 10, 3), (3, 10, 24, 10)):
+        s = solver_for(p)
+        runs.append({m: s.solve(np.zeros(p.n), mode=capi.SOLVE_WOLFE, history=m, max_iter=40, tol=1e-9)[0]
+                     for m in order})
+    for m in (3, 10, 24):
+        assert np.array_equal(runs[0][m], runs[1][m])
