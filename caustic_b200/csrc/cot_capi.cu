@@ -436,6 +436,19 @@ extern "C" int cot_eval_counters(cot_handle *h, int *out4)
     return COT_OK;
 }
 
+extern "C" int cot_ring_counters(cot_handle *h, int *out2)
+{
+    if (!h || !out2) return COT_EINVAL;
+    if (!h->has_problem) return fail(h, COT_ENOPROBLEM, "cot_ring_counters: no problem set", nullptr);
+    COT_CUDA_TRY(cudaSetDevice(h->device));
+    int c[2];
+    COT_CUDA_TRY(cudaMemcpyAsync(c, h->P.ovf_count + 14, sizeof c, cudaMemcpyDeviceToHost, h->stream));
+    COT_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    out2[0] = c[0];
+    out2[1] = c[1];
+    return COT_OK;
+}
+
 extern "C" int cot_last_error(cot_handle *h, char *buf, size_t n)
 {
     const std::string &m = h ? h->err : g_create_err;

@@ -362,6 +362,15 @@ COT_API int cot_get_kernel_stats(cot_handle *h, cot_kernel_stats *out, int reset
  * warps.  Waits for the handle's stream; valid until the next evaluation. */
 COT_API int cot_eval_counters(cot_handle *h, int *out4);
 
+/* Which cells the last evaluation rebuilt and walked with a warp each, instead
+ * of a few lanes (diagnostics; no counterpart in the reference; problems of
+ * 16,384 sites and more, with the default cells_per_warp -- 0 and 0 elsewhere,
+ * where every cell has a warp or its share of one): out[0] cells without an
+ * ordered ring of at most 8 edges from the evaluation before, or whose ring did
+ * not stand, out[1] cells whose certificate was left to the walk, those among
+ * them.  Waits for the handle's stream; valid until the next evaluation. */
+COT_API int cot_ring_counters(cot_handle *h, int *out2);
+
 /* Message of the last failure on this handle (or of the last failed
  * cot_create when h is NULL). */
 COT_API int cot_last_error(cot_handle *h, char *buf, size_t n);

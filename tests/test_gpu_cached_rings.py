@@ -82,3 +82,33 @@ def test_clustered_sites_have_the_bits_of_a_cold_evaluation(gpu, n, width):
         f0, mu0, g0, fc0 = fresh.eval(w)
         assert np.array_equal(mu, mu0) and np.array_equal(fc, fc0) and f == f0, amp
         fresh.close()
+
+
+@pytest.mark.parametrize("g", [129, 210])  # 8 lanes a cell, and 4
+def test_most_cells_of_a_warm_evaluation_take_the_short_path(gpu, g):
+    """The bits are the warp kernels' whichever cells they take: that the short
+    path takes most of them where little moves, leaves those that move, and
+    none in a domain whose squares vanish, shows in the counters alone."""
+    p = problems.make(4, g=g, res=200)
+    n = p.n
+    rng = np.random.default_rng(g)
+    s = solver_for(p)
+    w = rng.normal(0.0, 0.05 / n, n)
+    left = {}
+    for amp in (None, 0.0, 0.01, 3.0):
+        w = w + (0.0 if amp is None else rng.normal(0.0, amp / n, n))
+        s.eval(w)
+        c = s.ring_counters()
+        assert c["rings_by_warp"] <= n and c["walks_by_warp"] <= n
+        left[amp] = c
+    assert left[None]["rings_by_warp"] == n  # no ring yet
+    assert left[0.0]["rings_by_warp"] + left[0.0]["walks_by_warp"] < n // 4, left
+    assert left[0.01]["rings_by_warp"] + left[0.01]["walks_by_warp"] < n // 2, left
+    assert left[3.0]["rings_by_warp"] > n // 4, left
+    k = 2.0 ** -90
+    small = solver_for(problems.SDOTProblem("small", p.xy * k, p.nu * k * k, p.picture, p.size,
+                                            np.asarray(p.proj_domain) * k))
+    for _ in range(2):
+        small.eval(np.zeros(n))
+    c = small.ring_counters()
+    assert c["rings_by_warp"] < n // 2 and c["walks_by_warp"] == n, c
