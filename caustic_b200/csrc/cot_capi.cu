@@ -1732,7 +1732,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
             }
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
-            }
+        }
         return rr;
     };
     if ((r = report_start(COT_PHASE_PREPASS)) != COT_OK) return r;
@@ -1747,7 +1747,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
             }
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
-                return r;
+            return r;
         }
         evals += pre.evals;
         // 3. nu again from the centroids at the pre-pass result
@@ -1775,7 +1775,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
         for (int i = 0; i < cnt; i++)
             for (int j = 0; j < cnt; j++) As[(size_t)i * cnt + j] = A[(size_t)i * M + j] + (i == j ? 1e-10 : 0.0);
         if (!ldlt_solve_ones(As, cnt, a)) {
-                return fail(h, COT_ENOTCONV, "cot_solve_aarl: singular Anderson system", nullptr);
+            return fail(h, COT_ENOTCONV, "cot_solve_aarl: singular Anderson system", nullptr);
         }
         double sa = 0;
         for (double v : a) sa += v;
@@ -1833,7 +1833,7 @@ extern "C" int cot_solve_aarl(cot_handle *h, double *w_inout, const cot_aarl_inp
                 }
                 cudaEventDestroy(e0);
                 cudaEventDestroy(e1);
-                        return r;
+                return r;
             }
         }
         if (conv_now) {

@@ -1985,12 +1985,10 @@ __device__ __noinline__ RegPoly scan_all_buckets(const CotGeo &g, const double *
 
 // One cell, worked by one segment of LPC lanes (lane = index in the segment),
 // in three phases: cell_first (the first candidates), cell_walk (the
-// certificate over the bound tree) and cell_finish (integrals or the ring
-// buffer, the next evaluation's cache, the per-cell outputs).  A ring that
+// certificate over the bound tree) and cell_finish (the ring buffer and the
+// next evaluation's cache).  A ring that
 // outgrows LPC vertices has nv = -1 from then on and goes to olist / ocount
-// for the next pass.  EXACT = true: the per-pixel path that also yields
-// centroids (with the reference's 1e-10 piece rule) and the render, a whole
-// warp per cell; false: the solver's hot path (masses and objective only).
+// for the next pass.
 //
 // Phase 1: the domain rectangle clipped by the last evaluation's ring (or
 // neighbours), else by the 3x3 buckets around the site.  cached: the cell
@@ -2263,8 +2261,8 @@ __device__ __forceinline__ RegPoly cell_walk(const CotGeo &g, const CellsArgs &a
     return P;
 }
 
-// Phase 3: overflow hand-off, or the ring's integrals (EXACT) / the ring
-// buffer (solve path), the next evaluation's cache and the per-cell outputs.
+// Phase 3: overflow hand-off, or the ring to the ring buffer and the next
+// evaluation's cache.
 template <int LPC, bool KEEP = false>
 __device__ __forceinline__ void cell_finish(const CotGeo &g, const CellsArgs &a, const int i, const double2 si,
                                             const double wi, RegPoly P, FastScratch &S, int *olist, int *ocount)
@@ -2472,7 +2470,6 @@ __global__ void __launch_bounds__(128, MINB) k_cells_first(const __grid_constant
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) k_bucket_walk(CotGeo g, CellsArgs a)
 {
-    constexpr int LPC = 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FastScratch &S = reinterpret_cast<FastScratch *>(smem_raw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -2592,9 +2589,9 @@ __global__ void __launch_bounds__(128, MINB) k_bucket_walk(CotGeo g, CellsArgs a
 // k_cells_first and k_cells_walk.  The lines, vertices and final tests are
 // those of the warp kernels in the same explicitly rounded forms, so a cell
 // has the same bits whichever took it.
-// At 262,144 sites (us): k_cells_first 217 -> 43 + 17 for the cells left to
-// it, k_cells_walk 423 -> 143 + 43, latency of dependent loads and double
-// precision chains the bound (360 warp instructions a cell, 60 % issued).
+// At 262,144 sites (us, with the tree's levels in the first): k_cells_first
+// 217 + 33 -> 64 + 20 for the cells left to it, k_cells_walk 423 -> 148 + 50;
+// latency of dependent loads and double precision chains the bound.
 #define FAST_THREADS 128
 #define FAST_NV 8      // largest ring of these kernels
 #define FAST_LEFT 12   // leaves whose sites k_certify looks through (3.6 on average)
@@ -3861,7 +3858,7 @@ __global__ void __launch_bounds__(128, MINB) k_cells(CotGeo g, CellsArgs a, int 
                 a.ring_lab[(size_t)i * a.ring_cap + k] = P.L[k];
             }
         }
-        if (a.solid != nullptr && lane == 0) 
+        if (a.solid != nullptr && lane == 0)
             a.solid[i] = nv >= 3 ? solid_angle_of([&](int k) { return make_double2(P.X[k], P.Y[k]); }, nv, si, a.solid_z,
                                                   a.solid_light)
                                  : 0.0;
@@ -4018,7 +4015,7 @@ static size_t cells_smem(int maxv, int warps)
 #ifndef COT_FAST_G8_N
 #define COT_FAST_G8_N 40000
 #endif
-static int g_blocks_per_sm32 = 0, g_blocks_per_sm16 = 0, g_blocks_per_sm8 = 0, g_blocks_per_smi = 0;
+static int g_blocks_per_sm16 = 0, g_blocks_per_sm8 = 0, g_blocks_per_smi = 0;
 static int g_blocks_per_smf = 0, g_blocks_per_smw = 0, g_blocks_per_smb = 0, g_blocks_per_smp = 0;
 
 template <int LPC>
@@ -4069,12 +4066,11 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     a.hlist = lpc != 32 ? nullptr : a.ovf_list2;
     if (lpc != 32 || few) a.wlist = nullptr;
     if (lpc != 32) a.hsplit = nullptr;
-    const int per_sm32 = g_blocks_per_sm32 > 0 ? g_blocks_per_sm32 : CELLS_MINB;
     const int per_sm16 = g_blocks_per_sm16 > 0 ? g_blocks_per_sm16 : CELLS_MINB;
     const int per_sm8 = g_blocks_per_sm8 > 0 ? g_blocks_per_sm8 : 1;
     const int cells_per_block = CELLS_WPB * (32 / lpc);
     const int want = (g.n + cells_per_block - 1) / cells_per_block;
-    const int blocks = std::min(want, sms * (lpc == 32 ? per_sm32 : (lpc == 16 ? per_sm16 : per_sm8)));
+    const int blocks = std::min(want, sms * (lpc == 16 ? per_sm16 : per_sm8));  // of launch_fast
     bool timed = c.profile && c.ev != nullptr && c.ev_used + 2 <= c.ev_cap;
     if (timed) cudaEventRecord(c.ev[c.ev_used], s);
     if (lpc != 32 && upper > 0) {
@@ -4191,10 +4187,6 @@ void configure_cells_kernels()
     cudaFuncSetAttribute(k_cells_fast<CELLS_MINB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm8);
     cudaFuncSetAttribute(k_cells<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cells_smem(256, 1));
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, 32>, 32 * CELLS_WPB,
-                                                      sm32) == cudaSuccess && nb > 0)
-        g_blocks_per_sm32 = nb;
-    nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cells_fast<CELLS_MINB, 16>, 32 * CELLS_WPB,
                                                       sm16) == cudaSuccess && nb > 0)
         g_blocks_per_sm16 = nb;

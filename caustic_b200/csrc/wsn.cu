@@ -31,7 +31,7 @@ using bf16 = __nv_bfloat16;
 // ---------------------------------------------------------------------------
 // GEMM: D[M,N] (fp32, row-major) = alpha * A[M,K] * B[K,N] + beta * D
 // ---------------------------------------------------------------------------
-// One GEMM configuration per operand layout: 128x128x64 tiles on one SM,
+// One GEMM configuration per operand layout: MT x NT x 64 tiles on one SM,
 // fp32 accumulators in tensor memory, fp32 output.
 #define WS_GEMM_CONFIG(NAME, LA, LB, MT, NT)                                                                        \
     namespace NAME {                                                                                                \
@@ -83,7 +83,7 @@ WS_GEMM_CONFIG(GemmCR, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor, 
 // of rows to add up.  Its rows are one chain of sums in the tensor memory, in
 // order (sharing them out would round elsewhere), so more and lighter tiles
 // are what shortens it.
-WS_GEMM_CONFIG(GemmCR32, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor, 64, 64)
+WS_GEMM_CONFIG(GemmCR64, cutlass::layout::ColumnMajor, cutlass::layout::RowMajor, 64, 64)
 // A[M,K], B[K,N] both row-major         (input gradient: dcols = dZ W)
 WS_GEMM_CONFIG(GemmRR, cutlass::layout::RowMajor, cutlass::layout::RowMajor, 128, 128)
 
@@ -659,7 +659,7 @@ WS_API int ws_gemm(int layout, int M, int N, int K, const void *A, const void *B
     case WS_GEMM_RC: return GemmRC::run(M, N, K, A, B, D, alpha, beta, workspace, workspace_bytes, s);
     case WS_GEMM_CR:
         if (M % 8 != 0 || N % 8 != 0) return WS_EINVAL;
-        if (narrow_cr(M, N)) return GemmCR32::run(M, N, K, A, B, D, alpha, beta, workspace, workspace_bytes, s);
+        if (narrow_cr(M, N)) return GemmCR64::run(M, N, K, A, B, D, alpha, beta, workspace, workspace_bytes, s);
         return GemmCR::run(M, N, K, A, B, D, alpha, beta, workspace, workspace_bytes, s);
     case WS_GEMM_RR:
         if (N % 8 != 0) return WS_EINVAL;
@@ -672,7 +672,7 @@ WS_API size_t ws_gemm_workspace(int layout, int M, int N, int K)
 {
     switch (layout) {
     case WS_GEMM_RC: return GemmRC::workspace(M, N, K);
-    case WS_GEMM_CR: return narrow_cr(M, N) ? GemmCR32::workspace(M, N, K) : GemmCR::workspace(M, N, K);
+    case WS_GEMM_CR: return narrow_cr(M, N) ? GemmCR64::workspace(M, N, K) : GemmCR::workspace(M, N, K);
     case WS_GEMM_RR: return GemmRR::workspace(M, N, K);
     default: return 0;
     }
