@@ -1569,8 +1569,11 @@ __device__ __forceinline__ void warp_sort(double &key, int &idx, int lane)
 // lane first tests its own candidate against the whole ring (snapshot in
 // shared memory); only candidates that cut are then applied one by one with a
 // register clip (one that no longer cuts after an earlier clip is a no-op).
-// `nearest` applies the cutting ones in order of distance from the site.
-template <int LPC>
+// `nearest` applies the cutting ones in order of distance from the site.  DEEP:
+// many that cut go deepest first; not for the last evaluation's neighbours, which
+// nearly all remain edges (40 cold iterations at 65,536 sites 21.8 -> 21.1 ms
+// without).
+template <int LPC, bool DEEP = true>
 __device__ __forceinline__ RegPoly apply_chunk(RegPoly P, int jl, const double2 *__restrict__ sxy, double2 si, double wi,
                                             const double *__restrict__ wt, int lane, FastScratch &S, bool nearest)
 {
@@ -1595,7 +1598,7 @@ __device__ __forceinline__ RegPoly apply_chunk(RegPoly P, int jl, const double2 
     PSTAT_ADD(4, ntested);
 #endif
     if (have == 0u) return P;
-    if constexpr (LPC == 32) {
+    if constexpr (LPC == 32 && DEEP) {
         // many that cut: the one whose line goes deepest into the ring next,
         // and the others tested again on what it leaves.  A clip is a chain
         // of some 500 cycles whether or not it still cuts; the deepest first
@@ -1793,7 +1796,7 @@ __device__ __forceinline__ RegPoly ring_from_cache(int lab, int m, const double2
 
 // Sites of `cnt[k]` consecutive ranges starting at `st[k]` (k = lane, up to
 // LPC ranges), applied in chunks of LPC.  inc = inclusive scan of cnt.
-template <int LPC>
+template <int LPC, bool DEEP = true>
 __device__ __forceinline__ RegPoly apply_ranges(RegPoly P, int st, int cnt, int inc, int self, const double2 *__restrict__ sxy,
                                              double2 si, double wi, const double *__restrict__ wt, int lane,
                                              FastScratch &S, bool nearest)
@@ -1814,7 +1817,7 @@ __device__ __forceinline__ RegPoly apply_ranges(RegPoly P, int st, int cnt, int 
         const int ck = W.shfl(cnt, k & (LPC - 1));
         int j = (t < tot) ? sk + (t - (ik - ck)) : -1;
         if (j == self) j = -1;
-        P = apply_chunk<LPC>(P, j, sxy, si, wi, wt, lane, S, nearest);
+        P = apply_chunk<LPC, DEEP>(P, j, sxy, si, wi, wt, lane, S, nearest);
         if (P.nv < 0) return P;
     }
     return P;
@@ -1837,7 +1840,7 @@ __device__ __noinline__ RegPoly apply_chunk_cold(RegPoly P, int jl, const double
                                                  double wi, const double *__restrict__ wt, int lane, FastScratch &S,
                                                  bool nearest)
 {
-    return apply_chunk<LPC>(P, jl, sxy, si, wi, wt, lane, S, nearest);
+    return apply_chunk<LPC, false>(P, jl, sxy, si, wi, wt, lane, S, nearest);
 }
 
 // Upper bound of P_j(x) = x.s_j - phi_j over the sites of a tree node at the
