@@ -3986,8 +3986,12 @@ static size_t cells_smem(int maxv, int warps)
 // 8.8 and 8.7 8.8 9.1 9.7 9.3, 14,400 10.0 9.8 10.0 10.6 10.5, 25,600 14.9 14.2 13.9
 // 14.6 14.7, 40,000 19.8 18.6 17.7 18.2 18.5, 65,536 39.3 36.5 33.6 33.1 33.6, 90,000
 // 25.4 23.0 21.1 20.5 20.7, 262,144 69.9 56.7 45.9 39.6 38.2.
+// A Newton solve's evaluations (newton) of few sites have a handful of long walks
+// each, which twelve leaves part best: the warm pipeline of 64 problems of 1,024 to
+// 32,768 sites 19.0 solves a second, 18.5 without.
 #ifndef COT_DEFER
-#define COT_DEFER(n) ((n) <= 8192 ? COT_FRMAX : std::min(std::max((n) / 1800, 20), COT_FRMAX))
+#define COT_DEFER(n, newton) \
+    ((n) <= 8192 ? ((newton) ? 12 : COT_FRMAX) : std::min(std::max((n) / 1800, 20), COT_FRMAX))
 #endif
 // sites above which four cells share a warp of the integration: at 4,096 a
 // warp a cell still fits the GPU at once (148 x 32 warps) and each cell is
@@ -4053,7 +4057,7 @@ void launch_eval(const CotGeo &g, const CellsArgs &args, int cells_per_warp, int
     int upper = 0;  // nodes of levels 1..lmax
     for (int L = 1; L <= lmax; L++) upper += g.lev_w[L] * g.lev_h[L];
     const int sms = num_sms > 0 ? num_sms : 148;
-    a.defer = COT_DEFER(g.n);
+    a.defer = COT_DEFER(g.n, a.keep_labels);
     // what needs each pixel's part of a cell: weighted centroids (the
     // reference leaves tiny parts out) and the render; plain centroids and
     // solid angles need the rings alone
