@@ -89,21 +89,23 @@ def peaks():
 
 
 def committed_figure(key):
-    """A per-launch figure of the cell kernels from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "k_cells_config2.md")
-    try:
-        with open(path) as f:
-            for line in f:
-                if line.strip().startswith(key + ":"):
-                    return float(line.split(":", 1)[1].strip().split()[0])
-    except Exception:
-        pass
+    """A figure of the cell kernels from the committed ncu summaries: the
+    present kernels' (per evaluation), else those before them (per launch)."""
+    for name in ("evaluation_kernels.md", "k_cells_config2.md"):
+        try:
+            with open(os.path.join(ROOT, "profiles", name)) as f:
+                for line in f:
+                    if line.strip().startswith(key + ":"):
+                        return float(line.split(":", 1)[1].strip().split()[0])
+        except Exception:
+            pass
     return None
 
 
 def committed_traffic():
-    """Per-launch DRAM bytes of the cell kernels from the committed ncu summary."""
-    return committed_figure("traffic_bytes_per_launch")
+    """DRAM bytes of the cell kernels of an evaluation, mean of the cold solve,
+    from the committed ncu summary."""
+    return committed_figure("traffic_bytes_per_evaluation")
 
 
 class Clocks:
@@ -478,7 +480,7 @@ def run_ours(args):
     traffic = committed_traffic()
     roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
             "frac": (achieved / hbm) if achieved else None, "traffic": traffic,
-            "kernel": "k_cells_first + k_bucket_walk + k_cells_walk + k_cells_heavy + k_integrate (power-cell rings, the bucket lists, their certificate, the overflowed certificates a block each, their integration; timed together)",
+            "kernel": "k_rings_cached + k_cells_first + k_bucket_walk + k_certify + k_cells_walk + k_cells_heavy + k_integrate (power-cell rings, the bucket lists, their certificate, the overflowed certificates a block each, their integration; timed together)",
             "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms, "launches": kp["cell_launches"],
             "timing": "CUDA events around each launch, one host-driven solve of the same workload",
             "peak_kind": f"{peak_kind} hbm_gbs (burst copy)"}
@@ -543,7 +545,7 @@ def run_ours(args):
                 "gpu_launches": ks["launches"]}
         # the bound that does hold: warp-instruction issue (4 schedulers per
         # SM, one warp instruction per cycle each, at the sampled SM clock)
-        insts = committed_figure("warp_instructions_per_launch")
+        insts = committed_figure("warp_instructions_per_evaluation")
         ck = line["clocks"]
         mhz = ck.get("sm_mhz") or ck.get("sm_max_mhz") or 1965.0
         sms = torch.cuda.get_device_properties(local).multi_processor_count
@@ -553,7 +555,7 @@ def run_ours(args):
             line["roofline_issue"] = {"bound": "issue", "achieved": ach, "peak": issue_peak, "unit": "warp-inst/s",
                                       "frac": ach / issue_peak, "insts_per_launch": insts,
                                       "peak_kind": f"{sms} SMs x 4 schedulers x 1 warp-inst/cycle at {mhz:.0f} MHz",
-                                      "insts_source": "smsp__inst_executed.sum, committed ncu summary"}
+                                      "insts_source": "smsp__inst_executed.sum, mean of the cold solve's evaluations, committed ncu summary"}
         if world == 1 and not args.no_warm_start:
             line["warm_start"] = warm_start_arms(args, p, tot_ms / args.steps,
                                                  e2e["ms_per_step"] if e2e else None, local)
