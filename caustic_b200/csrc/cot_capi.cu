@@ -1541,7 +1541,7 @@ extern "C" int cot_solve_batch(cot_handle *const *hs_in, int count, double *cons
     }
     // the handles' graph, unless the last batch was theirs: building it for 12
     // instances of 1,024 to 8,100 sites takes 4 ms, their 12 iterations 7.  (Each
-    // handle's own trial graph on its own stream: 9.4.)
+    // handle's own trial graph on its own stream: 9.7.)
     BatchGraph &bg = h0->batch;
     bool kept = bg.exec != nullptr && (int)bg.of.size() == count;
     for (int k = 0; k < count && kept; k++)

@@ -1225,9 +1225,9 @@ __device__ __forceinline__ int line_before(double p, double s, double is, double
 // it out and nothing of the edge is looked up again.  The lane-per-piece form
 // of integrate_fast keeps 32 lanes busy on one cell but pays four times the
 // instructions a piece; with 8 lanes a cell the edges (6) and lines (5 to 8)
-// fill the lanes by themselves.  Bound by instruction issue (129 M warp
-// instructions at 262,144 sites on 2048^2 against 450 M, k_integrate 205
-// against 566 us; 65 against 150 us at 65,536 sites on 1024^2, where the
+// fill the lanes by themselves.  Bound by instruction issue (133 M warp
+// instructions at 262,144 sites on 2048^2 against 450 M, k_integrate 213
+// against 566 us; 72 against 150 us at 65,536 sites on 1024^2, where the
 // largest cells now take longest).
 //
 // The terms of a piece are taken about its middle (am, bm) with half extents
