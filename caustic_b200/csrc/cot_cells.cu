@@ -1603,7 +1603,8 @@ __device__ __forceinline__ RegPoly apply_chunk(RegPoly P, int jl, const double2 
         // and the others tested again on what it leaves.  A clip is a chain
         // of some 500 cycles whether or not it still cuts; the deepest first
         // leaves little for the rest (a chunk of a far too large ring 8 to 10
-        // us in order of the lanes).
+        // us in order of the lanes).  The depths are in single precision: they
+        // only order the clips.
         if (__popc(have) >= COT_DEEP_MIN) {
             const float rs = cut ? rsqrtf((float)key) : 0.0f;
             while (true) {
